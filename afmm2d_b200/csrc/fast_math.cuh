@@ -2,77 +2,83 @@
 // (near field, FP64 tensor-tile near field, on-the-fly M2L); the setup keeps
 // the correctly rounded log_cr / exp_cr of exact_math.cuh.
 //
-// log_tang:
-// Method: P. T. P. Tang, "Table-driven implementation of the logarithm
-// function in IEEE floating-point arithmetic", ACM TOMS 16(4), 1990.
-// x = 2^k m with m in [1, 2); F = 1 + j/128 is the breakpoint nearest m (j
-// from the top mantissa bits, rounded), f = m - F exactly (|f| <= 2^-8), and
-//   ln x = (k ln2_hi + lnF_hi) + (u0 + (k ln2_lo + lnF_lo + u1 + p(u0))),
-// where u0 + u1 = f/F (u0 = f * (1/F), u1 from its exact FMA residual), and
-// p(u) = ln(1 + u) - u = -u^2/2 + u^3/3 - ... - u^6/6 + u^7/7 (truncation
-// below 2^-59 relative for |u| <= 2^-8).  ln2_hi and lnF_hi are multiples of
-// 2^-42, so the first bracket is exact for every exponent; near x = 1 from
-// either side it is exactly zero (j = 0, k = 0, or j = 128, k = -1), so small
-// results keep full relative accuracy.  About 16 FP64 operations and two
-// table loads (math_tables.cuh, L1-resident).  Error within about one ulp for
-// positive normal x (tests compare it with the correctly rounded log); zero,
-// subnormal and non-finite inputs give an unspecified value without a trap,
-// which the kernel functors select away (their R2 < 1e-10 branch).
+// Both are table-driven (P. T. P. Tang, ACM TOMS 16(4), 1990, and 15(2),
+// 1989) with tables of 32 entries only, kept as one 128-byte line per 32-bit
+// word of an entry.  A warp's 32 lanes look up 32 different entries, and what
+// such a gather costs is the number of lines it touches, served one after
+// another by the L1 that the SM's four FP64 pipes share: the earlier tables
+// (129 entries of 8 and 16 bytes, 24 lines) took ~24 L1 cycles per 32 entries
+// where the ~25 FP64 operations of an entry take 13 (64 lanes per SM and
+// cycle), so the FP64 near field of the log kernel was bound by its table.  A
+// word line is one L1 cycle: four of them here, at the price of two more
+// polynomial steps.  FP64 near field at 1,048,576 uniform points, log: 1.48 ->
+// 1.34 ms; on-the-fly M2L of 262,144 spiral points, log: 0.87 -> 0.80 ms.
 #pragma once
 
 #include "math_tables.cuh"
 
 namespace afmm {
 
-__device__ __forceinline__ double log_tang(double x) {
-  const int hx = __double2hiint(x), lx = __double2loint(x);
-  const int frac_hi = hx & 0x000fffff;
-  const int j = (frac_hi + 0x1000) >> 13;  // round(128 (m - 1)), 0..128
-  const double m = __hiloint2double(frac_hi | 0x3ff00000, lx);
-  const double F = __hiloint2double(0x3ff00000 + (j << 13), 0);  // 1 + j/128 (2 for j = 128)
+// ln x for positive normal x.  x = 2^k m with m in [1 - 2^-6, 2 - 2^-6);
+// F = 1 + j/32 is the breakpoint nearest m, c = 1/F to 21 bits, u = m c - 1
+// (one rounding, below 2^-59; exact for j = 0, where c = 1), |u| <= 2^-6:
+//   ln x = (k ln2_hi + L_hi) + (u + (k ln2_lo + L_lo + u^2 q(u))),  L = -ln c.
+// ln2_hi and L_hi are multiples of 2^-42, so the first bracket is exact for
+// every exponent, and it is zero around x = 1 (j = 0, k = 0, on both sides),
+// where small results keep full relative accuracy.  q is the truncated
+// Chebyshev expansion of (ln(1+u) - u)/u^2 (error below 2^-57 of u).  14 FP64
+// operations.  Within one ulp (tests compare it with the correctly rounded
+// log); zero, subnormal and non-finite inputs give an unspecified value
+// without a trap, which the kernel functors select away.
+__device__ __forceinline__ double log_t32(double x) {
+  const int hx = __double2hiint(x);
+  const int t = hx + 0x4000;  // rounds the fraction to 5 bits, carrying into the exponent
+  const int j = (t >> 15) & 31;
+  const double m = __hiloint2double(hx - ((t & 0xfff00000) - 0x3ff00000), __double2loint(x));
   // k = biased exponent - 1023, as a double without an integer conversion
-  const double kd = __hiloint2double(0x43300000, (hx >> 20) & 0x7ff) - 4503599627371519.0;  // - (2^52 + 1023)
-  const double f = m - F;
-  const double inv = __ldg(&kLogInvF[j]);
-  const double2 lnF = __ldg(&kLogLnF[j]);
-  const double hi = fma(kd, kLn2Hi, lnF.x);  // exact
-  const double u0 = f * inv;
-  const double u1 = fma(-u0, F, f) * inv;    // the residual f - u0 F is exact
-  double q = fma(1.0 / 7.0, u0, -1.0 / 6.0);
-  q = fma(q, u0, 1.0 / 5.0);
-  q = fma(q, u0, -0.25);
-  q = fma(q, u0, 1.0 / 3.0);
-  q = fma(q, u0, -0.5);
-  const double p = q * (u0 * u0);
-  const double lo = (fma(kd, kLn2Lo, lnF.y) + u1) + p;
-  return hi + (u0 + lo);
+  const double kd = __hiloint2double(0x43300000, (t >> 20) & 0x7ff) - 4503599627371519.0;  // - (2^52 + 1023)
+  const unsigned int* T = &kLogT32[0][j];
+  const double c = __hiloint2double((int)__ldg(T), 0);
+  const double Lh = __hiloint2double((int)__ldg(T + 32), (int)__ldg(T + 64));
+  const double Ll = __hiloint2double((int)__ldg(T + 96), 0);
+  const double u = fma(m, c, -1.0);
+  const double hi = fma(kd, kLn2Hi, Lh);  // exact
+  const double lo = fma(kd, kLn2Lo, Ll);
+  double q = fma(kLogQ6, u, kLogQ5);
+  q = fma(q, u, kLogQ4);
+  q = fma(q, u, kLogQ3);
+  q = fma(q, u, kLogQ2);
+  q = fma(q, u, kLogQ1);
+  q = fma(q, u, kLogQ0);
+  return hi + (u + fma(q, u * u, lo));
 }
 
-// exp_tang: P. T. P. Tang, "Table-driven implementation of the exponential
-// function in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989.
-// x = (32 m + j) ln2/32 + r with N = 32 m + j the integer nearest x 32/ln2,
-// j = N mod 32, |r| <= ln2/64 (r = x - N L1 - N L2, N L1 exact);
+// exp x.  x = (32 m + j) ln2/32 + r with N = 32 m + j the integer nearest
+// x 32/ln2, j = N mod 32, |r| <= ln2/64 (r = x - N L1 - N L2, N L1 exact);
 //   exp(x) = 2^m (S_hi + (S_lo + S p(r))),  S = 2^(j/32) = S_hi + S_lo,
 // p(r) = exp(r) - 1 by its Taylor polynomial to r^6 (truncation below
-// 2^-58).  About 13 FP64 operations and one table load.  Error within about
-// one ulp for x in [-708, 709.7] (tests compare it with the correctly rounded
-// exp); below -708 it returns 0 (the true value is under 2^-1021).
-__device__ __forceinline__ double exp_tang(double x) {
+// 2^-58); 2^m is added to the exponent bits.  13 FP64 operations.  Error
+// within about one ulp for x in [-708, 709.7] (tests compare it with the
+// correctly rounded exp); below -708 it returns 0 (the true value is under
+// 2^-1021).
+__device__ __forceinline__ double exp_t32(double x) {
   const double shifter = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
   const double t = fma(x, k32OverLn2, shifter);
   const int N = __double2loint(t);
   const double nd = t - shifter;
   double r = fma(-nd, kLn2Over32Hi, x);  // exact
   r = fma(-nd, kLn2Over32Lo, r);
-  const double2 S = __ldg(&kExp2J32[N & 31]);
+  const unsigned int* T = &kExpT32[0][N & 31];
+  const double Sh = __hiloint2double((int)__ldg(T), (int)__ldg(T + 32));
+  const double Sl = __hiloint2double((int)__ldg(T + 64), 0);
   double q = fma(1.0 / 720.0, r, 1.0 / 120.0);
   q = fma(q, r, 1.0 / 24.0);
   q = fma(q, r, 1.0 / 6.0);
   q = fma(q, r, 0.5);
   const double p = fma(q * r, r, r);
-  const double v = S.x + fma(S.x, p, fma(S.y, p, S.y));
-  const double scale = __hiloint2double(((N >> 5) + 1023) << 20, 0);  // 2^m
-  return x < -708.0 ? 0.0 : v * scale;
+  const double v = Sh + fma(Sh, p, fma(Sl, p, Sl));
+  const double y = __hiloint2double(__double2hiint(v) + ((N >> 5) << 20), __double2loint(v));
+  return x < -708.0 ? 0.0 : y;
 }
 
 }  // namespace afmm
