@@ -107,14 +107,20 @@ struct afmm_handle {
   bool have_last = false;
   // host-pointer matvecs: copy streams
   cudaStream_t s_h2d = nullptr, s_d2h = nullptr;
+  // the one-column near field's stream, output and the leaves that a shard runs
+  cudaStream_t s_near = nullptr;
+  cudaEvent_t ev_q = nullptr, ev_near = nullptr;
+  double* d_near = nullptr;
+  int32_t* d_near_run = nullptr;
   cudaEvent_t ev_in[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr}, ev_out[2] = {nullptr, nullptr};
   cudaEvent_t ev_sync = nullptr;
   std::string err;
   ~afmm_handle() {
-    for (cudaEvent_t e : {ev_in[0], ev_in[1], ev_done[0], ev_done[1], ev_out[0], ev_out[1], ev_sync})
+    for (cudaEvent_t e : {ev_in[0], ev_in[1], ev_done[0], ev_done[1], ev_out[0], ev_out[1], ev_sync, ev_q, ev_near})
       if (e) cudaEventDestroy(e);
     if (s_h2d) cudaStreamDestroy(s_h2d);
     if (s_d2h) cudaStreamDestroy(s_d2h);
+    if (s_near) cudaStreamDestroy(s_near);
   }
 };
 
@@ -321,6 +327,23 @@ void apply_shard(afmm_handle* h) {
   const long sl = 1L << (2 * (h->L - lev));
   p.near_own.leaf0 = k0 * sl;
   p.near_own.nleaf = (k1 - k0) * sl;
+  {
+    // the one-column FP64 near field works a pair of leaves out once, in the
+    // leaf that has the other in its slots 0..3: the shard runs its own leaves
+    // and those with one of them there
+    const long l0 = k0 * sl, l1 = k1 * sl;
+    std::vector<int32_t> nbr((size_t)p.near.nleaf * 8), run;
+    AFMM_CUDA(cudaMemcpy(nbr.data(), p.near.nbr, sizeof(int32_t) * nbr.size(), cudaMemcpyDeviceToHost));
+    for (long b = 0; b < p.near.nleaf; ++b) {
+      bool on = b >= l0 && b < l1;
+      for (int t = 0; t < 4; ++t) on = on || (nbr[b * 8 + t] >= l0 && nbr[b * 8 + t] < l1);
+      if (on) run.push_back((int32_t)b);
+    }
+    if (!h->d_near_run) h->d_near_run = h->arena.alloc<int32_t>(p.near.nleaf);
+    AFMM_CUDA(cudaMemcpy(h->d_near_run, run.data(), sizeof(int32_t) * run.size(), cudaMemcpyHostToDevice));
+    p.near_own.run = h->d_near_run;
+    p.near_own.nrun = (long)run.size();
+  }
   p.shard_index = h->shard_index;
   p.shard_count = h->shard_count;
   p.shard_level = lev;
@@ -418,6 +441,11 @@ void build_plan(afmm_handle* h) {
   nv.leaf_start = h->d_leaf_start;
   nv.leaf_cnt = h->d_leaf_cnt;
   nv.nbr = h->lv[h->L].nbr;
+  nv.part = h->d_near;
+  nv.n = h->N;
+  p.s_near = h->s_near;
+  p.ev_q = h->ev_q;
+  p.ev_near = h->ev_near;
   apply_shard(h);
 }
 
@@ -426,15 +454,16 @@ void create_layout(afmm_handle* h);
 // Streams and events of a handle (afmm_create, afmm_load).
 void create_streams(afmm_handle* h) {
   AFMM_CUDA(cudaGetDevice(&h->device));
-  // the handle's stream at the highest priority: batched passes run their
-  // near field beside the far field on a lowest-priority stream
+  // the handle's stream at the highest priority: the near field runs beside
+  // the far field on a lowest-priority stream
   int least = 0, greatest = 0;
   AFMM_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
   AFMM_CUDA(cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, greatest));
+  AFMM_CUDA(cudaStreamCreateWithPriority(&h->s_near, cudaStreamNonBlocking, least));
   AFMM_CUDA(cudaStreamCreateWithFlags(&h->s_h2d, cudaStreamNonBlocking));
   AFMM_CUDA(cudaStreamCreateWithFlags(&h->s_d2h, cudaStreamNonBlocking));
   for (cudaEvent_t* e : {&h->ev_in[0], &h->ev_in[1], &h->ev_done[0], &h->ev_done[1], &h->ev_out[0], &h->ev_out[1],
-                         &h->ev_sync})
+                         &h->ev_sync, &h->ev_q, &h->ev_near})
     AFMM_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
 }
 
@@ -534,6 +563,7 @@ void create_layout(afmm_handle* h) {
   AFMM_CUDA(cudaMemcpyAsync(lf.node_ids, ids.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
   h->d_qs = h->arena.alloc<double>(N + 2);  // + 16 B: whole-piece L2 prefetches of source rows
   h->d_ys = h->arena.alloc<double>(N);
+  h->d_near = h->arena.alloc<double>((size_t)kNearParts * N);
   h->d_q = h->arena.alloc<double>(N);
   h->d_y = h->arena.alloc<double>(N);
   AFMM_CUDA(cudaStreamSynchronize(s));
@@ -2062,7 +2092,7 @@ afmm_status afmm_set_create(afmm_handle* const* handles, int n, afmm_set** out) 
   afmm_status rc = guard(nullptr, [&] {
     check_device();
     if (!handles || n < 1) throw Error{AFMM_BAD_ARG, "afmm_set_create: need n >= 1 handles"};
-    std::vector<SetProblem> probs;
+    std::vector<const MatvecPlan*> probs;
     int dev = -1;
     AFMM_CUDA(cudaGetDevice(&dev));
     for (int p = 0; p < n; ++p) {
@@ -2073,10 +2103,12 @@ afmm_status afmm_set_create(afmm_handle* const* handles, int n, afmm_set** out) 
       if (!h->m2l_stored) throw Error{AFMM_BAD_ARG, "afmm_set_create: a handle has no stored M2L blocks"};
       if (h->shard_count > 1) throw Error{AFMM_BAD_ARG, "afmm_set_create: a handle is sharded"};
       if (h->device != dev) throw Error{AFMM_BAD_ARG, "afmm_set_create: handle on another device"};
-      probs.push_back({&h->plan, p2p_shape(h->plan.near.nmax)});
+      probs.push_back(&h->plan);
     }
     st = new afmm_set();
-    AFMM_CUDA(cudaStreamCreateWithFlags(&st->stream, cudaStreamNonBlocking));
+    int least = 0, greatest = 0;  // above the near field, which runs beside the far field
+    AFMM_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    AFMM_CUDA(cudaStreamCreateWithPriority(&st->stream, cudaStreamNonBlocking, greatest));
     for (int p = 0; p < n; ++p) AFMM_CUDA(cudaStreamSynchronize(handles[p]->stream));
     st->plan.kernel_id = handles[0]->kernel_id;
     set_build(st->plan, probs, st->arena, st->stream);

@@ -208,7 +208,17 @@ struct NearView {
   const double2* anchor = nullptr;     // leaf anchors (FP64)
   const float2* rel = nullptr;         // point minus its leaf anchor (FP32), sorted order
   const float* span = nullptr;         // per leaf max |rel| component
+  // FP64 near field of one column (near_leaf): its outputs, and for a shard
+  // the leaves to run (the shard's own, and those that hold a pair with one of
+  // its leaves); null: leaves leaf0 .. leaf0 + nleaf - 1
+  double* part = nullptr;  // kNearParts x n
+  long n = 0;              // points
+  const int32_t* run = nullptr;
+  long nrun = 0;
 };
+// Near-field sums of a point: its leaf's own work, and what the four leaves
+// before it (neighbour slots 4..7) worked out for it.
+constexpr int kNearParts = 5;
 
 // CUDA-event marks for per-stage device timing.
 struct StageTimer {
@@ -297,6 +307,10 @@ struct MatvecPlan {
   int n1max[kMaxLevels] = {0};  // largest node count per level
   LevelSet levels;       // levels 2..L for the M2L launch
   NearView near;
+  // the near field of a one-column product runs on this lower-priority stream
+  // beside the far field, into near.part; the scatter adds the two
+  cudaStream_t s_near = nullptr;
+  cudaEvent_t ev_q = nullptr, ev_near = nullptr;
   Tuning tune;
   // A shard of one problem (afmm_set_shard): the stored-block M2L and the
   // L2L of the levels at and below shard_level, and the near field, run only
@@ -309,6 +323,18 @@ struct MatvecPlan {
   LevelView lv_down[kMaxLevels];
   NearView near_own;
 };
+
+// Runs near(stream) on the plan's near-field stream, after what is queued on s
+// so far; p.ev_near marks its end.
+template <class F>
+inline void near_beside(const MatvecPlan& p, cudaStream_t s, StageTimer* tm, F&& near) {
+  AFMM_CUDA(cudaEventRecord(p.ev_q, s));
+  AFMM_CUDA(cudaStreamWaitEvent(p.s_near, p.ev_q, 0));
+  const int sp = tm ? tm->span_begin(p.s_near, "p2p_kernel") : -1;  // the kernel's own duration
+  near(p.s_near);
+  if (tm) tm->span_end(p.s_near, sp);
+  AFMM_CUDA(cudaEventRecord(p.ev_near, p.s_near));
+}
 
 // Level and box range [k0, k1) of shard `index` of `count` on a tree of
 // levels 2..L: the shallowest level with at least four boxes per shard (the
@@ -330,18 +356,42 @@ inline bool shard_range(int L, int index, int count, int& level, long& k0, long&
   return true;
 }
 
-// Near-field launch shape: NT threads per target group (targets rounded up to
-// a warp multiple), G groups splitting the (up to 9) source leaves.
-struct P2pShape {
-  int nt, g, threads;
-};
-inline P2pShape p2p_shape(int nmax) {
-  P2pShape p;
-  p.nt = (nmax + 31) / 32 * 32;
-  p.g = std::max(1, std::min(9, 256 / p.nt));
-  p.threads = p.nt * p.g;
-  return p;
+// Warps per CTA of the FP64 near field of leaves of up to nmax points
+// (near_leaf): the leaf's five source leaves make blocks of 32 points, up to
+// kNearJ of them a warp at a time.
+constexpr int kNearJ = 2;
+inline int near_warps(int nmax) {
+  const int blocks = (5 * nmax + 31) / 32;
+  int best = 1;
+  double fill = 0.0;  // how evenly the warps share the blocks
+  for (int w = 1; w <= 8; ++w) {
+    const int per = (blocks + w - 1) / w;  // blocks of the busiest warp
+    const double f = (double)blocks / (per * w) - (per > 2 * kNearJ && w < 8 ? 1.0 : 0.0);
+    if (f >= fill) {
+      fill = f;
+      best = w;
+    }
+  }
+  return best;
 }
+// Targets that a warp goes round: n, or (leaves below 32 points) the next
+// power of two, with the lanes in groups of that many.
+__host__ __device__ __forceinline__ int near_ring(int n) {
+  if (n >= 32) return n;
+  int r = 1;
+  while (r < n) r *= 2;
+  return r;
+}
+// The leaf's points and charges are repeated behind their end, and a warp's
+// row of target sums is as long, so that no lane's index wraps.
+__host__ __device__ __forceinline__ int near_row(int n) { return (n < 32 ? 32 : n) + 32; }
+inline size_t near_smem(int nmax, int warps) {
+  const size_t row = near_row(nmax);
+  return row * (sizeof(double2) + sizeof(double)) + nmax * sizeof(double) + (size_t)warps * row * sizeof(double);
+}
+// Stand-in coordinates of padded points (finite entries for every kernel,
+// their results are not used).
+constexpr double kPadPoint = 1.0e100;
 
 // ------------------------------------------------ FP64 sweep rows
 // The arithmetic of one output of each FP64 sweep, shared by the
@@ -481,71 +531,171 @@ __device__ __forceinline__ NearSlots near_slots(const NearView& nv, long b, int 
   return r;
 }
 
-// Near field (src/AFMM2DTree.cpp:1199-1213) of leaf b: neighbours 0..7 and the
-// leaf itself, kernel evaluated on the fly.  Run by one CTA of at least
-// NT * G threads: all source leaves are staged in shared memory (`smem`:
-// 9 * nmax double2 + 9 * nmax double + NT * G double); G groups of NT
-// threads split the source leaves (group g takes leaves g, g+G, ...), each
-// thread owns one target, and the groups' sums are added in group order.
+// One block of J x 32 source points of near_leaf: lane l owns the points f0 + l,
+// f0 + 32 + l, ... of the flat list of leaf b's source leaves, and meets leaf
+// b's point (l + t) mod n at step t, so that in every step the lanes of the
+// warp hold different targets.  KIND: the block's points all belong to leaf b
+// (0), all to neighbours (1), or neither (2: some lanes take no part in leaf
+// b's sums).
+template <class K, int J, int KIND>
+__device__ __forceinline__ void near_block(const NearView& nv, const KernelParams& kp, const double* __restrict__ qs,
+                                           int f0, int total, const int* s_off, const int* s_src, const int* s_dst,
+                                           int ns, int ring, const double2* px, const double* pq, double* acc,
+                                           double* self) {
+  const int lane = threadIdx.x & 31;
+  double2 x[J];
+  double w[J], sum[J];
+  int idx[J], dst[J];  // sorted point; its part (0: leaf b itself, -1: unused lane, kNearParts: not stored)
+#pragma unroll
+  for (int u = 0; u < J; ++u) {
+    const int f = f0 + 32 * u + lane;
+    const int g = min(f, total - 1);  // lanes past the end repeat the last point, unused
+    int m = 0;
+    while (m + 1 < ns && g >= s_off[m + 1]) ++m;
+    idx[u] = s_src[m] + (g - s_off[m]);
+    dst[u] = f < total ? s_dst[m] : -1;
+    x[u] = nv.pts[idx[u]];
+    w[u] = qs[idx[u]];
+    sum[u] = 0.0;
+  }
+#pragma unroll 4
+  for (int t = 0; t < ring; ++t) {
+    const double2 p = px[t];
+    const double qi = pq[t];
+    double a = KIND > 0 ? acc[t] : 0.0;
+#pragma unroll
+    for (int u = 0; u < J; ++u) {
+      const double dx = x[u].x - p.x, dy = x[u].y - p.y;
+      const double k = K::eval(dx * dx + dy * dy, kp);
+      sum[u] += k * qi;
+      if (KIND == 1) a += k * w[u];
+      if (KIND == 2) a += (dst[u] > 0 ? k : 0.0) * w[u];
+    }
+    if (KIND > 0) {
+      acc[t] = a;
+      __syncwarp();  // the next lane takes the target over
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < J; ++u) {
+    if (dst[u] > 0 && dst[u] < kNearParts) nv.part[(size_t)dst[u] * nv.n + idx[u]] = sum[u];
+    else if (dst[u] == 0) self[f0 + 32 * u + lane] = sum[u];  // leaf b comes first in the flat list
+  }
+}
+
+// Near field (src/AFMM2DTree.cpp:1199-1213) of leaf b, kernel evaluated on the
+// fly, every unordered pair of leaves once: K(x, y) depends on |x - y| only, so
+// the pairs of leaf b with the neighbours in slots 0..3 give both leaves' sums
+// (slots 4..7 are their opposites: those pairs belong to the neighbours), and
+// with itself the leaf's own.  Per point nv.part[0] takes the leaf's own
+// work and part[1 + s] what its neighbour in slot 4 + s worked out for it
+// (zero without one); the scatter adds the five in that order.  An entry costs
+// 15 to 22 FP64 operations and about as many integer ones, its use two, so
+// working it out once for both leaves (5/9 of the entries) pays for the target
+// sums that go from lane to lane through shared memory (four cycles of 18 an
+// entry pair takes there).  What bounds it now is issue (63% of the slots,
+// FP64 pipe 49% busy) and the polynomials' dependent steps: 80 registers (24
+// warps an SM) measured faster than 102 or 64.  Near field at 1,048,576 uniform
+// points, one CTA per leaf, all nine source leaves before -> now: log 1.34 ->
+// 0.79 ms, Gaussian 1.03 -> 0.66, 1/r (mixture) 0.64 -> 0.42; 100,003 points of
+// scaled 1/r (M = 100) 0.63 -> 0.42.  Run by one CTA of near_warps(nmax) warps
+// that share the blocks of 32 source points evenly (more may be present); the
+// sums of the warps are added in warp order.
 template <class K>
-__device__ __forceinline__ void p2p64_leaf(const NearView& nv, const KernelParams& kp, const double* __restrict__ qs,
-                                           double* __restrict__ ys, int NT, int G, long b, unsigned char* smem) {
-  __shared__ int s_src[9], s_cnt[9], s_off[10], s_ns;
+__device__ __forceinline__ void near_leaf(const NearView& nv, const KernelParams& kp, const double* __restrict__ qs,
+                                          int warps, long b, unsigned char* smem) {
+  __shared__ int s_src[5], s_off[6], s_dst[5], s_back[4], s_ns;
   const int n = nv.leaf_cnt[b];
   const int s0 = nv.leaf_start[b];
+  const bool own = b >= nv.leaf0 && b < nv.leaf0 + nv.nleaf;
   if (threadIdx.x < 32) {
-    const NearSlots sl = near_slots<1>(nv, b, threadIdx.x);
-    if (sl.m >= 0) {
-      s_src[sl.m] = sl.start;
-      s_cnt[sl.m] = sl.cnt;
-      s_off[sl.m] = sl.off;
-    }
-    if (threadIdx.x == 0) {
-      s_off[sl.ns] = sl.total;
-      s_ns = sl.ns;
-    }
-  }
-  __syncthreads();
-  const int ns = s_ns;
-  double2* sx = (double2*)smem;
-  double* sq = (double*)(sx + 9 * nv.nmax);
-  double* red = sq + 9 * nv.nmax;  // G x NT
-  for (int m = 0; m < ns; ++m)
-    for (int t = threadIdx.x; t < s_cnt[m]; t += blockDim.x) {
-      sx[s_off[m] + t] = nv.pts[s_src[m] + t];
-      sq[s_off[m] + t] = qs[s_src[m] + t];
-    }
-  __syncthreads();
-  const bool active = (int)threadIdx.x < NT * G;
-  const int i = threadIdx.x % NT, g = threadIdx.x / NT;
-  double acc = 0.0;
-  if (active && i < n) {
-    const double2 xi = nv.pts[s0 + i];
-    for (int m = g; m < ns; m += G) {
-      const int o = s_off[m], nc = s_cnt[m];
-      double a0 = 0.0, a1 = 0.0;
-      int t = 0;
-      for (; t + 1 < nc; t += 2) {
-        const double2 p0 = sx[o + t], p1 = sx[o + t + 1];
-        const double dx0 = xi.x - p0.x, dy0 = xi.y - p0.y, dx1 = xi.x - p1.x, dy1 = xi.y - p1.y;
-        a0 += K::eval(dx0 * dx0 + dy0 * dy0, kp) * sq[o + t];
-        a1 += K::eval(dx1 * dx1 + dy1 * dy1, kp) * sq[o + t + 1];
+    const int lane = threadIdx.x;
+    // lane 0: the leaf; lanes 1..4: neighbour slots 0..3; lanes 5..8: slots 4..7
+    long c = -1;
+    int cnt = 0, start = 0;
+    if (lane < 9) {
+      c = lane == 0 ? b : (long)nv.nbr[b * 8 + lane - 1];
+      if (c >= 0 && lane < 5) {
+        start = nv.leaf_start[c];
+        cnt = nv.leaf_cnt[c];
       }
-      if (t < nc) {
-        const double2 p0 = sx[o + t];
-        const double dx0 = xi.x - p0.x, dy0 = xi.y - p0.y;
-        a0 += K::eval(dx0 * dx0 + dy0 * dy0, kp) * sq[o + t];
-      }
-      acc += a0 + a1;
     }
+    const unsigned valid = __ballot_sync(0xffffffffu, lane < 5 && c >= 0);
+    int pre = cnt;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, pre, o);
+      if (lane >= o) pre += t;
+    }
+    if (lane < 5 && c >= 0) {
+      const int m = __popc(valid & ((1u << lane) - 1u));
+      s_src[m] = start;
+      s_off[m] = pre - cnt;
+      // (a leaf outside the shard gets no sums)
+      s_dst[m] = lane == 0 ? 0 : (c >= nv.leaf0 && c < nv.leaf0 + nv.nleaf ? lane : kNearParts);
+    }
+    if (lane == 4) {
+      s_ns = __popc(valid);
+      s_off[__popc(valid)] = pre;
+    }
+    if (lane >= 5 && lane < 9) s_back[lane - 5] = c >= 0;
   }
-  if (active) red[g * NT + i] = acc;
+  const int row = near_row(n), ring = near_ring(n);
+  double2* px = (double2*)smem;
+  double* pq = (double*)(px + row);
+  double* self = pq + row;
+  double* accs = self + n;
+  for (int t = threadIdx.x; t < row; t += blockDim.x) {
+    const int i = t % ring;
+    px[t] = i < n ? nv.pts[s0 + i] : make_double2(kPadPoint, kPadPoint);
+    pq[t] = i < n ? qs[s0 + i] : 0.0;
+  }
+  for (int i = threadIdx.x; i < warps * row; i += blockDim.x) accs[i] = 0.0;
   __syncthreads();
-  if (active && g == 0 && i < n) {
-    double s = ys[s0 + i];
-    for (int h = 0; h < G; ++h) s += red[h * NT + i];
-    ys[s0 + i] = s;
+  const int ns = s_ns, total = s_off[ns], nblk = (total + 31) >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < warps) {
+    // lane l starts at target l (of its group's row)
+    const int l0 = n < 32 ? lane & (ring - 1) : lane;
+    double* acc = accs + warp * row + (n < 32 ? 2 * (lane - l0) : 0) + l0;
+    const int b1 = (warp + 1) * nblk / warps;
+#define AFMM_NEAR(J, KIND) \
+  near_block<K, J, KIND>(nv, kp, qs, 32 * k, total, s_off, s_src, s_dst, ns, ring, px + l0, pq + l0, acc, self)
+    for (int k = warp * nblk / warps; k < b1;) {
+      const int nb = min(kNearJ, b1 - k);
+      const int kind = 32 * (k + nb) <= n ? 0 : (32 * k >= n && 32 * (k + nb) <= total ? 1 : 2);
+      if (nb == 2) {
+        if (kind == 0) AFMM_NEAR(2, 0);
+        else if (kind == 1) AFMM_NEAR(2, 1);
+        else AFMM_NEAR(2, 2);
+      } else {
+        if (kind == 0) AFMM_NEAR(1, 0);
+        else if (kind == 1) AFMM_NEAR(1, 1);
+        else AFMM_NEAR(1, 2);
+      }
+      k += nb;
+    }
+#undef AFMM_NEAR
   }
+  __syncthreads();
+  if (!own) return;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    double v = self[i];
+    for (int x = 0; x < warps; ++x) {
+      const double* r = accs + x * row + i;
+      if (n >= 32) v += i < 32 ? r[0] + r[n] : r[0];
+      else
+        for (int c = 0; c < 64; c += 2 * ring) v += r[c] + r[c + ring];
+    }
+    nv.part[s0 + i] = v;
+    for (int s = 0; s < 4; ++s)
+      if (!s_back[s]) nv.part[(size_t)(1 + s) * nv.n + s0 + i] = 0.0;
+  }
+}
+
+// Sum of the near field's parts of sorted point i.
+__device__ __forceinline__ double near_sum(const double* __restrict__ part, long n, long i) {
+  return (((part[i] + part[n + i]) + part[2 * n + i]) + part[3 * n + i]) + part[4 * n + i];
 }
 
 void build_lists(int j, long nbox, int32_t* nbr, int32_t* il, cudaStream_t s);

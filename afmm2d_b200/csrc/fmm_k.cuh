@@ -40,21 +40,20 @@ struct M2lAssembleRun {
   }
 };
 
-// Near field (src/AFMM2DTree.cpp:1199-1213): one CTA per leaf.
+// Near field (src/AFMM2DTree.cpp:1199-1213): one CTA per leaf, into nv.part.
 template <class K>
-__global__ void k_p2p64(NearView nv, KernelParams kp, const double* __restrict__ qs, double* __restrict__ ys, int NT,
-                        int G) {
+__global__ void __launch_bounds__(256, 3) k_p2p64(NearView nv, KernelParams kp, const double* __restrict__ qs, int warps) {
   extern __shared__ __align__(16) unsigned char smem[];
-  p2p64_leaf<K>(nv, kp, qs, ys, NT, G, nv.leaf0 + blockIdx.x, smem);
+  near_leaf<K>(nv, kp, qs, warps, nv.run ? (long)nv.run[blockIdx.x] : nv.leaf0 + blockIdx.x, smem);
 }
 
 template <class K>
 struct P2p64Run {
-  static void run(const NearView& nv, const KernelParams& kp, const double* qs, double* ys, cudaStream_t s) {
-    P2pShape sh = p2p_shape(nv.nmax);
-    size_t smem = (size_t)9 * nv.nmax * (sizeof(double2) + sizeof(double)) + sizeof(double) * sh.threads;
+  static void run(const NearView& nv, const KernelParams& kp, const double* qs, cudaStream_t s) {
+    const int warps = near_warps(nv.nmax);
+    const size_t smem = near_smem(nv.nmax, warps);
     allow_smem(k_p2p64<K>, smem);
-    k_p2p64<K><<<(int)nv.nleaf, sh.threads, smem, s>>>(nv, kp, qs, ys, sh.nt, sh.g);
+    k_p2p64<K><<<(int)(nv.run ? nv.nrun : nv.nleaf), 32 * warps, smem, s>>>(nv, kp, qs, warps);
     AFMM_LAUNCH_CHECK();
   }
 };

@@ -18,7 +18,7 @@ namespace afmm {
 
 // Bumped whenever KernelTable or an argument type of its launchers changes:
 // a table compiled against other headers is refused at registration.
-constexpr int kKernelTableAbi = 4;
+constexpr int kKernelTableAbi = 5;
 
 // Fingerprint of the layouts of the launchers' argument types (sizes and a
 // few field offsets), recorded in every table where it is compiled: a table
@@ -37,8 +37,8 @@ struct KernelTable {
   const char* name = nullptr;
   // M2L blocks K(R_b, R_c) of one level, setup arithmetic (fmm_k.cuh)
   void (*m2l_assemble)(const LevelView&, const KernelParams&, cudaStream_t) = nullptr;
-  // FP64 near field, one column (fmm_k.cuh)
-  void (*p2p64)(const NearView&, const KernelParams&, const double*, double*, cudaStream_t) = nullptr;
+  // FP64 near field, one column, into NearView::part (fmm_k.cuh)
+  void (*p2p64)(const NearView&, const KernelParams&, const double*, cudaStream_t) = nullptr;
   // single-RHS mixed path: M2L on the fly (FP64), FP32 near field (mixed_k.cuh)
   void (*m2l_otf)(const LevelSet&, const KernelParams&, cudaStream_t) = nullptr;
   void (*p2p32)(const NearView&, const KernelParams&, const float*, double*, cudaStream_t) = nullptr;

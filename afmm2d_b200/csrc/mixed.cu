@@ -66,9 +66,10 @@ __global__ void k_gather_mixed(const double* __restrict__ q, const int64_t* __re
   qs32[i] = (float)v;
 }
 
-__global__ void k_scatter64(const double* __restrict__ ys, const int64_t* __restrict__ perm, int N, double* y) {
+__global__ void k_scatter64(const double* __restrict__ ys, const double* __restrict__ near,
+                            const int64_t* __restrict__ perm, int N, double* y) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < N) y[perm[i]] = ys[i];
+  if (i < N) y[perm[i]] = ys[i] + near[i];
 }
 
 inline int nb(long n, int t) { return (int)((n + t - 1) / t); }
@@ -118,10 +119,21 @@ void matvec_mixed(const MatvecPlan& p, MixedState& ms, const double* q, int64_t 
   nv.span = ms.leaf_span;
   for (int c = 0; c < nrhs; ++c) {
     if (tm) tm->mark(s, "gather");
-    if (p.shard_count > 1) AFMM_CUDA(cudaMemsetAsync(ms.ys, 0, sizeof(double) * (size_t)N, s));
+    if (p.shard_count > 1) {
+      AFMM_CUDA(cudaMemsetAsync(ms.ys, 0, sizeof(double) * (size_t)N, s));
+      AFMM_CUDA(cudaMemsetAsync(p.near.part, 0, sizeof(double) * (size_t)N, s));
+    }
     k_gather_mixed<<<nb(N, 256), 256, 0, s>>>(q + (long)c * ldq, p.perm, N, ms.qs, ms.qs32);
     AFMM_LAUNCH_CHECK();
     ++*launches;
+    // the near field beside the far field, as in the FP64 path (nv.part as its output: same single
+    // addition to the far field's potentials)
+    const bool beside = !(tm && tm->serial);
+    auto near = [&](cudaStream_t st) {
+      kernel_table(p.kp.id).p2p32(nv, p.kp, ms.qs32, nv.part, st);
+      ++*launches;
+    };
+    if (beside) near_beside(p, s, tm, near);
     if (tm) tm->mark(s, "m2m");
     sweep_m2m(p, ms.qs, s, launches);
     if (tm) tm->mark(s, "m2l");
@@ -144,10 +156,10 @@ void matvec_mixed(const MatvecPlan& p, MixedState& ms, const double* q, int64_t 
     if (tm) tm->mark(s, "l2l");
     sweep_l2l(p, ms.ys, s, launches);
     if (tm) tm->mark(s, "p2p");
-    kernel_table(p.kp.id).p2p32(nv, p.kp, ms.qs32, ms.ys, s);
-    ++*launches;
+    if (beside) AFMM_CUDA(cudaStreamWaitEvent(s, p.ev_near, 0));
+    else near(s);
     if (tm) tm->mark(s, "scatter");
-    k_scatter64<<<nb(N, 256), 256, 0, s>>>(ms.ys, p.perm, N, y + (long)c * ldy);
+    k_scatter64<<<nb(N, 256), 256, 0, s>>>(ms.ys, nv.part, p.perm, N, y + (long)c * ldy);
     AFMM_LAUNCH_CHECK();
     ++*launches;
   }

@@ -80,13 +80,14 @@ __device__ __forceinline__ float near_pair(const NearView& nv, const KernelParam
 
 // Near field in FP32 from leaf-relative coordinates.  One CTA per leaf; all
 // source leaves (neighbours 0..7, then the leaf) are staged in shared memory
-// at once, with each source leaf's anchor offset folded in FP64; G groups of
-// NT threads split the source leaves, each thread owns one target, FP32
-// partial sums per source leaf are added in FP64, and the groups' sums are
-// added in group order.
+// at once, with each source leaf's anchor offset folded in FP64; each thread
+// owns one target and sums all of its source leaves (the FP32 entries are
+// cheap, so splitting the leaves over thread groups only adds imbalance and a
+// reduction: 1.12 vs 1.62 ms at 1M uniform points, log), FP32 partial sums
+// per source leaf added in FP64.  Writes the sums of leaf b's points to
+// `out`; the scatter adds them to the far field's.
 template <class K>
-__global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ qs32, double* __restrict__ ys, int NT,
-                        int G) {
+__global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ qs32, double* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_src[9], s_cnt[9], s_off[10], s_ns;
   __shared__ float s_dx[9], s_dy[9], s_thr[9];
@@ -114,18 +115,17 @@ __global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ 
   const int ns = s_ns;
   float2* sx = (float2*)smem;
   float* sq = (float*)(sx + 9 * nv.nmax);
-  double* red = (double*)(((uintptr_t)(sq + 9 * nv.nmax) + 15) & ~(uintptr_t)15);  // G x NT
   for (int m = 0; m < ns; ++m)
     for (int t = threadIdx.x; t < s_cnt[m]; t += blockDim.x) {
       sx[s_off[m] + t] = nv.rel[s_src[m] + t];
       sq[s_off[m] + t] = qs32[s_src[m] + t];
     }
   __syncthreads();
-  const int i = threadIdx.x % NT, g = threadIdx.x / NT;
+  const int i = threadIdx.x;
   double acc = 0.0;
   if (i < n) {
     const float2 xi = nv.rel[s0 + i];
-    for (int m = g; m < ns; m += G) {
+    for (int m = 0; m < ns; ++m) {
       const int o = s_off[m], nc = s_cnt[m];
       const float ox = xi.x + s_dx[m], oy = xi.y + s_dy[m], thr = s_thr[m];
       float a0 = 0.0f, a1 = 0.0f;
@@ -154,27 +154,16 @@ __global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ 
       acc += (double)a0 + (double)a1;
     }
   }
-  red[g * NT + i] = acc;
-  __syncthreads();
-  if (g == 0 && i < n) {
-    double s = ys[s0 + i];
-    for (int h = 0; h < G; ++h) s += red[h * NT + i];
-    ys[s0 + i] = s;
-  }
+  if (i < n) out[s0 + i] = acc;
 }
 
 template <class K>
 struct P2p32Run {
-  static void run(const NearView& nv, const KernelParams& kp, const float* qs32, double* ys, cudaStream_t s) {
-    // one group: every thread sums all of its target's source leaves (the
-    // FP32 entries are cheap, so splitting the leaves over groups only adds
-    // imbalance and a reduction: 1.12 vs 1.62 ms at 1M uniform points, log)
-    P2pShape sh = p2p_shape(nv.nmax);
-    sh.g = 1;
-    sh.threads = sh.nt;
-    size_t smem = (size_t)9 * nv.nmax * (sizeof(float2) + sizeof(float)) + 16 + sizeof(double) * sh.threads;
+  static void run(const NearView& nv, const KernelParams& kp, const float* qs32, double* out, cudaStream_t s) {
+    const int threads = (nv.nmax + 31) / 32 * 32;
+    const size_t smem = (size_t)9 * nv.nmax * (sizeof(float2) + sizeof(float));
     allow_smem(k_p2p32<K>, smem);
-    k_p2p32<K><<<(int)nv.nleaf, sh.threads, smem, s>>>(nv, kp, qs32, ys, sh.nt, sh.g);
+    k_p2p32<K><<<(int)nv.nleaf, threads, smem, s>>>(nv, kp, qs32, out);
     AFMM_LAUNCH_CHECK();
   }
 };

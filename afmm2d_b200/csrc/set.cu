@@ -22,14 +22,16 @@ __global__ void k_set_gather(SetDev d, SetSegs sg, const double* __restrict__ q)
   d.qs[p][i] = q[d.off[p] + d.perm[p][i]];
 }
 
-// y[off[p] + perm_p[i]] = ys_p[i]  (src/AFMM2D.cpp:61-63 per problem)
+// y[off[p] + perm_p[i]] = ys_p[i] + near field  (src/AFMM2D.cpp:61-63 per problem)
 __global__ void k_set_scatter(SetDev d, SetSegs sg, double* __restrict__ y) {
   const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= sg.total) return;
   const int s = seg_of(sg, g);
   const int p = sg.prob[s];
   const long i = g - sg.first[s];
-  y[d.off[p] + d.perm[p][i]] = d.ys[p][i];
+  const double v = d.ys[p][i] + near_sum(d.nv[p].part, d.nv[p].n, i);
+  d.ys[p][i] = v;
+  y[d.off[p] + d.perm[p][i]] = v;
 }
 
 // ------------------------------------------------ persistent sweeps
@@ -241,6 +243,14 @@ void record(SetPlan& sp, cudaStream_t s) {
   k_set_gather<<<nb(sp.gather.total, 256), 256, 0, s>>>(sp.dev, sp.gather, sp.q);
   AFMM_LAUNCH_CHECK();
   ++n;
+  // the near field beside the far field (lower-priority branch)
+  AFMM_CUDA(cudaEventRecord(sp.ev_q, s));
+  AFMM_CUDA(cudaStreamWaitEvent(sp.s_near, sp.ev_q, 0));
+  AFMM_CUDA(cudaEventRecordWithFlags(sp.near_mark[0], sp.s_near, cudaEventRecordExternal));
+  kernel_table(sp.kernel_id).set_p2p_run(sp, sp.s_near);
+  AFMM_CUDA(cudaEventRecordWithFlags(sp.near_mark[1], sp.s_near, cudaEventRecordExternal));
+  AFMM_CUDA(cudaEventRecord(sp.ev_near, sp.s_near));
+  ++n;
   mark("m2m");
   if (sp.up.nitems > 0) {
     k_set_up<<<sp.up.grid, kSweepTile, 0, s>>>(sp.dev, sp.up, sp.sync);
@@ -259,9 +269,8 @@ void record(SetPlan& sp, cudaStream_t s) {
     AFMM_LAUNCH_CHECK();
     ++n;
   }
-  mark("p2p");
-  kernel_table(sp.kernel_id).set_p2p_run(sp, s);
-  ++n;
+  mark("p2p");  // the wait for the near field's end
+  AFMM_CUDA(cudaStreamWaitEvent(s, sp.ev_near, 0));
   mark("scatter");
   k_set_scatter<<<nb(sp.gather.total, 256), 256, 0, s>>>(sp.dev, sp.gather, sp.y);
   AFMM_LAUNCH_CHECK();
@@ -273,12 +282,12 @@ void record(SetPlan& sp, cudaStream_t s) {
 
 }  // namespace
 
-void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& arena, cudaStream_t s) {
+void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevArena& arena, cudaStream_t s) {
   const int np = (int)probs.size();
   std::vector<LevelView> lv((size_t)np * kMaxLevels);
   std::vector<NearView> nv(np);
   std::vector<KernelParams> kp(np);
-  std::vector<int2> shape(np);
+  std::vector<int> warps(np);
   std::vector<const int64_t*> perm(np);
   std::vector<double*> qs(np), ys(np);
   std::vector<int64_t> off(np + 1, 0);
@@ -287,11 +296,11 @@ void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& aren
   sp.p2p_threads = 0;
   sp.p2p_smem = 0;
   for (int p = 0; p < np; ++p) {
-    const MatvecPlan& mp = *probs[p].plan;
+    const MatvecPlan& mp = *probs[p];
     for (int j = 0; j <= mp.L; ++j) lv[(size_t)p * kMaxLevels + j] = mp.lv[j];
     nv[p] = mp.near;
     kp[p] = mp.kp;
-    shape[p] = make_int2(probs[p].shape.nt, probs[p].shape.g);
+    warps[p] = near_warps(mp.near.nmax);
     perm[p] = mp.perm;
     qs[p] = mp.qs;
     ys[p] = mp.ys;
@@ -300,9 +309,8 @@ void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& aren
     for (int j = 2; j <= mp.L; ++j) m2l.add(p, j, mp.lv[j].nrows);
     p2p.add(p, mp.L, mp.near.nleaf);
     maxL = std::max(maxL, mp.L);
-    sp.p2p_threads = std::max(sp.p2p_threads, probs[p].shape.threads);
-    sp.p2p_smem = std::max(sp.p2p_smem, (size_t)9 * mp.near.nmax * (sizeof(double2) + sizeof(double)) +
-                                            sizeof(double) * probs[p].shape.threads);
+    sp.p2p_threads = std::max(sp.p2p_threads, 32 * warps[p]);
+    sp.p2p_smem = std::max(sp.p2p_smem, near_smem(mp.near.nmax, warps[p]));
   }
   // M2M by depth below the leaf level; L2L by level from the top; each
   // sweep's items are the depth tables' row tiles in that order
@@ -319,7 +327,7 @@ void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& aren
   for (int depth = 0; depth + 2 <= maxL; ++depth) {
     SegBuilder b;
     for (int p = 0; p < np; ++p) {
-      const MatvecPlan& mp = *probs[p].plan;
+      const MatvecPlan& mp = *probs[p];
       const int j = mp.L - depth;
       if (j >= 2) b.add(p, j, mp.lv[j].nrows);
     }
@@ -331,7 +339,7 @@ void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& aren
   for (int j = 2; j <= maxL; ++j) {
     SegBuilder b;
     for (int p = 0; p < np; ++p) {
-      const MatvecPlan& mp = *probs[p].plan;
+      const MatvecPlan& mp = *probs[p];
       if (j <= mp.L) b.add(p, j, mp.lv[j].nnodes);
     }
     if (b.first.back() > 0) {
@@ -371,7 +379,7 @@ void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& aren
   sp.dev.lv = upload(lv, arena, s);
   sp.dev.nv = upload(nv, arena, s);
   sp.dev.kp = upload(kp, arena, s);
-  sp.dev.p2p = upload(shape, arena, s);
+  sp.dev.p2p_warps = upload(warps, arena, s);
   sp.dev.perm = upload(perm, arena, s);
   sp.dev.qs = upload(qs, arena, s);
   sp.dev.ys = upload(ys, arena, s);
@@ -380,6 +388,12 @@ void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& aren
   sp.q = arena.alloc<double>(off[np]);
   sp.y = arena.alloc<double>(off[np]);
   AFMM_CUDA(cudaStreamSynchronize(s));
+  int least = 0, greatest = 0;
+  AFMM_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  AFMM_CUDA(cudaStreamCreateWithPriority(&sp.s_near, cudaStreamNonBlocking, least));
+  AFMM_CUDA(cudaEventCreateWithFlags(&sp.ev_q, cudaEventDisableTiming));
+  AFMM_CUDA(cudaEventCreateWithFlags(&sp.ev_near, cudaEventDisableTiming));
+  for (cudaEvent_t& e : sp.near_mark) AFMM_CUDA(cudaEventCreate(&e));
   // kernel attributes are set before capture; then the graph is recorded once
   kernel_table(sp.kernel_id).set_p2p_prepare(sp.p2p_smem);
   set_recapture(sp, s);
@@ -413,6 +427,9 @@ void set_stage_times(const SetPlan& sp, std::vector<std::pair<std::string, doubl
     AFMM_CUDA(cudaEventElapsedTime(&ms, sp.marks[i].second, sp.marks[i + 1].second));
     out.push_back({sp.marks[i].first, ms});
   }
+  float ms = 0;
+  AFMM_CUDA(cudaEventElapsedTime(&ms, sp.near_mark[0], sp.near_mark[1]));
+  out.push_back({"p2p_kernel", ms});
 }
 
 void set_release(SetPlan& sp) {
@@ -421,6 +438,12 @@ void set_release(SetPlan& sp) {
   if (sp.exec) cudaGraphExecDestroy(sp.exec);
   if (sp.graph) cudaGraphDestroy(sp.graph);
   for (auto& m : sp.marks) cudaEventDestroy(m.second);
+  for (cudaEvent_t* e : {&sp.ev_q, &sp.ev_near, &sp.near_mark[0], &sp.near_mark[1]}) {
+    if (*e) cudaEventDestroy(*e);
+    *e = nullptr;
+  }
+  if (sp.s_near) cudaStreamDestroy(sp.s_near);
+  sp.s_near = nullptr;
   sp.marks.clear();
   sp.exec = nullptr;
   sp.graph = nullptr;

@@ -14,7 +14,7 @@ struct SetDev {
   const LevelView* lv = nullptr;    // nprob x kMaxLevels, level j of problem p at p*kMaxLevels + j
   const NearView* nv = nullptr;     // nprob
   const KernelParams* kp = nullptr; // nprob
-  const int2* p2p = nullptr;        // nprob: near-field launch shape (NT, G)
+  const int* p2p_warps = nullptr;   // nprob: warps of the near field's CTAs
   const int64_t* const* perm = nullptr;  // nprob: sorted -> original index
   double* const* qs = nullptr;      // nprob: sorted charges
   double* const* ys = nullptr;      // nprob: sorted potentials
@@ -41,12 +41,6 @@ __device__ __forceinline__ int seg_of(const SetSegs& sg, long g) {
   }
   return lo;
 }
-
-// Host description of one problem of the set.
-struct SetProblem {
-  const MatvecPlan* plan;
-  P2pShape shape;
-};
 
 // A persistent sweep (every level of every problem in one launch): items are
 // tiles of kSweepTile rows of one depth's flat row space (segs[depth]), listed
@@ -89,13 +83,17 @@ struct SetPlan {
   int launches_per_matvec = 0;
   // events recorded inside the graph between stages (per-stage device time)
   std::vector<std::pair<std::string, cudaEvent_t>> marks;
+  // the near field runs on this lower-priority stream beside the far field
+  // (a parallel branch of the graph); near_mark times it
+  cudaStream_t s_near = nullptr;
+  cudaEvent_t ev_q = nullptr, ev_near = nullptr, near_mark[2] = {nullptr, nullptr};
 };
 
 // Per-stage milliseconds of the last replay, accumulated by stage name.
 void set_stage_times(const SetPlan& sp, std::vector<std::pair<std::string, double>>& out);
 
 // Builds the device tables (allocated from `arena`) and the graph on stream s.
-void set_build(SetPlan& sp, const std::vector<SetProblem>& probs, DevArena& arena, cudaStream_t s);
+void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevArena& arena, cudaStream_t s);
 // One FP64 matvec of every problem: sp.q -> sp.y (graph replay on s).  After
 // the stream completes, *sp.h_err is nonzero if a sweep's bounded wait gave up.
 void set_matvec(SetPlan& sp, cudaStream_t s);

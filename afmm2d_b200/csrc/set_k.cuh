@@ -8,16 +8,17 @@ namespace afmm {
 
 namespace set_detail {
 
-// Near field: one CTA per leaf of every problem, each problem with its own
-// (NT, G) shape so the group sums add in the same order as its own launch.
+// Near field: one CTA per leaf of every problem, each problem with the number
+// of warps of its own launch, so the warps' sums add in the same order.
 template <class K>
-__global__ void k_set_p2p64(SetDev d, SetSegs sg) {
+__global__ void __launch_bounds__(256, 3) k_set_p2p64(SetDev d, SetSegs sg) {
   extern __shared__ __align__(16) unsigned char smem[];
   const long g = blockIdx.x;
   const int s = seg_of(sg, g);
   const int p = sg.prob[s];
-  const int2 sh = d.p2p[p];
-  p2p64_leaf<K>(d.nv[p], d.kp[p], d.qs[p], d.ys[p], sh.x, sh.y, g - sg.first[s], smem);
+  const NearView nv = d.nv[p];
+  const KernelParams kp = d.kp[p];
+  near_leaf<K>(nv, kp, d.qs[p], d.p2p_warps[p], g - sg.first[s], smem);
 }
 
 template <class K>

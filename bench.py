@@ -620,7 +620,7 @@ def run_many(args):
     hbm, _, peak_kind = load_peaks()
     fp64_peak, _ = A.measure_fma_peaks()
     dom = max(stages, key=lambda k: stages[k])
-    if dom == "p2p":
+    if dom in ("p2p", "p2p_kernel"):
         flops = 8.0 * cnt["near_evals"]
         roof = {"bound": "fp64", "kernel": "k_set_p2p64 (near field, FP64 kernel entries)", "unit": "TFLOP/s",
                 "achieved": flops / (stages[dom] * 1e-3) / 1e12, "peak": fp64_peak,

@@ -381,3 +381,22 @@ def test_m2l_on_the_fly_matches_stored_blocks(kernel):
         A.AFMMSet([ot])
     with pytest.raises(A.AFMMError):
         st.set_m2l_storage("auto")  # after assemble
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel,N,M", [("log", 17, 1), ("one_over_r", 130, 2), ("gaussian", 600, 9), ("log", 500, 31),
+                                        ("one_over_r_scaled", 512, 32), ("one_over_r", 531, 33), ("log", 1600, 80),
+                                        ("one_over_r_scaled", 6250, 101), ("gaussian", 16380, 300)])
+def test_pairwise_near_field_leaf_sizes(kernel, N, M):
+    """The one-column FP64 near field (every pair of leaves evaluated once, in one of the two) against the
+    FP64 tensor-tile near field of the batched passes (both directions), at leaves of 1 to 1,024 points: below,
+    at and above a warp, and of uneven sizes.  Only the summation order differs: the bound of the batched
+    passes' own test."""
+    rng = np.random.default_rng(N)
+    a = A.AFMM(N, M, 6, rng.uniform(0, 1, (N, 2)), kernel=kernel, kparam=0.01 if kernel == "gaussian" else None)
+    a.assemble()
+    Q = rng.standard_normal((N, 3))
+    Yb = a.computeMatVecProduct(Q, precision="fp64_batched")
+    for c in range(3):
+        y = a.computeMatVecProduct(Q[:, c])
+        assert np.linalg.norm(y - Yb[:, c]) <= FP64_BATCHED_TOL * np.linalg.norm(y)
