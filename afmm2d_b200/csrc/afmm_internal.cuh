@@ -317,6 +317,11 @@ struct LevelDev {
   int64_t* qs_sum = nullptr;
   double* qhat = nullptr;       // outgoing charges, skel_off layout
   double* yhat = nullptr;       // incoming potentials, skel_off layout
+  struct ForwardBox* fwd = nullptr;  // one-column M2L (fmm.cuh): per box its forward columns,
+  double* back = nullptr;            // their sums, box b's from back_off[b] on,
+  int64_t* back_off = nullptr;
+  int64_t* back_src = nullptr;       // and where a box finds its own among them
+  int32_t* m2l_run = nullptr;   // boxes of the one-column M2L of a shard
   // host copies
   std::vector<int32_t> h_rank, h_skel_off;
   std::vector<int32_t> h_node_off;

@@ -315,14 +315,31 @@ void apply_shard(afmm_handle* h) {
     if (j >= 2) {
       LevelView m = p.lv[j];
       narrow_table(m.cgrp_box, m.cgrp_row, m.ncgroups, bl, bh);
-      narrow_table(m.wgrp_box, m.wgrp_row, m.nwgroups, bl, bh);
+      // the one-column M2L works a pair of boxes out in the one that has the
+      // other in a forward slot: the shard runs its own boxes and those with
+      // one of them there
+      const std::vector<int32_t>& il = h->h_il[j];
+      std::vector<int32_t> run;
+      for (long b = 0; b < m.nbox; ++b) {
+        bool on = b >= bl && b < bh;
+        for (int f = 0; f < kForwardSlots; ++f) {
+          const int32_t c = il[b * 40 + forward_slot(f)];
+          on = on || (c >= bl && c < bh);
+        }
+        if (on) run.push_back((int32_t)b);
+      }
+      LevelDev& dev = h->lv[j];
+      if (!dev.m2l_run) dev.m2l_run = h->arena.alloc<int32_t>(m.nbox);
+      AFMM_CUDA(cudaMemcpy(dev.m2l_run, run.data(), sizeof(int32_t) * run.size(), cudaMemcpyHostToDevice));
+      m.m2l_run = dev.m2l_run;
+      m.nm2l_run = (long)run.size();
       p.levels_m2l.lv[j - 2] = m;
     }
   }
   LevelSet& ls = p.levels_m2l;
   for (int t = 0; t < ls.nlev; ++t) {
     ls.cgrp0[t + 1] = ls.cgrp0[t] + ls.lv[t].ncgroups;
-    ls.wgrp0[t + 1] = ls.wgrp0[t] + ls.lv[t].nwgroups;
+    ls.m0[t + 1] = ls.m0[t] + (ls.lv[t].m2l_run ? ls.lv[t].nm2l_run : ls.lv[t].nbox);
   }
   const long sl = 1L << (2 * (h->L - lev));
   p.near_own.leaf0 = k0 * sl;
@@ -376,6 +393,10 @@ void build_plan(afmm_handle* h) {
     v.skel_xy = d.skel_xy;
     v.qhat = d.qhat;
     v.yhat = d.yhat;
+    v.fwd = d.fwd;
+    v.back = d.back;
+    v.back_off = d.back_off;
+    v.back_src = d.back_src;
     v.skel_box = d.skel_box;
     v.node_box = d.node_box;
     v.grp_box = d.grp_box;
@@ -414,20 +435,20 @@ void build_plan(afmm_handle* h) {
   p.levels.row0[0] = 0;
   p.levels.grp0[0] = 0;
   p.levels.cgrp0[0] = 0;
-  p.levels.wgrp0[0] = 0;
   p.levels.pt0[0] = 0;
   p.levels.t0[0] = 0;
   p.levels.b0[0] = 0;
+  p.levels.m0[0] = 0;
   for (int j = 2; j <= h->L; ++j) {
     p.levels.lv[p.levels.nlev] = p.lv[j];
     p.levels.src[p.levels.nlev] = p.levels.nlev;
     p.levels.row0[p.levels.nlev + 1] = p.levels.row0[p.levels.nlev] + p.lv[j].nrows;
     p.levels.grp0[p.levels.nlev + 1] = p.levels.grp0[p.levels.nlev] + p.lv[j].ngroups;
     p.levels.cgrp0[p.levels.nlev + 1] = p.levels.cgrp0[p.levels.nlev] + p.lv[j].ncgroups;
-    p.levels.wgrp0[p.levels.nlev + 1] = p.levels.wgrp0[p.levels.nlev] + p.lv[j].nwgroups;
     p.levels.pt0[p.levels.nlev + 1] = p.levels.pt0[p.levels.nlev] + p.lv[j].nptiles;
     p.levels.t0[p.levels.nlev + 1] = p.levels.t0[p.levels.nlev] + p.lv[j].ntiles;
     p.levels.b0[p.levels.nlev + 1] = p.levels.b0[p.levels.nlev] + p.lv[j].nbox;
+    p.levels.m0[p.levels.nlev + 1] = p.levels.m0[p.levels.nlev] + p.lv[j].nbox;
     ++p.levels.nlev;
   }
   for (int j = 0; j <= h->L; ++j) {
@@ -707,17 +728,22 @@ void finish_assemble(afmm_handle* h) {
   // M2L blocks, levels 2..L: sizes first, then the storage decision
   const double t_tab = now_s();
   int64_t m2l_total = 0, l2p_total = 0, rows_total = 0;
+  std::vector<std::vector<int64_t>> back_off(L + 1);  // one-column M2L: sums of the forward columns
   for (int j = 2; j <= L; ++j) {
     LevelDev& v = h->lv[j];
     const std::vector<int32_t>& il = h->h_il[j];
     v.h_m2l_off.assign(v.nbox + 1, 0);
+    back_off[j].assign(v.nbox + 1, 0);
     for (long b = 0; b < v.nbox; ++b) {
-      int64_t e = 0;
+      int64_t e = 0, f = 0;
       for (int t = 0; t < 40; ++t) {
         int c = il[b * 40 + t];
-        if (c >= 0) e += (int64_t)v.h_rank[b] * v.h_rank[c];
+        if (c < 0) continue;
+        e += v.h_rank[c];
+        if (t < 8 || (t >= 16 && t < 28)) f += v.h_rank[c];
       }
-      v.h_m2l_off[b + 1] = v.h_m2l_off[b] + e;
+      v.h_m2l_off[b + 1] = v.h_m2l_off[b] + e * v.h_rank[b];
+      back_off[j][b + 1] = back_off[j][b] + f;
     }
     m2l_total += v.h_m2l_off[v.nbox];
     l2p_total += v.h_l2p_off[v.nbox];
@@ -745,6 +771,11 @@ void finish_assemble(afmm_handle* h) {
     h->setup_phase[5].second += now_s() - t_al;
     v.qhat = h->arena.alloc<double>(v.total_rank + 2);  // + 16 B: whole-piece L2 prefetches
     v.yhat = h->arena.alloc<double>(v.total_rank);
+    v.fwd = h->arena.alloc<ForwardBox>(v.nbox);
+    v.back = h->arena.alloc<double>(back_off[j][v.nbox]);
+    v.back_off = h->arena.alloc<int64_t>(v.nbox + 1);
+    v.back_src = h->arena.alloc<int64_t>((size_t)v.nbox * kForwardSlots);
+    AFMM_CUDA(cudaMemcpyAsync(v.back_off, back_off[j].data(), sizeof(int64_t) * (v.nbox + 1), cudaMemcpyHostToDevice, s));
     // row -> box maps for the thread-per-row sweeps
     v.skel_box = h->arena.alloc<int32_t>(v.total_rank);
     v.node_box = h->arena.alloc<int32_t>(v.h_node_off[v.nbox]);
@@ -877,7 +908,8 @@ void finish_assemble(afmm_handle* h) {
   t_ph = now_s();
   for (int j = 2; j <= L; ++j) {
     l2p_transpose(h->plan.lv[j], h->lv[j].l2p, h->lv[j].l2p_rm, s);
-    ++h->launches;
+    forward_boxes(h->plan.lv[j], s);
+    h->launches += 3;
   }
   mixed_setup(h->plan, h->lv, h->mixed, h->arena, s, &h->launches);
   build_plan(h);

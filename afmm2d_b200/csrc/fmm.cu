@@ -203,86 +203,52 @@ void l2p_transpose(const LevelView& v, const double* cm, double* rm, cudaStream_
   AFMM_LAUNCH_CHECK();
 }
 
-// Level of flat warp chunk g of a LevelSet (wgrp0: prefix of chunk counts).
-__device__ __forceinline__ int level_of_wchunk(const LevelSet& ls, long g) {
+// One-column M2L of every level in one launch, one CTA per box (m2l_pair_box,
+// fmm.cuh: every unordered pair of boxes once), the upper levels' boxes with
+// their larger ranks first.  1,048,576 uniform points, log, TOL 10 (2.3 GB of
+// blocks): 0.95 ms with every block read by a warp per 32 rows -> 0.55, 4.2 TB/s
+// of the 6.5 measured (fixed point 0.48); a third of a CTA's time is the latency
+// of its tables and charges.  Two warps a box instead of four: 0.57, and 26
+// instead of 19 us at 4,096 points; copies through shared memory (cp.async)
+// instead of registers: 0.67.
+template <bool Q32>
+__global__ void __launch_bounds__(32 * kPairWarps, 6) k_m2l_pair(LevelSet ls) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const long g = blockIdx.x;
   int j = 0;
-  while (j + 1 < ls.nlev && g >= ls.wgrp0[j + 1]) ++j;
-  return j;
+  while (j + 1 < ls.nlev && g >= ls.m0[j + 1]) ++j;
+  const LevelView& v = ls.lv[j];
+  const long t = g - ls.m0[j];
+  m2l_pair_box<Q32>(v, v.m2l_run ? (long)v.m2l_run[t] : t, ls.pf_ahead, smem);
 }
 
-// M2L (src/AFMM2DTree.cpp:1156-1178) for every level in one launch, one warp
-// per chunk of up to 32 skeleton rows of one box, lane = row.  Each row's
-// arithmetic is m2l_row's (slots in the reference's order, four partial sums
-// per block), so the result has the same bits as the thread-per-row form; the
-// warp's loads of one block column are contiguous, every lane of a warp
-// takes the same slots, and the box's block region is streamed into L2 ahead
-// of the loads.  Q32: the 32-bit fixed-point blocks (decode_q32) instead of
-// the FP64 ones (the single-RHS mixed path).
-template <bool Q32>
-__global__ void __launch_bounds__(128) k_m2l_apply_w(LevelSet ls) {
-  const long gw = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= ls.wgrp0[ls.nlev]) return;  // whole warps only
-  const int j = level_of_wchunk(ls, gw);
-  const LevelView& v = ls.lv[j];
-  const long g = gw - ls.wgrp0[j];
-  const int b = v.wgrp_box[g];
-  const int r0 = v.wgrp_row[g];
-  const int box_end = v.skel_off[b] + v.rank[b];
-  const int next = g + 1 < v.nwgroups ? min(box_end, v.wgrp_row[g + 1]) : box_end;
-  const int r = v.rank[b];
-  const int i = r0 - v.skel_off[b] + lane;
-  const bool act = lane < next - r0;
-  // slot table: lane l holds slot l (and slot 32 + l for l < 8)
-  const int sa = v.il[(long)b * 40 + lane];
-  const int sb = lane < 8 ? v.il[(long)b * 40 + 32 + lane] : -1;
-  const int ra = sa >= 0 ? v.rank[sa] : 0, rb = sb >= 0 ? v.rank[sb] : 0;
-  const int oa = sa >= 0 ? v.skel_off[sa] : 0, ob = sb >= 0 ? v.skel_off[sb] : 0;
-  const long base = v.m2l_off[b];
-  const long stop = v.m2l_off[b + 1];
-  long pos = base;  // first entry of the current slot's block
-  L2Stream pf(Q32 ? (const void*)(v.m2l_q + base) : (const void*)(v.m2l + base),
-              Q32 ? (const void*)(v.m2l_q + stop) : (const void*)(v.m2l + stop), ls.pf_ahead);
-  double acc = 0.0;
-  for (int s = 0; s < 40; ++s) {
-    const int rc = __shfl_sync(0xffffffffu, s < 32 ? ra : rb, s & 31);
-    if (rc == 0) continue;  // empty slot or rank-0 box: no block stored
-    const int sc = __shfl_sync(0xffffffffu, s < 32 ? oa : ob, s & 31);
-    const double* qc = v.qhat + sc;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    int cc = 0;
-    if (Q32) {
-      const double2 dec = v.m2l_dec[(long)b * 40 + s];
-      pf.advance(v.m2l_q + pos, lane);
-      const uint32_t* M = v.m2l_q + pos + i;
-#define AFMM_ENT(c) (act ? decode_q32(M[(long)(c) * r], dec) : 0.0)
-#pragma unroll 2
-      for (; cc + 3 < rc; cc += 4) {
-        a0 += AFMM_ENT(cc) * qc[cc];
-        a1 += AFMM_ENT(cc + 1) * qc[cc + 1];
-        a2 += AFMM_ENT(cc + 2) * qc[cc + 2];
-        a3 += AFMM_ENT(cc + 3) * qc[cc + 3];
-      }
-      for (; cc < rc; ++cc) a0 += AFMM_ENT(cc) * qc[cc];
-#undef AFMM_ENT
-    } else {
-      pf.advance(v.m2l + pos, lane);
-      const double* M = v.m2l + pos + i;
-#define AFMM_ENT(c) (act ? M[(long)(c) * r] : 0.0)
-#pragma unroll 2
-      for (; cc + 3 < rc; cc += 4) {
-        a0 += AFMM_ENT(cc) * qc[cc];
-        a1 += AFMM_ENT(cc + 1) * qc[cc + 1];
-        a2 += AFMM_ENT(cc + 2) * qc[cc + 2];
-        a3 += AFMM_ENT(cc + 3) * qc[cc + 3];
-      }
-      for (; cc < rc; ++cc) a0 += AFMM_ENT(cc) * qc[cc];
-#undef AFMM_ENT
-    }
-    acc += (a0 + a1) + (a2 + a3);
-    pos += (long)r * rc;
-  }
-  if (act) v.yhat[r0 + lane] = acc;
+__global__ void __launch_bounds__(128) k_forward_boxes(LevelView v) {
+  const long b = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (b < v.nbox) v.fwd[b].make(v, b, threadIdx.x & 31);
+}
+
+__global__ void __launch_bounds__(128) k_back_src(LevelView v) {
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= v.nbox * kForwardSlots) return;
+  const int f = (int)(t % kForwardSlots);
+  const int c = v.il[t / kForwardSlots * 40 + backward_slot(f)];
+  v.back_src[t] = c >= 0 && v.rank[c] > 0 ? v.fwd[c].sums + v.fwd[c].col[f] : -1;
+}
+
+void forward_boxes(const LevelView& v, cudaStream_t s) {
+  k_forward_boxes<<<(int)((v.nbox * 32 + 127) / 128), 128, 0, s>>>(v);
+  AFMM_LAUNCH_CHECK();
+  k_back_src<<<(int)((v.nbox * kForwardSlots + 127) / 128), 128, 0, s>>>(v);
+  AFMM_LAUNCH_CHECK();
+}
+
+// The sums that other boxes worked out, added to every level's rows.
+__global__ void __launch_bounds__(256) k_m2l_back(LevelSet ls) {
+  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= ls.row0[ls.nlev]) return;
+  int j = 0;
+  while (j + 1 < ls.nlev && g >= ls.row0[j + 1]) ++j;
+  m2l_back_row(ls.lv[j], g - ls.row0[j]);
 }
 
 // End of warp chunk g of a chunk table (the next chunk's first row, or the
@@ -344,30 +310,33 @@ void sweep_l2l(const MatvecPlan& p, double* ys, cudaStream_t s, int64_t* launche
   }
 }
 
-void m2l_apply(const MatvecPlan& p, cudaStream_t s) {
-  const long rows = p.levels.row0[p.levels.nlev];
-  if (rows == 0) return;
-  if (p.levels.lv[0].m2l == nullptr) {  // blocks not stored: entries on the fly
-    m2l_apply_otf(p, p.levels, s);
-    return;
-  }
-  LevelSet ls = p.levels_m2l;  // a shard's boxes at the sharded levels
-  ls.pf_ahead = p.tune.pf_fp64;
-  const long warps = ls.wgrp0[ls.nlev];
-  k_m2l_apply_w<false><<<(int)((warps * 32 + 127) / 128), 128, 0, s>>>(ls);
+int m2l_back(const LevelSet& ls, cudaStream_t s) {
+  const long rows = ls.row0[ls.nlev];
+  k_m2l_back<<<(int)((rows + 255) / 256), 256, 0, s>>>(ls);
   AFMM_LAUNCH_CHECK();
+  return 1;
 }
 
-void m2l_apply_stored(const MatvecPlan& p, const LevelSet& levels, bool q32, cudaStream_t s) {
+int m2l_apply(const MatvecPlan& p, cudaStream_t s) {
+  const long rows = p.levels.row0[p.levels.nlev];
+  if (rows == 0) return 0;
+  if (p.levels.lv[0].m2l == nullptr) return m2l_apply_otf(p, p.levels, s);  // blocks not stored: entries on the fly
+  return m2l_apply_stored(p, p.levels_m2l, false, s);  // a shard's boxes at the sharded levels
+}
+
+int m2l_apply_stored(const MatvecPlan& p, const LevelSet& levels, bool q32, cudaStream_t s) {
   LevelSet ls = levels;
   ls.pf_ahead = p.tune.pf_fp64;
-  const long warps = ls.wgrp0[ls.nlev];
-  if (warps == 0) return;
+  const long boxes = ls.m0[ls.nlev];
+  if (boxes == 0 || ls.row0[ls.nlev] == 0) return 0;
   if (q32 && ls.lv[0].m2l_q == nullptr) throw Error{AFMM_BAD_ARG, "no fixed-point M2L blocks stored"};
   if (!q32 && ls.lv[0].m2l == nullptr) throw Error{AFMM_BAD_ARG, "no M2L blocks stored"};
-  if (q32) k_m2l_apply_w<true><<<(int)((warps * 32 + 127) / 128), 128, 0, s>>>(ls);
-  else k_m2l_apply_w<false><<<(int)((warps * 32 + 127) / 128), 128, 0, s>>>(ls);
+  const size_t smem = m2l_pair_smem(*std::max_element(p.rmax, p.rmax + kMaxLevels));
+  auto fn = q32 ? k_m2l_pair<true> : k_m2l_pair<false>;
+  allow_smem(fn, smem);
+  fn<<<(int)boxes, 32 * kPairWarps, smem, s>>>(ls);
   AFMM_LAUNCH_CHECK();
+  return 1 + m2l_back(ls, s);
 }
 
 void matvec_fp64(const MatvecPlan& p, const double* q, double* y, cudaStream_t s, StageTimer* tm, int64_t* launches) {
@@ -393,8 +362,7 @@ void matvec_fp64(const MatvecPlan& p, const double* q, double* y, cudaStream_t s
   if (tm) tm->mark(s, "m2m");
   sweep_m2m(p, p.qs, s, launches);
   if (tm) tm->mark(s, "m2l");
-  m2l_apply(p, s);
-  ++*launches;
+  *launches += m2l_apply(p, s);
   if (tm) tm->mark(s, "l2l");
   sweep_l2l(p, p.ys, s, launches);
   if (tm) tm->mark(s, "p2p");

@@ -12,10 +12,11 @@ namespace afmm {
 
 constexpr int kMaxLevels = 16;
 
-// Allows `bytes` of dynamic shared memory for kernel `fn` (needed above 48 KB).
+// Allows `bytes` of dynamic shared memory for kernel `fn` (needed above 48 KB
+// with the kernel's static shared memory, a few KB at most).
 template <class F>
 inline void allow_smem(F* fn, size_t bytes) {
-  if (bytes > 48 * 1024) {
+  if (bytes > 40 * 1024) {
     if (bytes > 227 * 1024) throw Error{AFMM_BAD_ARG, "per-box rank too large for the sweep kernels"};
     AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   }
@@ -68,6 +69,16 @@ struct LevelView {
   int64_t* qs_sum = nullptr;
   uint32_t* m2l_q = nullptr;          // 32-bit fixed-point blocks (null when not stored)
   double2* m2l_dec = nullptr;         // per (box, slot) decode constants
+  // one-column M2L (m2l_pair_box): per box its forward columns, the columns'
+  // sums (box b's from back_off[b] on) and where a box finds its own among
+  // them (kForwardSlots per box, -1 = none); the boxes to run for a shard
+  // (null: all)
+  struct ForwardBox* fwd = nullptr;
+  double* back = nullptr;
+  const int64_t* back_off = nullptr;
+  int64_t* back_src = nullptr;
+  const int32_t* m2l_run = nullptr;
+  long nm2l_run = 0;
   long nrows = 0;                     // skeleton rows (sum of ranks)
   long nnodes = 0;                    // node rows (sum of node counts)
 };
@@ -80,10 +91,10 @@ struct LevelSet {
   long row0[kMaxLevels + 1] = {0};
   long grp0[kMaxLevels + 1] = {0};   // prefix of row-group counts
   long cgrp0[kMaxLevels + 1] = {0};  // prefix of row-chunk counts
-  long wgrp0[kMaxLevels + 1] = {0};  // prefix of warp row-chunk counts
   long pt0[kMaxLevels + 1] = {0};    // prefix of parent row-tile counts
   long t0[kMaxLevels + 1] = {0};     // prefix of 128-row tile counts
   long b0[kMaxLevels + 1] = {0};     // prefix of box counts
+  long m0[kMaxLevels + 1] = {0};     // prefix of the boxes that the one-column M2L runs (a shard's, else all)
   int src[kMaxLevels] = {0};         // index of entry j among levels 2..L (per-level device tables)
   uint32_t pf_ahead = 12 * 1024;     // L2 prefetch window of the stored-block M2L kernels (bytes)
 };
@@ -101,10 +112,10 @@ inline LevelSet level_subset(const LevelSet& ls, uint32_t mask, bool keep) {
     o.row0[n + 1] = o.row0[n] + (ls.row0[t + 1] - ls.row0[t]);
     o.grp0[n + 1] = o.grp0[n] + (ls.grp0[t + 1] - ls.grp0[t]);
     o.cgrp0[n + 1] = o.cgrp0[n] + (ls.cgrp0[t + 1] - ls.cgrp0[t]);
-    o.wgrp0[n + 1] = o.wgrp0[n] + (ls.wgrp0[t + 1] - ls.wgrp0[t]);
     o.pt0[n + 1] = o.pt0[n] + (ls.pt0[t + 1] - ls.pt0[t]);
     o.t0[n + 1] = o.t0[n] + (ls.t0[t + 1] - ls.t0[t]);
     o.b0[n + 1] = o.b0[n] + (ls.b0[t + 1] - ls.b0[t]);
+    o.m0[n + 1] = o.m0[n] + (ls.m0[t + 1] - ls.m0[t]);
     ++o.nlev;
   }
   return o;
@@ -374,25 +385,16 @@ inline int near_warps(int nmax) {
   }
   return best;
 }
-// Targets that a warp goes round: n, or (leaves below 32 points) the next
-// power of two, with the lanes in groups of that many.
-__host__ __device__ __forceinline__ int near_ring(int n) {
-  if (n >= 32) return n;
-  int r = 1;
-  while (r < n) r *= 2;
-  return r;
-}
-// The leaf's points and charges are repeated behind their end, and a warp's
-// row of target sums is as long, so that no lane's index wraps.
-__host__ __device__ __forceinline__ int near_row(int n) { return (n < 32 ? 32 : n) + 32; }
+// A warp goes round the n targets, lane l from target l on; with fewer than 32
+// the lanes go round in groups of n, each group with target sums of its own.
+// The targets are repeated behind their end, and a row of target sums is as
+// long, so that no lane's index wraps.
+__host__ __device__ __forceinline__ int near_row(int n) { return n >= 32 ? n + 32 : 2 * n * ((31 + n) / n); }
+constexpr int kNearRowMax = 128;  // of n < 32
 inline size_t near_smem(int nmax, int warps) {
-  const size_t row = near_row(nmax);
+  const size_t row = std::max(near_row(nmax), kNearRowMax);
   return row * (sizeof(double2) + sizeof(double)) + nmax * sizeof(double) + (size_t)warps * row * sizeof(double);
 }
-// Stand-in coordinates of padded points (finite entries for every kernel,
-// their results are not used).
-constexpr double kPadPoint = 1.0e100;
-
 // ------------------------------------------------ FP64 sweep rows
 // The arithmetic of one output of each FP64 sweep, shared by the
 // single-problem kernels (fmm.cu) and the fused many-problem kernels (set.cu)
@@ -432,33 +434,253 @@ __device__ __forceinline__ void m2m_row(const LevelView& v, const double* __rest
   v.qhat[row] = (a0 + a1) + (a2 + a3);
 }
 
-// M2L (src/AFMM2DTree.cpp:1156-1178): row i of box b sums, slot by slot in
-// the reference's order (inner 0..15, outer 0..23), row i of the stored block
-// M2L[b][c] (column-major) times the outgoing charges of c.
-__device__ __forceinline__ void m2l_row(const LevelView& v, long row) {
-  const int b = v.skel_box[row];
-  const int r = v.rank[b];
-  const int i = (int)(row - v.skel_off[b]);
-  const double* M = v.m2l + v.m2l_off[b] + i;
-  double acc = 0.0;
-  for (int s = 0; s < 40; ++s) {
-    const int c = v.il[(long)b * 40 + s];
-    if (c < 0) continue;
-    const int rc = v.rank[c];
-    const double* qc = v.qhat + v.skel_off[c];
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    int cc = 0;
-    for (; cc + 3 < rc; cc += 4) {
-      a0 += M[(long)cc * r] * qc[cc];
-      a1 += M[(long)(cc + 1) * r] * qc[cc + 1];
-      a2 += M[(long)(cc + 2) * r] * qc[cc + 2];
-      a3 += M[(long)(cc + 3) * r] * qc[cc + 3];
+// M2L (src/AFMM2DTree.cpp:1156-1178) of one column from the stored blocks,
+// every unordered pair of boxes once: the block of (c, b) is the transpose of
+// that of (b, c), so box b reads its blocks with the boxes in its forward
+// slots (inner 0..7, outer 0..11: the opposites of inner 8..15, outer 12..23)
+// and gives the potentials of both sides: its own rows' to yhat, and those of
+// its forward boxes, one value per column, to v.back, from where m2l_back_row
+// adds them to their rows.  Half the bytes of reading every block.
+constexpr int kForwardSlots = 20;
+__host__ __device__ __forceinline__ int forward_slot(int f) { return f < 8 ? f : 8 + f; }    // f -> slot of the list
+__host__ __device__ __forceinline__ int backward_slot(int f) { return f < 8 ? 8 + f : 20 + f; }  // its opposite
+
+// What the M2L needs of a box in one piece of memory (made at setup): its
+// forward columns -- those before slot f, first skeleton row of slot f's box
+// -- and where the columns' sums go.
+struct ForwardBox {
+  int64_t first;  // of the box's blocks (m2l_off)
+  int64_t sums;   // of its columns in v.back
+  int32_t r, row0;
+  int32_t skip;   // stored columns between the inner and the outer forward blocks
+  int32_t col[kForwardSlots + 1], row[kForwardSlots];
+  // By one warp.
+  __device__ __forceinline__ void make(const LevelView& v, long b, int lane) {
+    const int c = lane < kForwardSlots ? v.il[b * 40 + forward_slot(lane)] : -1;
+    const int d = lane < 8 ? v.il[b * 40 + 8 + lane] : -1;
+    const int rc = c >= 0 ? v.rank[c] : 0;
+    int pre = rc, sk = d >= 0 ? v.rank[d] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, pre, o);
+      if (lane >= o) pre += t;
+      sk += __shfl_xor_sync(0xffffffffu, sk, o);
     }
-    for (; cc < rc; ++cc) a0 += M[(long)cc * r] * qc[cc];
-    acc += (a0 + a1) + (a2 + a3);
-    M += (long)r * rc;
+    if (lane < kForwardSlots) {
+      col[lane] = pre - rc;
+      row[lane] = c >= 0 ? v.skel_off[c] : 0;
+    }
+    if (lane == kForwardSlots) col[kForwardSlots] = pre;
+    if (lane == 0) {
+      first = v.m2l_off[b];
+      sums = v.back_off[b];
+      r = v.rank[b];
+      row0 = v.skel_off[b];
+      skip = sk;
+    }
   }
-  v.yhat[row] = acc;
+  // Slot of column c (< col[kForwardSlots]): the last one that starts at or before c.
+  __device__ __forceinline__ int slot_of(int c) const {
+    int lo = 0, hi = kForwardSlots - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (col[mid] <= c) lo = mid;
+      else hi = mid - 1;
+    }
+    return lo;
+  }
+};
+
+constexpr int kPairWarps = 4;    // warps per box
+constexpr int kPairCols = 128;   // columns a warp stages the charges of at once
+constexpr int kPairRows = 1024;  // rows of a box at once
+inline size_t m2l_pair_smem(int rmax) {
+  return kPairWarps * kPairCols * 2 * sizeof(double) +
+         (size_t)std::min(rmax, kPairRows) * (1 + kPairWarps) * sizeof(double);
+}
+
+// One group of (up to) 32 columns of m2l_pair_panel: P is the entry of the
+// lane's first row in its first column.  Only the last tile can hold rows past
+// the panel's end, and only a tail group columns past the warp's.
+template <bool Q32, int NT, bool FULL>
+__device__ __forceinline__ double m2l_pair_group(const void* __restrict__ P, long r, int left, const double* sq,
+                                                 bool last, const double (&qb)[NT], double (&y)[NT]) {
+  const int lane = threadIdx.x & 31, rsub = lane & 7, csub = lane >> 3;
+  double t[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const bool vc = FULL || 4 * j + csub < left;
+    const double qc = sq[4 * j];  // (zero past the warp's columns)
+    double m[NT];
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+      const bool ok = (FULL || vc) && (k + 1 < NT || last);
+      if (Q32) {
+        const uint32_t u = ok ? __ldg((const uint32_t*)P + 4 * j * r + 8 * k) : 0x80000000u;
+        m[k] = __hiloint2double(0x43300000, (int)u) - 4503601774854144.0;  // u - 2^31, exact
+      } else {
+        m[k] = ok ? __ldg((const double*)P + 4 * j * r + 8 * k) : 0.0;
+      }
+    }
+    t[j] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+      y[k] += m[k] * qc;
+      t[j] += m[k] * qb[k];
+    }
+  }
+  // sum over the eight row lanes; lane rsub keeps column 4 rsub + csub
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int j = 0; j < h; ++j) {
+      const bool up = rsub & h;
+      const double send = up ? t[j] : t[j + h], keep = up ? t[j + h] : t[j];
+      t[j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+    }
+  return t[0];
+}
+
+// A row panel (NT tiles of 8 rows) of `cols` columns stored one after the
+// other from `first` on: lane (rsub, csub) holds rows 8 k + rsub of columns
+// 32 g + 4 j + csub, so that a lane sums its rows of a column and its columns
+// of a row in registers, and 14 shuffles per 32 columns finish the columns'
+// sums.
+template <bool Q32, int NT>
+__device__ __forceinline__ void m2l_pair_panel(const LevelView& v, long first, int r, int i0, int nrow, int cols,
+                                               const double* sq, double* st, const double* sqb, double* yp) {
+  const int lane = threadIdx.x & 31, rsub = lane & 7, csub = lane >> 3;
+  constexpr int E = Q32 ? 4 : 8;
+  double y[NT], qb[NT];
+  const bool last = 8 * (NT - 1) + rsub < nrow;
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    y[k] = 0.0;
+    qb[k] = k + 1 < NT || last ? sqb[i0 + 8 * k + rsub] : 0.0;
+  }
+  const char* P = (Q32 ? (const char*)v.m2l_q : (const char*)v.m2l) + (first + (long)csub * r + i0 + rsub) * E;
+  int cg = 0;
+  for (; cg + 32 <= cols; cg += 32, P += 32l * r * E) {
+    const double t = m2l_pair_group<Q32, NT, true>(P, r, 32, sq + cg + csub, last, qb, y);
+    double* o = st + cg + 4 * rsub + csub;
+    *o = i0 == 0 ? t : *o + t;
+  }
+  if (cg < cols) {
+    const double t = m2l_pair_group<Q32, NT, false>(P, r, cols - cg, sq + cg + csub, last, qb, y);
+    double* o = st + cg + 4 * rsub + csub;
+    if (cg + 4 * rsub + csub < cols) *o = i0 == 0 ? t : *o + t;
+  }
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    y[k] += __shfl_xor_sync(0xffffffffu, y[k], 8);
+    y[k] += __shfl_xor_sync(0xffffffffu, y[k], 16);
+    if ((k + 1 < NT || last) && csub == 0) yp[i0 + 8 * k + rsub] += y[k];
+  }
+}
+
+// One CTA of kPairWarps warps per box, the forward columns shared evenly by
+// the warps, the rows in panels of up to 40; the warps meet only to add their
+// sums of the box's rows (in warp order).  Q32: the 32-bit fixed-point blocks;
+// (u - 2^31) is exact, and the block's power of two goes to the charge of a
+// column and to its sum (both exact).  At its start a warp asks for the first
+// `ahead` bytes of its columns in L2.
+template <bool Q32>
+__device__ __forceinline__ void m2l_pair_box(const LevelView& v, long b, uint32_t ahead, unsigned char* smem) {
+  __shared__ ForwardBox s_fb[kPairWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  ForwardBox& fb = s_fb[warp];
+  for (int i = lane; i < (int)(sizeof(ForwardBox) / 8); i += 32) ((int64_t*)&fb)[i] = ((const int64_t*)(v.fwd + b))[i];
+  __syncwarp();
+  const int r = fb.r;
+  if (r == 0) return;
+  const int C = fb.col[kForwardSlots], ca = fb.col[8];
+  const long gap = (long)fb.skip * r, first = fb.first;
+  const int w0 = (int)((long)warp * C / kPairWarps), w1 = (int)((long)(warp + 1) * C / kPairWarps);
+  if (ahead && lane == 0 && w1 > w0) {
+    const uintptr_t m = Q32 ? (uintptr_t)v.m2l_q : (uintptr_t)v.m2l, E = Q32 ? 4 : 8;
+    const uintptr_t a = (m + (uintptr_t)(first + (long)w0 * r + (w0 >= ca ? gap : 0)) * E) & ~(uintptr_t)15;
+    const uintptr_t n = min((uintptr_t)ahead, ((uintptr_t)(w1 - w0) * r * E + 15) & ~(uintptr_t)15);
+    if (w0 >= ca || w1 <= ca) prefetch_l2_bulk(a, (uint32_t)n);
+  }
+  const int nr = min(r, kPairRows);
+  double* sqb = (double*)smem;        // the box's own charges
+  double* yp = sqb + nr + warp * nr;  // the warp's sums of the box's rows
+  double* sq = sqb + (1 + kPairWarps) * nr + warp * 2 * kPairCols;  // charges of the staged columns
+  double* st = sq + kPairCols;                                       // their sums
+  for (int R0 = 0; R0 < r; R0 += kPairRows) {
+    const int R1 = min(r, R0 + kPairRows);
+    for (int i = lane; i < R1 - R0; i += 32) {
+      yp[i] = 0.0;
+      if (warp == 0) sqb[i] = v.qhat[fb.row0 + R0 + i];
+    }
+    for (int c0 = w0, c1; c0 < w1 || c0 == w0; c0 = c1) {
+      c1 = min(w1, c0 + kPairCols);
+      for (int c = lane; c < kPairCols; c += 32) {
+        double q = 0.0;
+        if (c0 + c < c1) {
+          const int f = fb.slot_of(c0 + c);
+          q = v.qhat[fb.row[f] + (c0 + c - fb.col[f])];
+          if (Q32) q *= v.m2l_dec[b * 40 + forward_slot(f)].x;
+        }
+        sq[c] = q;
+      }
+      if (c0 == w0) __syncthreads();  // sqb
+      else __syncwarp();
+      if (c0 == c1) break;  // (a warp without columns)
+      // the inner and the outer forward blocks: each one contiguous region of the box's storage
+      const int cut = max(c0, min(c1, ca));
+      const int nch = (R1 - R0 + 39) / 40, step = ((R1 - R0 + nch - 1) / nch + 7) / 8 * 8;
+      for (int part = 0; part < 2; ++part) {
+        const int a = part ? cut : c0, n = (part ? c1 : cut) - a;
+        if (n <= 0) continue;
+        const long e0 = first + (long)a * r + (part ? gap : 0) + R0;
+        for (int i0 = 0; i0 < R1 - R0; i0 += step) {
+          const int nrow = min(step, R1 - R0 - i0);
+#define AFMM_PANEL(NT) m2l_pair_panel<Q32, NT>(v, e0, r, i0, nrow, n, sq + (a - c0), st + (a - c0), sqb, yp)
+          switch ((nrow + 7) >> 3) {
+            case 1: AFMM_PANEL(1); break;
+            case 2: AFMM_PANEL(2); break;
+            case 3: AFMM_PANEL(3); break;
+            case 4: AFMM_PANEL(4); break;
+            default: AFMM_PANEL(5); break;
+          }
+#undef AFMM_PANEL
+        }
+      }
+      __syncwarp();
+      for (int c = c0 + lane; c < c1; c += 32) {
+        double t = Q32 ? st[c - c0] * v.m2l_dec[b * 40 + forward_slot(fb.slot_of(c))].x : st[c - c0];
+        if (R0 > 0) t += v.back[fb.sums + c];
+        v.back[fb.sums + c] = t;
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < R1 - R0; i += 32 * kPairWarps) {
+      double s = sqb[nr + i];
+#pragma unroll
+      for (int w = 1; w < kPairWarps; ++w) s += sqb[(1 + w) * nr + i];
+      v.yhat[fb.row0 + R0 + i] = s;
+    }
+    __syncthreads();
+  }
+}
+
+// Adds to yhat[row] what the boxes that have row's box in a forward slot
+// worked out for it.
+__device__ __forceinline__ void m2l_back_row(const LevelView& v, long row) {
+  const int b = v.skel_box[row];
+  const int64_t* src = v.back_src + (long)b * kForwardSlots;
+  const long i = row - v.skel_off[b];
+  double s = v.yhat[row], t[kForwardSlots];
+#pragma unroll
+  for (int f = 0; f < kForwardSlots; ++f) {
+    const int64_t o = src[f];
+    t[f] = o >= 0 ? v.back[o + i] : 0.0;
+  }
+#pragma unroll
+  for (int f = 0; f < kForwardSlots; ++f) s += t[f];
+  v.yhat[row] = s;
 }
 
 // L2L (src/AFMM2DTree.cpp:1180-1197): t = (L2P_b yhat_b)[node row g] over the
@@ -531,35 +753,51 @@ __device__ __forceinline__ NearSlots near_slots(const NearView& nv, long b, int 
   return r;
 }
 
-// One block of J x 32 source points of near_leaf: lane l owns the points f0 + l,
-// f0 + 32 + l, ... of the flat list of leaf b's source leaves, and meets leaf
-// b's point (l + t) mod n at step t, so that in every step the lanes of the
-// warp hold different targets.  KIND: the block's points all belong to leaf b
-// (0), all to neighbours (1), or neither (2: some lanes take no part in leaf
-// b's sums).
+// Source segments of a CTA's targets: points src[m] .. of the arrays, from
+// position off[m] of the flat list on.  Their sums go to part dst[m] - 1
+// (dst = 0: the targets themselves, kNoPart: nowhere), or, without dst, to
+// their place in the flat list.
+constexpr int kNoPart = 1 << 20;
+struct PairSegs {
+  const int *src, *off, *dst;
+  int n, total;
+};
+// What the source and target points are (the near field: leaf points and
+// sorted charges; the on-the-fly M2L: skeletons and outgoing charges).
+struct PairPoints {
+  const double2* xy;
+  const double* q;
+  double* part;     // sums of the sources' side: the flat list's,
+  long stride = 0;  // or parts of `stride` values
+};
+
+// One block of J x 32 sources: lane l owns the sources f0 + l, f0 + 32 + l, ...
+// of the flat list, and meets target (l + t) mod n at step t, so that in every
+// step the lanes (of a group) hold different targets.  KIND: the block's
+// sources are all targets too (0: their sums go to `self`), all of another set
+// (1), or neither (2: some lanes take no part in the targets' sums).
 template <class K, int J, int KIND>
-__device__ __forceinline__ void near_block(const NearView& nv, const KernelParams& kp, const double* __restrict__ qs,
-                                           int f0, int total, const int* s_off, const int* s_src, const int* s_dst,
-                                           int ns, int ring, const double2* px, const double* pq, double* acc,
-                                           double* self) {
+__device__ __forceinline__ void pair_block(const PairPoints& P, const KernelParams& kp, const PairSegs& sg, int f0,
+                                           int n, const double2* px, const double* pq, double* acc, double* self,
+                                           bool add) {
   const int lane = threadIdx.x & 31;
   double2 x[J];
   double w[J], sum[J];
-  int idx[J], dst[J];  // sorted point; its part (0: leaf b itself, -1: unused lane, kNearParts: not stored)
+  int idx[J], dst[J];  // dst -1: unused lane
 #pragma unroll
   for (int u = 0; u < J; ++u) {
     const int f = f0 + 32 * u + lane;
-    const int g = min(f, total - 1);  // lanes past the end repeat the last point, unused
+    const int g = min(f, sg.total - 1);  // lanes past the end repeat the last source, unused
     int m = 0;
-    while (m + 1 < ns && g >= s_off[m + 1]) ++m;
-    idx[u] = s_src[m] + (g - s_off[m]);
-    dst[u] = f < total ? s_dst[m] : -1;
-    x[u] = nv.pts[idx[u]];
-    w[u] = qs[idx[u]];
+    while (m + 1 < sg.n && g >= sg.off[m + 1]) ++m;
+    idx[u] = sg.src[m] + (g - sg.off[m]);
+    dst[u] = f < sg.total ? (sg.dst ? sg.dst[m] : 1) : -1;
+    x[u] = P.xy[idx[u]];
+    w[u] = P.q[idx[u]];
     sum[u] = 0.0;
   }
 #pragma unroll 4
-  for (int t = 0; t < ring; ++t) {
+  for (int t = 0; t < n; ++t) {
     const double2 p = px[t];
     const double qi = pq[t];
     double a = KIND > 0 ? acc[t] : 0.0;
@@ -578,9 +816,77 @@ __device__ __forceinline__ void near_block(const NearView& nv, const KernelParam
   }
 #pragma unroll
   for (int u = 0; u < J; ++u) {
-    if (dst[u] > 0 && dst[u] < kNearParts) nv.part[(size_t)dst[u] * nv.n + idx[u]] = sum[u];
-    else if (dst[u] == 0) self[f0 + 32 * u + lane] = sum[u];  // leaf b comes first in the flat list
+    if (dst[u] > 0 && dst[u] != kNoPart) {
+      double* o = P.part + (sg.dst ? (long)(dst[u] - 1) * P.stride + idx[u] : f0 + 32 * u + lane);
+      *o = add ? *o + sum[u] : sum[u];
+    } else if (dst[u] == 0) self[f0 + 32 * u + lane] = sum[u];  // the targets come first in the flat list
   }
+}
+
+// Shared memory of pair_targets, for n targets.
+struct PairSmem {
+  double2* px;
+  double *pq, *self, *accs;
+  int row;
+  __device__ __forceinline__ PairSmem(unsigned char* smem, int n) : row(near_row(n)) {
+    px = (double2*)smem;
+    pq = (double*)(px + row);
+    self = pq + row;
+    accs = self + n;
+  }
+};
+
+// The sums of n targets (from point t0 on) against the sources of sg, and the
+// sources' sums against the targets, by `warps` warps of the CTA that share
+// the blocks of 32 sources evenly.  The caller's segments must be visible to
+// every thread; nself: the leading sources that are the targets themselves
+// (n or 0); add: the sources' sums are added to what their places hold.
+// Afterwards pair_target_sum gives a target's sum.
+template <class K>
+__device__ __forceinline__ void pair_targets(const PairPoints& P, const KernelParams& kp, const PairSegs& sg, long t0,
+                                             int n, int nself, int warps, const PairSmem& sm, bool add = false) {
+  for (int t = threadIdx.x; t < sm.row; t += blockDim.x) {
+    const int i = t % n;
+    sm.px[t] = P.xy[t0 + i];
+    sm.pq[t] = P.q[t0 + i];
+  }
+  for (int i = threadIdx.x; i < warps * sm.row; i += blockDim.x) sm.accs[i] = 0.0;
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < warps) {
+    const int l0 = n >= 32 ? lane : lane % n;  // the lane's first target
+    double* acc = sm.accs + warp * sm.row + (n >= 32 ? 0 : 2 * (lane - l0)) + l0;
+    const int nblk = (sg.total + 31) >> 5, b1 = (warp + 1) * nblk / warps;
+#define AFMM_PAIR(J, KIND) pair_block<K, J, KIND>(P, kp, sg, 32 * k, n, sm.px + l0, sm.pq + l0, acc, sm.self, add)
+    for (int k = warp * nblk / warps; k < b1;) {
+      const int nb = min(kNearJ, b1 - k);
+      const int kind = 32 * (k + nb) <= nself ? 0 : (32 * k >= nself && 32 * (k + nb) <= sg.total ? 1 : 2);
+      if (nb == 2) {
+        if (kind == 0) AFMM_PAIR(2, 0);
+        else if (kind == 1) AFMM_PAIR(2, 1);
+        else AFMM_PAIR(2, 2);
+      } else {
+        if (kind == 0) AFMM_PAIR(1, 0);
+        else if (kind == 1) AFMM_PAIR(1, 1);
+        else AFMM_PAIR(1, 2);
+      }
+      k += nb;
+    }
+#undef AFMM_PAIR
+  }
+  __syncthreads();
+}
+
+// Target i's sum over the sources that are not targets: the warps' sums in
+// warp order (each the sum of its lane groups' rows and of their two laps).
+__device__ __forceinline__ double pair_target_sum(const PairSmem& sm, int n, int warps, int i, double v) {
+  for (int x = 0; x < warps; ++x) {
+    const double* r = sm.accs + x * sm.row + i;
+    if (n >= 32) v += i < 32 ? r[0] + r[n] : r[0];
+    else
+      for (int c = 0; c < sm.row; c += 2 * n) v += r[c] + r[c + n];
+  }
+  return v;
 }
 
 // Near field (src/AFMM2DTree.cpp:1199-1213) of leaf b, kernel evaluated on the
@@ -631,8 +937,8 @@ __device__ __forceinline__ void near_leaf(const NearView& nv, const KernelParams
       const int m = __popc(valid & ((1u << lane) - 1u));
       s_src[m] = start;
       s_off[m] = pre - cnt;
-      // (a leaf outside the shard gets no sums)
-      s_dst[m] = lane == 0 ? 0 : (c >= nv.leaf0 && c < nv.leaf0 + nv.nleaf ? lane : kNearParts);
+      // (a leaf outside the shard gets no sums; part 0 is the leaf's own)
+      s_dst[m] = lane == 0 ? 0 : (c >= nv.leaf0 && c < nv.leaf0 + nv.nleaf ? lane + 1 : kNoPart);
     }
     if (lane == 4) {
       s_ns = __popc(valid);
@@ -640,54 +946,13 @@ __device__ __forceinline__ void near_leaf(const NearView& nv, const KernelParams
     }
     if (lane >= 5 && lane < 9) s_back[lane - 5] = c >= 0;
   }
-  const int row = near_row(n), ring = near_ring(n);
-  double2* px = (double2*)smem;
-  double* pq = (double*)(px + row);
-  double* self = pq + row;
-  double* accs = self + n;
-  for (int t = threadIdx.x; t < row; t += blockDim.x) {
-    const int i = t % ring;
-    px[t] = i < n ? nv.pts[s0 + i] : make_double2(kPadPoint, kPadPoint);
-    pq[t] = i < n ? qs[s0 + i] : 0.0;
-  }
-  for (int i = threadIdx.x; i < warps * row; i += blockDim.x) accs[i] = 0.0;
+  const PairSmem sm(smem, n);
   __syncthreads();
-  const int ns = s_ns, total = s_off[ns], nblk = (total + 31) >> 5;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < warps) {
-    // lane l starts at target l (of its group's row)
-    const int l0 = n < 32 ? lane & (ring - 1) : lane;
-    double* acc = accs + warp * row + (n < 32 ? 2 * (lane - l0) : 0) + l0;
-    const int b1 = (warp + 1) * nblk / warps;
-#define AFMM_NEAR(J, KIND) \
-  near_block<K, J, KIND>(nv, kp, qs, 32 * k, total, s_off, s_src, s_dst, ns, ring, px + l0, pq + l0, acc, self)
-    for (int k = warp * nblk / warps; k < b1;) {
-      const int nb = min(kNearJ, b1 - k);
-      const int kind = 32 * (k + nb) <= n ? 0 : (32 * k >= n && 32 * (k + nb) <= total ? 1 : 2);
-      if (nb == 2) {
-        if (kind == 0) AFMM_NEAR(2, 0);
-        else if (kind == 1) AFMM_NEAR(2, 1);
-        else AFMM_NEAR(2, 2);
-      } else {
-        if (kind == 0) AFMM_NEAR(1, 0);
-        else if (kind == 1) AFMM_NEAR(1, 1);
-        else AFMM_NEAR(1, 2);
-      }
-      k += nb;
-    }
-#undef AFMM_NEAR
-  }
-  __syncthreads();
+  pair_targets<K>(PairPoints{nv.pts, qs, nv.part, nv.n}, kp, PairSegs{s_src, s_off, s_dst, s_ns, s_off[s_ns]}, s0, n, n,
+                  warps, sm);
   if (!own) return;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    double v = self[i];
-    for (int x = 0; x < warps; ++x) {
-      const double* r = accs + x * row + i;
-      if (n >= 32) v += i < 32 ? r[0] + r[n] : r[0];
-      else
-        for (int c = 0; c < 64; c += 2 * ring) v += r[c] + r[c + ring];
-    }
-    nv.part[s0 + i] = v;
+    nv.part[s0 + i] = pair_target_sum(sm, n, warps, i, sm.self[i]);
     for (int s = 0; s < 4; ++s)
       if (!s_back[s]) nv.part[(size_t)(1 + s) * nv.n + s0 + i] = 0.0;
   }
@@ -708,16 +973,20 @@ void gather_points(const double2* pts, const int32_t* ids, long n, double2* out,
 void m2l_assemble(const LevelView& v, const KernelParams& kp, cudaStream_t s);
 // 32-bit fixed-point copy of the stored FP64 blocks (m2l_q, m2l_dec).
 void m2l_compress(const LevelView& v, cudaStream_t s);
+// Forward columns of a level's boxes (v.fwd, v.back_src).
+void forward_boxes(const LevelView& v, cudaStream_t s);
 void l2p_transpose(const LevelView& v, const double* cm, double* rm, cudaStream_t s);
 void matvec_fp64(const MatvecPlan& p, const double* q, double* y, cudaStream_t s, StageTimer* tm, int64_t* launches);
-// M2L of every level in FP64: the stored blocks (one thread per skeleton row),
-// or m2l_apply_otf when no blocks are stored.
-void m2l_apply(const MatvecPlan& p, cudaStream_t s);
+// One-column M2L of every level in FP64: the stored blocks, or m2l_apply_otf
+// when no blocks are stored.  These return the launches made.
+int m2l_apply(const MatvecPlan& p, cudaStream_t s);
 // M2L of the given levels from the stored blocks, 32-bit fixed point (q32)
-// or FP64, FP64 arithmetic, one warp per row chunk.
-void m2l_apply_stored(const MatvecPlan& p, const LevelSet& levels, bool q32, cudaStream_t s);
+// or FP64, FP64 arithmetic.
+int m2l_apply_stored(const MatvecPlan& p, const LevelSet& levels, bool q32, cudaStream_t s);
 // M2L of the given levels with the entries evaluated on the fly in FP64 (mixed.cu).
-void m2l_apply_otf(const MatvecPlan& p, const LevelSet& levels, cudaStream_t s);
+int m2l_apply_otf(const MatvecPlan& p, const LevelSet& levels, cudaStream_t s);
+// Their second launch: the sums that other boxes worked out (m2l_back_row).
+int m2l_back(const LevelSet& ls, cudaStream_t s);
 // The FP64 sweeps shared by both precisions (leaf charges qs in FP64).
 void sweep_m2m(const MatvecPlan& p, const double* qs, cudaStream_t s, int64_t* launches);
 void sweep_l2l(const MatvecPlan& p, double* ys, cudaStream_t s, int64_t* launches);

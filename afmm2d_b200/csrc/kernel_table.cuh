@@ -40,7 +40,7 @@ struct KernelTable {
   // FP64 near field, one column, into NearView::part (fmm_k.cuh)
   void (*p2p64)(const NearView&, const KernelParams&, const double*, cudaStream_t) = nullptr;
   // single-RHS mixed path: M2L on the fly (FP64), FP32 near field (mixed_k.cuh)
-  void (*m2l_otf)(const LevelSet&, const KernelParams&, cudaStream_t) = nullptr;
+  void (*m2l_otf)(const LevelSet&, int rmax, const KernelParams&, cudaStream_t) = nullptr;
   void (*p2p32)(const NearView&, const KernelParams&, const float*, double*, cudaStream_t) = nullptr;
   // batched passes (batched_k.cuh), [0] 8 / [1] 16 columns: M2L on the fly,
   // mixed near field, FP64 near field

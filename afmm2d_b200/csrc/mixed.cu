@@ -76,9 +76,10 @@ inline int nb(long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
-void m2l_apply_otf(const MatvecPlan& p, const LevelSet& levels, cudaStream_t s) {
-  if (levels.row0[levels.nlev] == 0) return;
-  kernel_table(p.kp.id).m2l_otf(levels, p.kp, s);
+int m2l_apply_otf(const MatvecPlan& p, const LevelSet& levels, cudaStream_t s) {
+  if (levels.row0[levels.nlev] == 0) return 0;
+  kernel_table(p.kp.id).m2l_otf(levels, *std::max_element(p.rmax, p.rmax + kMaxLevels), p.kp, s);
+  return 1 + m2l_back(levels, s);
 }
 
 
@@ -145,14 +146,8 @@ void matvec_mixed(const MatvecPlan& p, MixedState& ms, const double* q, int64_t 
     const uint32_t otf = stored ? p.tune.otf_mixed : 0xffffffffu;
     // a shard's boxes at the sharded levels for the stored form; the on-the-fly levels whole
     const LevelSet st = level_subset(p.levels_m2l, otf, false), fly = level_subset(p.levels, otf, true);
-    if (st.nlev > 0) {
-      m2l_apply_stored(p, st, q32, s);
-      ++*launches;
-    }
-    if (fly.nlev > 0) {
-      m2l_apply_otf(p, fly, s);
-      ++*launches;
-    }
+    if (st.nlev > 0) *launches += m2l_apply_stored(p, st, q32, s);
+    if (fly.nlev > 0) *launches += m2l_apply_otf(p, fly, s);
     if (tm) tm->mark(s, "l2l");
     sweep_l2l(p, ms.ys, s, launches);
     if (tm) tm->mark(s, "p2p");

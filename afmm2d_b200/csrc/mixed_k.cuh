@@ -17,53 +17,45 @@ __device__ __forceinline__ float fallback_r2(float span_b, float span_c) {
   return t;
 }
 
-// M2L on the fly in FP64 for every level, one thread per skeleton row
-// (upper levels first): row i of box b sums, slot by slot in the reference's
-// order, K(R_b[i], R_c[cc]) * qhat_c[cc] with the entries evaluated from the
-// skeleton coordinates (a warp's rows share the source points: broadcast
-// loads).
+// M2L on the fly in FP64 for every level, one CTA per box (upper levels
+// first): the box's skeleton points against those of its forward
+// interaction-list boxes, every entry worked out once for both (pair_targets,
+// as the FP64 near field; the sums as in m2l_pair_box).  Issue-bound like it:
+// 262,144 spiral points, log, TOL 12: 0.80 -> 0.34 ms (one thread per skeleton
+// row, every entry worked out for both sides).
+constexpr int kOtfWarps = 4;
 template <class K>
-__global__ void k_m2l_otf(LevelSet ls, KernelParams kp) {
-  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= ls.row0[ls.nlev]) return;
+__global__ void __launch_bounds__(32 * kOtfWarps, 6) k_m2l_otf(LevelSet ls, KernelParams kp) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ ForwardBox fb;
+  const long g = blockIdx.x;
   int j = 0;
-  while (j + 1 < ls.nlev && g >= ls.row0[j + 1]) ++j;
+  while (j + 1 < ls.nlev && g >= ls.b0[j + 1]) ++j;
   const LevelView& v = ls.lv[j];
-  const long row = g - ls.row0[j];
-  const int b = v.skel_box[row];
-  const double2 xi = v.skel_xy[row];
-  double acc = 0.0;
-  for (int s = 0; s < 40; ++s) {
-    const int c = v.il[(long)b * 40 + s];
-    if (c < 0) continue;
-    const int rc = v.rank[c];
-    const double2* xc = v.skel_xy + v.skel_off[c];
-    const double* qc = v.qhat + v.skel_off[c];
-    double a0 = 0.0, a1 = 0.0;
-    int cc = 0;
-    for (; cc + 1 < rc; cc += 2) {
-      const double2 p0 = xc[cc], p1 = xc[cc + 1];
-      const double dx0 = xi.x - p0.x, dy0 = xi.y - p0.y;
-      const double dx1 = xi.x - p1.x, dy1 = xi.y - p1.y;
-      a0 += K::eval(dx0 * dx0 + dy0 * dy0, kp) * qc[cc];
-      a1 += K::eval(dx1 * dx1 + dy1 * dy1, kp) * qc[cc + 1];
-    }
-    if (cc < rc) {
-      const double2 p0 = xc[cc];
-      const double dx0 = xi.x - p0.x, dy0 = xi.y - p0.y;
-      a0 += K::eval(dx0 * dx0 + dy0 * dy0, kp) * qc[cc];
-    }
-    acc += a0 + a1;
+  const long b = g - ls.b0[j];
+  if (threadIdx.x < sizeof(ForwardBox) / 8) ((int64_t*)&fb)[threadIdx.x] = ((const int64_t*)(v.fwd + b))[threadIdx.x];
+  __syncthreads();
+  const int r = fb.r;
+  if (r == 0) return;
+  const PairSegs sg{fb.row, fb.col, nullptr, kForwardSlots, fb.col[kForwardSlots]};
+  for (int R0 = 0; R0 < r; R0 += kPairRows) {  // (one round unless the rank is beyond kPairRows)
+    const int n = min(kPairRows, r - R0);
+    const PairSmem sm(smem, n);
+    pair_targets<K>(PairPoints{v.skel_xy, v.qhat, v.back + fb.sums}, kp, sg, fb.row0 + R0, n, 0, kOtfWarps, sm, R0 > 0);
+    for (int i = threadIdx.x; i < n; i += 32 * kOtfWarps)
+      v.yhat[fb.row0 + R0 + i] = pair_target_sum(sm, n, kOtfWarps, i, 0.0);
+    __syncthreads();
   }
-  v.yhat[row] = acc;
 }
 
 template <class K>
 struct M2lOtfRun {
-  static void run(const LevelSet& ls, const KernelParams& kp, cudaStream_t s) {
-    const long rows = ls.row0[ls.nlev];
-    if (rows == 0) return;  // every box of ACA rank 0: no far field
-    k_m2l_otf<K><<<(int)((rows + 127) / 128), 128, 0, s>>>(ls, kp);
+  static void run(const LevelSet& ls, int rmax, const KernelParams& kp, cudaStream_t s) {
+    const long boxes = ls.b0[ls.nlev];
+    if (boxes == 0) return;
+    const size_t smem = near_smem(std::min(rmax, kPairRows), kOtfWarps);
+    allow_smem(k_m2l_otf<K>, smem);
+    k_m2l_otf<K><<<(int)boxes, 32 * kOtfWarps, smem, s>>>(ls, kp);
     AFMM_LAUNCH_CHECK();
   }
 };

@@ -146,12 +146,21 @@ __global__ void __launch_bounds__(kSweepTile) k_set_up(SetDev d, SweepPlan sw, S
   }
 }
 
-// M2L of every level of every problem (skeleton rows).
-__global__ void k_set_m2l(SetDev d, SetSegs sg) {
+// M2L of every level of every problem, one CTA per box, and the sums that
+// other boxes worked out (skeleton rows).
+__global__ void __launch_bounds__(32 * kPairWarps, 6) k_set_m2l(SetDev d, SetSegs sg) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const long g = blockIdx.x;
+  const int s = seg_of(sg, g);
+  const LevelView v = d.lv[(long)sg.prob[s] * kMaxLevels + sg.level[s]];
+  m2l_pair_box<false>(v, g - sg.first[s], 12 * 1024, smem);
+}
+
+__global__ void __launch_bounds__(256) k_set_m2l_back(SetDev d, SetSegs sg) {
   const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= sg.total) return;
   const int s = seg_of(sg, g);
-  m2l_row(d.lv[(long)sg.prob[s] * kMaxLevels + sg.level[s]], g - sg.first[s]);
+  m2l_back_row(d.lv[(long)sg.prob[s] * kMaxLevels + sg.level[s]], g - sg.first[s]);
 }
 
 // Down-sweep: L2L of every problem from level 2 down to its leaf level (node
@@ -259,9 +268,11 @@ void record(SetPlan& sp, cudaStream_t s) {
   }
   mark("m2l");
   if (sp.m2l.total > 0) {
-    k_set_m2l<<<nb(sp.m2l.total, 128), 128, 0, s>>>(sp.dev, sp.m2l);
+    k_set_m2l<<<(int)sp.m2l_box.total, 32 * kPairWarps, sp.m2l_smem, s>>>(sp.dev, sp.m2l_box);
     AFMM_LAUNCH_CHECK();
-    ++n;
+    k_set_m2l_back<<<nb(sp.m2l.total, 256), 256, 0, s>>>(sp.dev, sp.m2l);
+    AFMM_LAUNCH_CHECK();
+    n += 2;
   }
   mark("l2l");
   if (sp.down.nitems > 0) {
@@ -291,7 +302,8 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
   std::vector<const int64_t*> perm(np);
   std::vector<double*> qs(np), ys(np);
   std::vector<int64_t> off(np + 1, 0);
-  SegBuilder g, m2l, p2p;
+  SegBuilder g, m2l, m2l_box, p2p;
+  int rmax = 0;
   int maxL = 0;
   sp.p2p_threads = 0;
   sp.p2p_smem = 0;
@@ -307,6 +319,9 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
     off[p + 1] = off[p] + mp.N;
     g.add(p, 0, mp.N);
     for (int j = 2; j <= mp.L; ++j) m2l.add(p, j, mp.lv[j].nrows);
+    for (int j = 2; j <= mp.L; ++j)
+      if (mp.lv[j].nrows > 0) m2l_box.add(p, j, mp.lv[j].nbox);
+    rmax = std::max(rmax, *std::max_element(mp.rmax, mp.rmax + kMaxLevels));
     p2p.add(p, mp.L, mp.near.nleaf);
     maxL = std::max(maxL, mp.L);
     sp.p2p_threads = std::max(sp.p2p_threads, 32 * warps[p]);
@@ -374,6 +389,9 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
   }
   sp.gather = g.upload(arena, s);
   sp.m2l = m2l.upload(arena, s);
+  sp.m2l_box = m2l_box.upload(arena, s);
+  sp.m2l_smem = m2l_pair_smem(rmax);
+  allow_smem(k_set_m2l, sp.m2l_smem);
   sp.p2p = p2p.upload(arena, s);
   sp.dev.nprob = np;
   sp.dev.lv = upload(lv, arena, s);

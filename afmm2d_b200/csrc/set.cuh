@@ -73,7 +73,8 @@ struct SetPlan {
   long total_points = 0;
   int p2p_threads = 0;
   size_t p2p_smem = 0;
-  SetSegs gather, m2l, p2p;
+  SetSegs gather, m2l, m2l_box, p2p;  // m2l: skeleton rows, m2l_box: boxes
+  size_t m2l_smem = 0;
   std::vector<SetSegs> m2m;  // by depth below each problem's leaf level
   std::vector<SetSegs> l2l;  // by level 2, 3, ...
   double* q = nullptr;       // set input (original order, problems concatenated)

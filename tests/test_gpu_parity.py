@@ -400,3 +400,28 @@ def test_pairwise_near_field_leaf_sizes(kernel, N, M):
     for c in range(3):
         y = a.computeMatVecProduct(Q[:, c])
         assert np.linalg.norm(y - Yb[:, c]) <= FP64_BATCHED_TOL * np.linalg.norm(y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel,N,M,tol,least", [("gaussian", 700, 40, 2, 1), ("log", 5000, 64, 4, 8),
+                                                  ("log", 16384, 256, 12, 41), ("one_over_r", 16000, 400, 12, 60)])
+def test_pairwise_m2l_ranks(kernel, N, M, tol, least):
+    """The one-column M2L (every pair of boxes once, forward columns) against the batched passes' (every box's
+    own blocks), at ranks of one tile of rows, a few, several panels of rows and more columns than a warp
+    stages at once; and with the entries on the fly.  Only the summation order differs."""
+    rng = np.random.default_rng(N)
+    pts = rng.uniform(0, 1, (N, 2))
+    Q = rng.standard_normal((N, 2))
+    ys = []
+    for storage in ("store", "on_the_fly"):
+        a = A.AFMM(N, M, tol, pts, kernel=kernel, kparam=0.1 if kernel == "gaussian" else None)
+        a.set_m2l_storage(storage)
+        a.assemble()
+        assert max(a.ranks(j).max() for j in range(2, a.nLevels + 1)) >= least
+        Yb = a.computeMatVecProduct(Q, precision="fp64_batched")
+        y = a.computeMatVecProduct(Q[:, 0])
+        assert np.linalg.norm(y - Yb[:, 0]) <= FP64_BATCHED_TOL * np.linalg.norm(y)
+        ym = a.computeMatVecProduct(Q[:, 0], precision="mixed")
+        assert np.linalg.norm(ym - y) <= MIXED_TOL * np.linalg.norm(y)
+        ys.append(y)
+    assert np.linalg.norm(ys[0] - ys[1]) <= 1e-10 * np.linalg.norm(ys[0])
