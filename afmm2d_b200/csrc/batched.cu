@@ -18,6 +18,7 @@
 //    sources tiles), tile sums per source leaf accumulated in FP64.
 // With RC = 4 the same products run on the FMA pipes.
 #include <algorithm>
+#include <type_traits>
 
 #include "batched_common.cuh"
 #include "kernel_table.cuh"
@@ -114,40 +115,11 @@ __device__ __forceinline__ void mma_rows(double (&c)[NT][RC / 8][2], const doubl
     double a[NT], bq[RC / 8];
 #pragma unroll
     for (int u = 0; u < NT; ++u) a[u] = (vk && rowok[u]) ? Ak[u * 8] : 0.0;
-#pragma unroll
-    for (int t = 0; t < RC / 8; ++t) bq[t] = vk ? B[(long)k * RC + t * 8 + trow] : 0.0;
+    load_b<RC>(B + (long)k * RC, trow, vk, bq);
 #pragma unroll
     for (int u = 0; u < NT; ++u)
 #pragma unroll
       for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(c[u][t][0], c[u][t][1], a[u], bq[t]);
-  }
-}
-
-// mma_rows with the 32-bit fixed-point M2L entries of one block (decode
-// constants `dec`, decode_q32): each 4-column step loads its A entries as
-// 32-bit words (half the bytes of FP64) and decodes them exactly before the
-// FP64 products.
-template <int RC, int NT>
-__device__ __forceinline__ void mma_rows_q32(double (&c)[NT][RC / 8][2], const uint32_t* __restrict__ A, int lda,
-                                             int K, double2 dec, const double* __restrict__ B,
-                                             const bool (&rowok)[NT], int trow, int tsrc) {
-#pragma unroll 4
-  for (int k0 = 0; k0 < K; k0 += 4) {
-    const int k = k0 + tsrc;
-    const bool vk = k < K;
-    const uint32_t* Ak = A + (long)k * lda;
-    uint32_t ua[NT];
-    double bq[RC / 8];
-#pragma unroll
-    for (int u = 0; u < NT; ++u) ua[u] = (vk && rowok[u]) ? Ak[u * 8] : 0x80000000u;  // 2^31 decodes to 0
-#pragma unroll
-    for (int t = 0; t < RC / 8; ++t) bq[t] = vk ? B[(long)k * RC + t * 8 + trow] : 0.0;
-#pragma unroll
-    for (int u = 0; u < NT; ++u) {
-      const double a = decode_q32(ua[u], dec);
-#pragma unroll
-      for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(c[u][t][0], c[u][t][1], a, bq[t]);
-    }
   }
 }
 
@@ -166,62 +138,131 @@ __device__ __forceinline__ void store_tiles(const double (&c)[NT][RC / 8][2], do
 #pragma unroll
   for (int u = 0; u < NT; ++u) {
     if (rowok[u]) {
-      double2* o = reinterpret_cast<double2*>(out + (long)(u * 8 + trow) * RC + 2 * tsrc);
+      // columns RC/4 tsrc .. of the row: two of a tile, four of two interleaved tiles
+      double2* o = reinterpret_cast<double2*>(out + (long)(u * 8 + trow) * RC + RC / 4 * tsrc);
 #pragma unroll
-      for (int t = 0; t < RC / 8; ++t) {
-        double2 w = make_double2(c[u][t][0], c[u][t][1]);
+      for (int h = 0; h < RC / 8; ++h) {
+        double2 w = RC == 16 ? make_double2(c[u][0][h], c[u][RC / 8 - 1][h]) : make_double2(c[u][0][0], c[u][0][1]);
         if (ADD) {
-          const double2 cur = o[t * 4];
+          const double2 cur = o[h];
           w.x += cur.x;
           w.y += cur.y;
         }
-        o[t * 4] = w;
+        o[h] = w;
       }
     }
   }
 }
 
-// M2L from the stored FP64 blocks (the same blocks the FP64 path applies)
-// with FP64 tensor-core tiles: one warp per chunk of up to kChunkRows skeleton
-// rows of one box, i.e. NT <= 5 tiles of 8 rows that share every B fragment.
-// The 40 slots' rank and skeleton offset are fetched once per warp and
-// broadcast by shuffles; the box's contiguous block region is streamed into
-// L2 ahead of the loads.
+// The 40 slots of a box as one list of columns: a box's blocks lie back to back,
+// one r x C column-major matrix.  Per slot the column after its last, what
+// turns its columns into skeleton rows, and its block's scale (fixed point).
+struct SlotTable {
+  int end[40], row[40];
+  double scale[40];
+};
+
+// M2L from the stored blocks (the same blocks the FP64 path applies) with FP64
+// tensor-core tiles: one warp per chunk of up to kChunkRows skeleton rows of
+// one box, i.e. NT <= 5 tiles of 8 rows that share every B fragment.  The
+// columns of all slots make one K loop (a step of 4 columns may straddle two
+// blocks: no padding per block), whose loads run three steps ahead of the
+// products in registers; the box's contiguous block region is streamed into L2
+// ahead of the loads.  Fixed point: u - 2^31 is exact, and the block's power
+// of two goes to the charges (exact).  4,194,304 points (mixture, 1/r), 16
+// columns: FP64 blocks 4.02 -> 3.5 ms, fixed point 3.77 -> 3.6 (FP64 tensor pipe
+// 52 -> 67% and 56 -> 60% busy; the FP64 form is then also at 82% of the L1's
+// wavefronts, the fixed-point one waits for its decoding on the same pipe).
+// Two, four or six steps ahead: 3.5 / 3.5 / 3.6 and 3.7 / 3.75 / 4.1 (registers).
 template <int RC, int NT, bool Q32>
 __device__ __forceinline__ void m2l_stored_chunk(const LevelView& v, const double* __restrict__ qh,
-                                                 double* __restrict__ yb, int b, int r0, int lane, uint32_t ahead) {
+                                                 double* __restrict__ yb, int b, int r0, int lane, uint32_t ahead,
+                                                 SlotTable& tab) {
+  typedef typename std::conditional<Q32, uint32_t, double>::type T;
+  constexpr int kM2lAhead = 3;
   const int r = v.rank[b];
   const int i0 = r0 - v.skel_off[b];
   const int nrow = min(8 * NT, r - i0);
   const int trow = lane >> 2, tsrc = lane & 3;
-  // slot table: lane l holds slot l (and slot 32 + l for l < 8)
+  const bool last = 8 * (NT - 1) + trow < nrow;  // only the last tile can hold rows past the chunk's
+  // slot table: lane l looks slot l up (and slot 32 + l for l < 8)
   const int sa = v.il[(long)b * 40 + lane];
   const int sb = lane < 8 ? v.il[(long)b * 40 + 32 + lane] : -1;
   const int ra = sa >= 0 ? v.rank[sa] : 0, rb = sb >= 0 ? v.rank[sb] : 0;
   const int oa = sa >= 0 ? v.skel_off[sa] : 0, ob = sb >= 0 ? v.skel_off[sb] : 0;
-  bool rowok[NT];
+  int pa = ra, pb = rb;
 #pragma unroll
-  for (int u = 0; u < NT; ++u) rowok[u] = u * 8 + trow < nrow;
-  long pos = v.m2l_off[b];  // first entry of the current slot's block
-  const long stop = v.m2l_off[b + 1];
-  L2Stream pf(Q32 ? (const void*)(v.m2l_q + pos) : (const void*)(v.m2l + pos),
-              Q32 ? (const void*)(v.m2l_q + stop) : (const void*)(v.m2l + stop), ahead);
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ta = __shfl_up_sync(0xffffffffu, pa, o), tb = __shfl_up_sync(0xffffffffu, pb, o);
+    if (lane >= o) {
+      pa += ta;
+      pb += tb;
+    }
+  }
+  const int na = __shfl_sync(0xffffffffu, pa, 31), C = na + __shfl_sync(0xffffffffu, pb, 31);
+  tab.end[lane] = pa;
+  tab.row[lane] = oa - (pa - ra);
+  if (Q32) tab.scale[lane] = v.m2l_dec[(long)b * 40 + lane].x;
+  if (lane < 8) {
+    tab.end[32 + lane] = na + pb;
+    tab.row[32 + lane] = ob - (na + pb - rb);
+    if (Q32) tab.scale[32 + lane] = v.m2l_dec[(long)b * 40 + 32 + lane].x;
+  }
+  __syncwarp();
+  const T* blk = (Q32 ? (const T*)v.m2l_q : (const T*)v.m2l) + v.m2l_off[b];
+  L2Stream pf(blk, blk + (long)C * r, ahead);
+  const T* P = blk + (long)tsrc * r + i0 + trow;  // the lane's entry of tile 0 in its next column to load
+  int s = -1, end = 0, row = 0;                   // slot of that column
+  double sc = 1.0;
+  T a[kM2lAhead][NT];
+  double bq[kM2lAhead][RC / 8], scale[kM2lAhead];
+  auto load = [&](int d, int k) {
+    const bool vk = k < C;
+    while (vk && k >= end) {
+      ++s;
+      end = tab.end[s];
+      row = tab.row[s];
+      if (Q32) sc = tab.scale[s];
+    }
+#pragma unroll
+    for (int u = 0; u < NT; ++u) a[d][u] = vk && (u + 1 < NT || last) ? __ldg(P + 8 * u) : (T)(Q32 ? 0x80000000u : 0u);
+    load_b<RC>(qh + (long)(k + row) * RC, trow, vk, bq[d]);
+    if (Q32) scale[d] = sc;
+    P += 4l * r;
+  };
   double c[NT][RC / 8][2];
   zero_tiles<RC, NT>(c);
-  for (int s = 0; s < 40; ++s) {
-    const int rc = __shfl_sync(0xffffffffu, s < 32 ? ra : rb, s & 31);
-    if (rc == 0) continue;  // empty slot or rank-0 box: no block stored
-    const int sc = __shfl_sync(0xffffffffu, s < 32 ? oa : ob, s & 31);
-    if (Q32) {
-      pf.advance(v.m2l_q + pos, lane);
-      mma_rows_q32<RC, NT>(c, v.m2l_q + pos + i0 + trow, r, rc, v.m2l_dec[(long)b * 40 + s], qh + (long)sc * RC,
-                           rowok, trow, tsrc);
-    } else {
-      pf.advance(v.m2l + pos, lane);
-      mma_rows<RC, NT>(c, v.m2l + pos + i0 + trow, r, rc, qh + (long)sc * RC, rowok, trow, tsrc);
+  pf.advance(blk, lane);
+#pragma unroll
+  for (int d = 0; d < kM2lAhead; ++d) load(d, 4 * d + tsrc);
+  for (int k0 = 0; k0 < C; k0 += 4 * kM2lAhead) {
+    pf.advance(blk + (long)k0 * r, lane);
+#pragma unroll
+    for (int d = 0; d < kM2lAhead; ++d) {
+      double bs[RC / 8];
+#pragma unroll
+      for (int t = 0; t < RC / 8; ++t) bs[t] = Q32 ? bq[d][t] * scale[d] : bq[d][t];
+      if constexpr (Q32) {
+        double x[NT];
+#pragma unroll
+        for (int u = 0; u < NT; ++u) x[u] = __hiloint2double(0x43300000, (int)a[d][u]) - 4503601774854144.0;  // u - 2^31
+        load(d, k0 + 4 * (kM2lAhead + d) + tsrc);  // (the stage's registers are free)
+#pragma unroll
+        for (int u = 0; u < NT; ++u)
+#pragma unroll
+          for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(c[u][t][0], c[u][t][1], x[u], bs[t]);
+      } else {
+#pragma unroll
+        for (int u = 0; u < NT; ++u)
+#pragma unroll
+          for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(c[u][t][0], c[u][t][1], a[d][u], bs[t]);
+        load(d, k0 + 4 * (kM2lAhead + d) + tsrc);
+      }
     }
-    pos += (long)r * rc;
   }
+  bool rowok[NT];
+#pragma unroll
+  for (int u = 0; u < NT; ++u) rowok[u] = u + 1 < NT || last;
   store_tiles<RC, NT, false>(c, yb + (long)r0 * RC, rowok, trow, tsrc);
 }
 
@@ -538,7 +579,7 @@ __global__ void __launch_bounds__(32 * S) k_l2l_mma_split(LevelView v, const dou
 }
 
 template <int RC, bool Q32>
-__global__ void __launch_bounds__(128) k_m2l_stored_mma(LevelSet ls, const double* const* __restrict__ qhat_lv,
+__global__ void __launch_bounds__(128, 4) k_m2l_stored_mma(LevelSet ls, const double* const* __restrict__ qhat_lv,
                                                         double* const* __restrict__ yhat_lv) {
   const long gw = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -549,7 +590,9 @@ __global__ void __launch_bounds__(128) k_m2l_stored_mma(LevelSet ls, const doubl
   const long g = gw - ls.cgrp0[j];
   const int b = v.cgrp_box[g];
   const int r0 = v.cgrp_row[g];
-#define AFMM_M2L(NT) m2l_stored_chunk<RC, NT, Q32>(v, qhat_lv[ls.src[j]], yhat_lv[ls.src[j]], b, r0, lane, ls.pf_ahead)
+  __shared__ SlotTable tab[4];
+#define AFMM_M2L(NT) \
+  m2l_stored_chunk<RC, NT, Q32>(v, qhat_lv[ls.src[j]], yhat_lv[ls.src[j]], b, r0, lane, ls.pf_ahead, tab[threadIdx.x >> 5])
   AFMM_NT_SWITCH(chunk_tiles(v.cgrp_row, g, v.ncgroups, v.skel_off[b] + v.rank[b]), AFMM_M2L)
 #undef AFMM_M2L
 }

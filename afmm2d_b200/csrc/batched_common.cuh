@@ -56,6 +56,21 @@ __device__ __forceinline__ void mma_f64_16x8x4(double (&c)[4], double a0, double
                : "d"(a0), "d"(a1), "d"(b));
 }
 
+// The 16 right-hand sides of a pass make two column tiles; tile t takes the
+// columns 2n + t (n = 0..7), so that a lane's two B values are neighbours (one
+// 16-byte load, one 128-byte line per point instead of two) and its results are
+// four neighbouring columns.
+template <int RC>
+__device__ __forceinline__ void load_b(const double* __restrict__ row, int trow, bool ok, double (&bq)[RC / 8]) {
+  if constexpr (RC == 16) {
+    const double2 w = ok ? __ldg(reinterpret_cast<const double2*>(row) + trow) : make_double2(0.0, 0.0);
+    bq[0] = w.x;
+    bq[1] = w.y;
+  } else {
+    bq[0] = ok ? __ldg(row + trow) : 0.0;
+  }
+}
+
 }  // namespace batched_common
 
 using namespace batched_common;

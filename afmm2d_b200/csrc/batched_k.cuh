@@ -323,8 +323,7 @@ __global__ void __launch_bounds__(128) k_p2p_dmma(NearView nv, KernelParams kp, 
         const double2 p = sx[st * 4 + tsrc];
         const bool vj = j < nc;
         double bq[RC / 8];
-#pragma unroll
-        for (int t = 0; t < RC / 8; ++t) bq[t] = vj ? qs[(long)(src + j) * RC + t * 8 + trow] : 0.0;
+        load_b<RC>(qs + (long)(src + j) * RC, trow, vj, bq);
 #pragma unroll
         for (int u = 0; u < NTT; ++u) {
           const double dx = x[u].x - p.x, dy = x[u].y - p.y;
@@ -334,18 +333,18 @@ __global__ void __launch_bounds__(128) k_p2p_dmma(NearView nv, KernelParams kp, 
         }
       }
     }
-    // D fragment: row trow, columns 2*tsrc, 2*tsrc + 1 of each 8-column block
+    // D fragment: row trow, columns RC/4 tsrc .. (load_b's column order)
 #pragma unroll
     for (int u = 0; u < NTT; ++u) {
       const int ti = tg * 32 + u * 8 + trow;
       if (ti < n) {
+        double2* o = reinterpret_cast<double2*>(ys + (long)(s0 + ti) * RC + RC / 4 * tsrc);
 #pragma unroll
-        for (int t = 0; t < RC / 8; ++t) {
-          double2* o = reinterpret_cast<double2*>(ys + (long)(s0 + ti) * RC + t * 8 + 2 * tsrc);
-          double2 w = *o;
-          w.x += c[u][t][0];
-          w.y += c[u][t][1];
-          *o = w;
+        for (int h = 0; h < RC / 8; ++h) {
+          double2 w = o[h];
+          w.x += RC == 16 ? c[u][0][h] : c[u][0][0];
+          w.y += RC == 16 ? c[u][RC / 8 - 1][h] : c[u][0][1];
+          o[h] = w;
         }
       }
     }
