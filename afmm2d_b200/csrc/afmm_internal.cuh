@@ -278,12 +278,6 @@ struct LevelDev {
   int32_t* ncgrp_box = nullptr;  // node-row chunk (<= kChunkRows node rows of one box) -> box
   int32_t* ncgrp_row = nullptr;  // node-row chunk -> first node row
   long nncgroups = 0;
-  int32_t* wgrp_box = nullptr;   // row chunk (<= 32 skeleton rows of one box: a warp's lanes) -> box
-  int32_t* wgrp_row = nullptr;   // row chunk -> first skeleton row
-  long nwgroups = 0;
-  int32_t* nwgrp_box = nullptr;  // node-row chunk (<= 32 node rows of one box) -> box
-  int32_t* nwgrp_row = nullptr;  // node-row chunk -> first node row
-  long nnwgroups = 0;
   int32_t* ptile_par = nullptr;  // parent row tile (<= 128 rows of the parent's four children) -> parent
   int32_t* ptile_row = nullptr;  // parent row tile -> first row in the children's concatenated rows
   long nptiles = 0;

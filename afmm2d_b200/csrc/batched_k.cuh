@@ -110,7 +110,7 @@ constexpr float kPadSrc = 1.0e15f, kPadTgt = -1.0e15f;
 // (independent MMA chains), which are added per source leaf into FP64 sums
 // kept in shared memory.
 template <class K, int RC>
-__global__ void __launch_bounds__(128) k_p2p_mma(NearView nv, KernelParams kp, const uint2* __restrict__ qhl,
+__global__ void __launch_bounds__(128, 5) k_p2p_mma(NearView nv, KernelParams kp, const uint2* __restrict__ qhl,
                                                  double* __restrict__ ys) {
   constexpr int NE = 2 * (RC / 8) * 4;  // FP64 sums per lane
   extern __shared__ __align__(16) unsigned char smem[];
@@ -218,17 +218,28 @@ __global__ void __launch_bounds__(128) k_p2p_mma(NearView nv, KernelParams kp, c
           split_tf32_mask(kv[2 * u + 1][1], ah[u][3], al[u][3]);
         }
         const bool va = j0 + tq < nc, vb = j0 + tq + 4 < nc;
-        const uint2* ra = qhl + (long)(src + j0 + tq) * RC + gq;
+        // column tile t of 16 columns takes the columns 2 gq + t: a lane's two charges are neighbours
+        const uint2* ra = qhl + (long)(src + j0 + tq) * RC + RC / 8 * gq;
         const uint2* rb = ra + 4 * RC;
+        uint2 b0[RC / 8], b1[RC / 8];
+        if constexpr (RC == 16) {
+          const uint4 w0 = va ? *reinterpret_cast<const uint4*>(ra) : make_uint4(0u, 0u, 0u, 0u);
+          const uint4 w1 = vb ? *reinterpret_cast<const uint4*>(rb) : make_uint4(0u, 0u, 0u, 0u);
+          b0[0] = make_uint2(w0.x, w0.y);
+          b0[1] = make_uint2(w0.z, w0.w);
+          b1[0] = make_uint2(w1.x, w1.y);
+          b1[1] = make_uint2(w1.z, w1.w);
+        } else {
+          b0[0] = va ? *ra : make_uint2(0u, 0u);
+          b1[0] = vb ? *rb : make_uint2(0u, 0u);
+        }
 #pragma unroll
         for (int t = 0; t < RC / 8; ++t) {
-          const uint2 b0 = va ? ra[t * 8] : make_uint2(0u, 0u);
-          const uint2 b1 = vb ? rb[t * 8] : make_uint2(0u, 0u);
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            mma_tf32_16x8x8(cm[u][t], ah[u], b0.x, b1.x);
-            mma_tf32_16x8x8(cc[u][t], ah[u], b0.y, b1.y);
-            mma_tf32_16x8x8(cc[u][t], al[u], b0.x, b1.x);
+            mma_tf32_16x8x8(cm[u][t], ah[u], b0[t].x, b1[t].x);
+            mma_tf32_16x8x8(cc[u][t], ah[u], b0[t].y, b1[t].y);
+            mma_tf32_16x8x8(cc[u][t], al[u], b0[t].x, b1[t].x);
           }
         }
       }
@@ -240,20 +251,22 @@ __global__ void __launch_bounds__(128) k_p2p_mma(NearView nv, KernelParams kp, c
           for (int e = 0; e < 4; ++e)
             sacc[((u * (RC / 8) + t) * 4 + e) * 32 + lane] += (double)cm[u][t][e] + (double)cc[u][t][e];
     }
-    // D fragment of tile u: rows gq (e = 0, 1) and gq + 8 (e = 2, 3), columns 2tq, 2tq + 1
+    // D fragment of tile u: rows gq (e = 0, 1) and gq + 8 (e = 2, 3), columns RC/4 tq ..: two of a tile,
+    // four of two interleaved tiles
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int hr = 0; hr < 2; ++hr) {
         const int ti = tg * 32 + (2 * u + hr) * 8 + gq;
         if (ti < n) {
+          double2* o = reinterpret_cast<double2*>(ys + (long)(s0 + ti) * RC + RC / 4 * tq);
+          auto sum = [&](int t, int e) { return sacc[((u * (RC / 8) + t) * 4 + 2 * hr + e) * 32 + lane]; };
 #pragma unroll
-          for (int t = 0; t < RC / 8; ++t) {
-            double2* o = reinterpret_cast<double2*>(ys + (long)(s0 + ti) * RC + t * 8 + 2 * tq);
-            double2 w = *o;
-            w.x += sacc[((u * (RC / 8) + t) * 4 + 2 * hr) * 32 + lane];
-            w.y += sacc[((u * (RC / 8) + t) * 4 + 2 * hr + 1) * 32 + lane];
-            *o = w;
+          for (int h = 0; h < RC / 8; ++h) {
+            double2 w = o[h];
+            w.x += RC == 16 ? sum(0, h) : sum(0, 0);
+            w.y += RC == 16 ? sum(1, h) : sum(0, 1);
+            o[h] = w;
           }
         }
       }

@@ -311,7 +311,8 @@ void apply_shard(afmm_handle* h) {
     const long sc = 1L << (2 * (j - lev)), bl = k0 * sc, bh = k1 * sc;
     LevelView& d = p.lv_down[j];
     narrow_table(d.ncgrp_box, d.ncgrp_row, d.nncgroups, bl, bh);
-    narrow_table(d.nwgrp_box, d.nwgrp_row, d.nnwgroups, bl, bh);
+    d.box0 = bl;
+    d.nrun = bh - bl;
     if (j >= 2) {
       LevelView m = p.lv[j];
       narrow_table(m.cgrp_box, m.cgrp_row, m.ncgroups, bl, bh);
@@ -380,6 +381,7 @@ void build_plan(afmm_handle* h) {
     LevelView& v = p.lv[j];
     v = LevelView();
     v.nbox = d.nbox;
+    v.nrun = d.nbox;
     v.il = d.il;
     v.rank = d.rank;
     v.skel_off = d.skel_off;
@@ -408,12 +410,6 @@ void build_plan(afmm_handle* h) {
     v.ncgrp_box = d.ncgrp_box;
     v.ncgrp_row = d.ncgrp_row;
     v.nncgroups = d.nncgroups;
-    v.wgrp_box = d.wgrp_box;
-    v.wgrp_row = d.wgrp_row;
-    v.nwgroups = d.nwgroups;
-    v.nwgrp_box = d.nwgrp_box;
-    v.nwgrp_row = d.nwgrp_row;
-    v.nnwgroups = d.nnwgroups;
     v.ptile_par = d.ptile_par;
     v.ptile_row = d.ptile_row;
     v.nptiles = d.nptiles;
@@ -785,25 +781,21 @@ void finish_assemble(afmm_handle* h) {
     // row groups of at most 8 skeleton rows of one box (on-the-fly M2L
     // tiles), balanced chunks of at most kChunkRows skeleton rows (M2L / M2M
     // tiles) or node rows (L2L tiles): a box of n rows is cut into
-    // ceil(n / kChunkRows) chunks of equal size rounded up to 8 rows; and
-    // balanced chunks of at most 32 skeleton rows (a warp's lanes, the
-    // one-column M2L)
-    // (and the same of at most 32 node rows, the one-column L2L); and tiles
+    // ceil(n / kChunkRows) chunks of equal size rounded up to 8 rows; and tiles
     // of 128 skeleton rows (the last shorter: the integer tensor-core M2L)
-    for (int kind = 0; kind < 6; ++kind) {
-      const int span = kind == 0 ? 8 : (kind == 5 ? 128 : (kind >= 3 ? 32 : kChunkRows));
-      const bool nodes = kind == 2 || kind == 4;
+    for (int kind = 0; kind < 4; ++kind) {
+      const int span = kind == 0 ? 8 : (kind == 3 ? 128 : kChunkRows);
+      const bool nodes = kind == 2;
       std::vector<int32_t> gb, gr;
       for (long b = 0; b < v.nbox; ++b) {
         const int rows = nodes ? v.h_node_off[b + 1] - v.h_node_off[b] : v.h_rank[b];
         const int first = nodes ? v.h_node_off[b] : v.h_skel_off[b];
         const int nch = (rows + span - 1) / span;
-        int step = nch > 0 ? (rows + nch - 1) / nch : 0;
-        if (kind == 1 || kind == 2) step = (step + 7) / 8 * 8;
-        if (kind == 5) step = span;  // whole 128-row tiles, the last one shorter
-        for (int i = 0; i < rows; i += (kind == 0 ? 8 : step)) {
+        int step = nch > 0 ? ((rows + nch - 1) / nch + 7) / 8 * 8 : 8;
+        if (kind == 0 || kind == 3) step = span;  // whole groups and tiles, the last one shorter
+        for (int i = 0; i < rows; i += step) {
           gb.push_back((int32_t)b);
-          gr.push_back(kind == 5 ? i : first + i);  // 128-row tiles: the row within the box
+          gr.push_back(kind == 3 ? i : first + i);  // 128-row tiles: the row within the box
         }
       }
       int32_t* db = h->arena.alloc<int32_t>(gb.size());
@@ -825,18 +817,10 @@ void finish_assemble(afmm_handle* h) {
         v.nncgroups = (long)gb.size();
         v.ncgrp_box = db;
         v.ncgrp_row = dr;
-      } else if (kind == 3) {
-        v.nwgroups = (long)gb.size();
-        v.wgrp_box = db;
-        v.wgrp_row = dr;
-      } else if (kind == 5) {
+      } else {
         v.ntiles = (long)gb.size();
         v.tile_box = db;
         v.tile_row = dr;
-      } else {
-        v.nnwgroups = (long)gb.size();
-        v.nwgrp_box = db;
-        v.nwgrp_row = dr;
       }
     }
     {

@@ -170,6 +170,7 @@ void m2l_compress(const LevelView& v, cudaStream_t s) {
 // qs[i] = q[perm[i]]  (src/AFMM2D.cpp:49-51)
 __global__ void k_gather(const double* __restrict__ q, const int64_t* __restrict__ perm, int n, double* qs) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  dep_release();
   if (i < n) qs[i] = q[perm[i]];
 }
 
@@ -219,7 +220,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, 6) k_m2l_pair(LevelSet ls) {
   while (j + 1 < ls.nlev && g >= ls.m0[j + 1]) ++j;
   const LevelView& v = ls.lv[j];
   const long t = g - ls.m0[j];
-  m2l_pair_box<Q32>(v, v.m2l_run ? (long)v.m2l_run[t] : t, ls.pf_ahead, smem);
+  dep_release();
+  m2l_pair_box<Q32>(v, v.m2l_run ? (long)v.m2l_run[t] : t, ls.pf_ahead, smem, [] { dep_wait(); });
 }
 
 __global__ void __launch_bounds__(128) k_forward_boxes(LevelView v) {
@@ -244,6 +246,8 @@ void forward_boxes(const LevelView& v, cudaStream_t s) {
 
 // The sums that other boxes worked out, added to every level's rows.
 __global__ void __launch_bounds__(256) k_m2l_back(LevelSet ls) {
+  dep_release();
+  dep_wait();
   const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= ls.row0[ls.nlev]) return;
   int j = 0;
@@ -251,50 +255,34 @@ __global__ void __launch_bounds__(256) k_m2l_back(LevelSet ls) {
   m2l_back_row(ls.lv[j], g - ls.row0[j]);
 }
 
-// End of warp chunk g of a chunk table (the next chunk's first row, or the
-// end of the box).
-__device__ __forceinline__ int wchunk_end(const int32_t* first, long g, long n, int box_end) {
-  return g + 1 < n ? min(box_end, first[g + 1]) : box_end;
+// One-column M2M and L2L of a level, one CTA per box (m2m_box, l2l_box): a
+// level is then two latencies deep (tables, then the box's whole operator and
+// its vector at once) instead of a warp per 32 rows that walks the operator.
+// M2M + L2L as dependent launches: 1,048,576 uniform points (log, TOL 10) 0.39 ->
+// 0.26 ms, 300,000 (mixture, 1/r) 0.29 -> 0.16, 4,096 43 -> 21 us.
+__global__ void __launch_bounds__(32 * kUpWarps, 20 / kUpWarps) k_m2m_box(LevelView v, const double* __restrict__ src_all,
+                                                                 int leaf) {
+  dep_release();
+  m2m_box<false>(v, src_all, leaf, blockIdx.x, [] {
+    dep_wait();
+    return true;
+  });
 }
 
-// M2M (m2m_row's arithmetic, so the same bits) with one warp per chunk of up
-// to 32 skeleton rows of one box: no warp straddles two boxes, and the box's
-// L2P block and source rows are brought into L2 up front.
-__global__ void __launch_bounds__(128) k_m2m_w(LevelView v, const double* __restrict__ src_all, int leaf) {
-  const long g = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (g >= v.nwgroups) return;
-  const int b = v.wgrp_box[g];
-  const int r0 = v.wgrp_row[g];
-  const int end = wchunk_end(v.wgrp_row, g, v.nwgroups, v.skel_off[b] + v.rank[b]);
-  const int n = v.node_off[b + 1] - v.node_off[b];
-  const double* src = src_all + (leaf ? v.leaf_start[b] : v.node_off[b]);
-  prefetch_l2_region(v.l2p_rm + v.l2p_off[b], v.l2p_rm + v.l2p_off[b + 1], lane);
-  prefetch_l2_region(src, src + n, lane);
-  if (r0 + lane < end) m2m_row(v, src_all, leaf, r0 + lane);
+__global__ void __launch_bounds__(32 * kDownWarps, 28 / kDownWarps) k_l2l_box(LevelView v, double* __restrict__ child_yhat,
+                                                                 double* __restrict__ ys, int leaf) {
+  dep_release();
+  l2l_box<false>(v, child_yhat, ys, leaf, v.box0 + blockIdx.x, [] {
+    dep_wait();
+    return true;
+  });
 }
-
-// L2L (l2l_row's arithmetic) with one warp per chunk of up to 32 node rows of
-// one box, the box's L2P block brought into L2 up front.
-__global__ void __launch_bounds__(128) k_l2l_w(LevelView v, double* __restrict__ child_yhat, double* __restrict__ ys,
-                                               int leaf) {
-  const long g = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (g >= v.nnwgroups) return;
-  const int b = v.nwgrp_box[g];
-  const int g0 = v.nwgrp_row[g];
-  const int end = wchunk_end(v.nwgrp_row, g, v.nnwgroups, v.node_off[b + 1]);
-  prefetch_l2_region(v.l2p + v.l2p_off[b] + (g0 - v.node_off[b]), v.l2p + v.l2p_off[b + 1], lane);
-  if (g0 + lane < end) l2l_row(v, child_yhat, ys, leaf, g0 + lane);
-}
-
 
 void sweep_m2m(const MatvecPlan& p, const double* qs, cudaStream_t s, int64_t* launches) {
   for (int j = p.L; j >= 2; --j) {
     const LevelView& v = p.lv[j];
     if (v.nrows == 0) continue;
-    k_m2m_w<<<(int)((v.nwgroups * 32 + 127) / 128), 128, 0, s>>>(v, j == p.L ? qs : p.lv[j + 1].qhat, j == p.L);
-    AFMM_LAUNCH_CHECK();
+    launch_dependent(k_m2m_box, v.nbox, 32 * kUpWarps, 0, s, v, j == p.L ? qs : p.lv[j + 1].qhat, j == p.L);
     ++*launches;
   }
 }
@@ -303,17 +291,14 @@ void sweep_l2l(const MatvecPlan& p, double* ys, cudaStream_t s, int64_t* launche
   for (int j = 2; j <= p.L; ++j) {
     const LevelView& v = p.lv_down[j];  // a shard's subtrees at the sharded levels
     if (v.nnodes == 0) continue;
-    k_l2l_w<<<(int)((v.nnwgroups * 32 + 127) / 128), 128, 0, s>>>(v, j < p.L ? p.lv[j + 1].yhat : nullptr, ys,
-                                                                  j == p.L);
-    AFMM_LAUNCH_CHECK();
+    launch_dependent(k_l2l_box, v.nrun, 32 * kDownWarps, 0, s, v, j < p.L ? p.lv[j + 1].yhat : nullptr, ys, j == p.L);
     ++*launches;
   }
 }
 
 int m2l_back(const LevelSet& ls, cudaStream_t s) {
   const long rows = ls.row0[ls.nlev];
-  k_m2l_back<<<(int)((rows + 255) / 256), 256, 0, s>>>(ls);
-  AFMM_LAUNCH_CHECK();
+  launch_dependent(k_m2l_back, (rows + 255) / 256, 256, 0, s, ls);
   return 1;
 }
 
@@ -334,8 +319,7 @@ int m2l_apply_stored(const MatvecPlan& p, const LevelSet& levels, bool q32, cuda
   const size_t smem = m2l_pair_smem(*std::max_element(p.rmax, p.rmax + kMaxLevels));
   auto fn = q32 ? k_m2l_pair<true> : k_m2l_pair<false>;
   allow_smem(fn, smem);
-  fn<<<(int)boxes, 32 * kPairWarps, smem, s>>>(ls);
-  AFMM_LAUNCH_CHECK();
+  launch_dependent(fn, boxes, 32 * kPairWarps, smem, s, ls);
   return 1 + m2l_back(ls, s);
 }
 

@@ -22,6 +22,43 @@ inline void allow_smem(F* fn, size_t bytes) {
   }
 }
 
+// The split of the SM's memory between shared memory and L1 that the kernels of
+// one product ask for (about 100 KB shared): an SM changes it only when it is
+// empty, so kernels that differ in it do not run side by side on one SM.
+// (300,000 points, mixed: 530 -> 448 us; 28%, 58%, 100%: 512, 482, 528.)
+constexpr int kCarveoutPercent = 44;
+template <class F>
+inline void same_carveout(F* fn) {
+  AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPercent));
+}
+
+// Launch on stream s as a programmatic dependent of the kernel before it: its
+// CTAs may start (tables, operators into L2) as soon as all of that kernel's
+// have, and wait at dep_wait() for its end.  The product's chain of small
+// kernels (a level is a launch) then loses neither the launch gap nor the
+// latency of the tables: 4,096 points, one column, 57 -> 50 us; 100,003 points
+// 265 -> 225 us.
+template <class... P, class... A>
+inline void launch_dependent(void (*fn)(P...), long grid, int block, size_t smem, cudaStream_t s, A&&... args) {
+  same_carveout(fn);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  AFMM_CUDA(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
+}
+// Lets the next dependent launch start once every CTA has got here.
+__device__ __forceinline__ void dep_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Waits for the end of the kernel that this one depends on (none: returns at
+// once); only constant data is read before.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Device pointers of one level, passed by value to kernels.
 struct LevelView {
   long nbox = 0;
@@ -34,6 +71,7 @@ struct LevelView {
   const double* l2p = nullptr;     // column-major (row index fastest)
   const double* l2p_rm = nullptr;  // row-major copy (rank index fastest)
   const int64_t* m2l_off = nullptr;
+  long box0 = 0, nrun = 0;  // boxes of the one-column L2L (a shard's, else all)
   double* m2l = nullptr;
   const double2* skel_xy = nullptr;
   double* qhat = nullptr;
@@ -49,12 +87,6 @@ struct LevelView {
   const int32_t* ncgrp_box = nullptr;  // node-row chunk (<= kChunkRows node rows of one box) -> box
   const int32_t* ncgrp_row = nullptr;  // node-row chunk -> first node row
   long nncgroups = 0;
-  const int32_t* wgrp_box = nullptr;  // row chunk (<= 32 skeleton rows of one box) -> box
-  const int32_t* wgrp_row = nullptr;  // row chunk -> first skeleton row
-  long nwgroups = 0;
-  const int32_t* nwgrp_box = nullptr;  // node-row chunk (<= 32 node rows of one box) -> box
-  const int32_t* nwgrp_row = nullptr;  // node-row chunk -> first node row
-  long nnwgroups = 0;
   const int32_t* ptile_par = nullptr;  // parent row tile (<= 128 rows of 4 children) -> parent box
   const int32_t* ptile_row = nullptr;  // parent row tile -> first row of the children's concatenated rows
   long nptiles = 0;
@@ -409,29 +441,126 @@ __device__ __forceinline__ double ld_src(const double* p) {
   else return *p;
 }
 
-// M2M (src/AFMM2DTree.cpp:1129-1154): qhat[row] = (L2P_b^T src_b)[row] over
-// the row-major L2P copy; src_b = leaf charges, or the concatenated outgoing
-// charges of children 0..3.
-template <bool kL2 = false>
-__device__ __forceinline__ void m2m_row(const LevelView& v, const double* __restrict__ src_all, int leaf, long row) {
-  const int b = v.skel_box[row];
+// y += A x for the rows of one panel (NT tiles of 8 rows, nrow of them) by one
+// warp: A column-major with leading dimension lda, at the panel's first row.
+// Lane (rsub, csub) holds rows 8 k + rsub of columns 4 j + csub; up to 40 loads
+// per lane are independent, so a box's operator is asked for in one go.
+// Afterwards every lane holds its rows' sums.
+template <int NT, bool FULL, bool kL2>
+__device__ __forceinline__ void gemv_group(const double* __restrict__ P, long lda, int left, bool last,
+                                           const double* x, double (&y)[NT]) {
+  const int csub = (threadIdx.x & 31) >> 3;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const bool vc = FULL || 4 * j + csub < left;
+    const double xv = vc ? ld_src<kL2>(x + 4 * j) : 0.0;
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+      const double m = vc && (k + 1 < NT || last) ? __ldg(P + 4 * j * lda + 8 * k) : 0.0;
+      y[k] += m * xv;
+    }
+  }
+}
+template <int NT, bool kL2>
+__device__ __forceinline__ void gemv_panel(const double* __restrict__ A, long lda, int nrow, int cols,
+                                           const double* x, double (&y)[NT]) {
+  const int lane = threadIdx.x & 31, rsub = lane & 7, csub = lane >> 3;
+  const bool last = 8 * (NT - 1) + rsub < nrow;
+  const double* P = A + csub * lda + rsub;
+  x += csub;
+#pragma unroll
+  for (int k = 0; k < NT; ++k) y[k] = 0.0;
+  int c = 0;
+  for (; c + 32 <= cols; c += 32, P += 32 * lda, x += 32) gemv_group<NT, true, kL2>(P, lda, 32, last, x, y);
+  if (c < cols) gemv_group<NT, false, kL2>(P, lda, cols - c, last, x, y);
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    y[k] += __shfl_xor_sync(0xffffffffu, y[k], 8);
+    y[k] += __shfl_xor_sync(0xffffffffu, y[k], 16);
+  }
+}
+#define AFMM_TILES(nrow, CALL)   \
+  switch (((nrow) + 7) >> 3) {   \
+    case 1: CALL(1); break;      \
+    case 2: CALL(2); break;      \
+    case 3: CALL(3); break;      \
+    case 4: CALL(4); break;      \
+    default: CALL(5); break;     \
+  }
+
+constexpr int kUpWarps = 4, kDownWarps = 4;  // warps per box of the one-column sweeps
+
+// M2M (src/AFMM2DTree.cpp:1129-1154): the box's outgoing charges L2P_b^T src_b
+// over the row-major L2P copy; src_b = leaf charges, or the concatenated
+// outgoing charges of children 0..3.  By one CTA: the warps share the node
+// columns evenly, their sums are added in warp order.  ready() (by every
+// thread, false: give up) comes between what is constant and the charges.
+template <bool kL2, class Ready>
+__device__ __forceinline__ void m2m_box(const LevelView& v, const double* __restrict__ src_all, int leaf, long b,
+                                        Ready&& ready) {
+  __shared__ double part[kUpWarps][40];
   const int r = v.rank[b];
-  const int c = (int)(row - v.skel_off[b]);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = v.node_off[b + 1] - v.node_off[b];
   const double* src = src_all + (leaf ? v.leaf_start[b] : v.node_off[b]);
-  const double* P = v.l2p_rm + v.l2p_off[b] + c;  // (i, c) at i*r + c
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-  int i = 0;
-  // (unrolled: more loads in flight; each partial sum keeps its order)
-#pragma unroll 4
-  for (; i + 3 < n; i += 4) {
-    a0 += P[(long)i * r] * ld_src<kL2>(src + i);
-    a1 += P[(long)(i + 1) * r] * ld_src<kL2>(src + i + 1);
-    a2 += P[(long)(i + 2) * r] * ld_src<kL2>(src + i + 2);
-    a3 += P[(long)(i + 3) * r] * ld_src<kL2>(src + i + 3);
+  const double* P = v.l2p_rm + v.l2p_off[b];  // (row c, column i) at i*r + c
+  if (warp == 0) prefetch_l2_region(P, P + (long)n * r, lane);
+  if (!ready() || r == 0) return;
+  double* out = v.qhat + v.skel_off[b];
+  const int c0 = warp * n / kUpWarps, c1 = (warp + 1) * n / kUpWarps;
+  const int nch = (r + 39) / 40, step = ((r + nch - 1) / nch + 7) / 8 * 8;
+  for (int i0 = 0; i0 < r; i0 += step) {
+    const int nrow = min(step, r - i0);
+#define AFMM_M2M(NT)                                                                              \
+  {                                                                                               \
+    double y[NT];                                                                                 \
+    gemv_panel<NT, kL2>(P + (long)c0 * r + i0, r, nrow, c1 - c0, src + c0, y);                    \
+    _Pragma("unroll") for (int k = 0; k < NT; ++k) if (lane < 8) part[warp][8 * k + lane] = y[k]; \
   }
-  for (; i < n; ++i) a0 += P[(long)i * r] * ld_src<kL2>(src + i);
-  v.qhat[row] = (a0 + a1) + (a2 + a3);
+    AFMM_TILES(nrow, AFMM_M2M)
+#undef AFMM_M2M
+    __syncthreads();
+    if ((int)threadIdx.x < nrow) {
+      double s = part[0][threadIdx.x];
+#pragma unroll
+      for (int w = 1; w < kUpWarps; ++w) s += part[w][threadIdx.x];
+      out[i0 + threadIdx.x] = s;
+    }
+    __syncthreads();
+  }
+}
+
+// L2L (src/AFMM2DTree.cpp:1180-1197): t = L2P_b yhat_b over the column-major
+// L2P, added to the children's incoming potentials (the box's nodes are rows of
+// level j + 1), or written as the leaf's potentials.  By one CTA whose warps
+// take the box's row panels in turn; ready() as in m2m_box.
+template <bool kL2, class Ready>
+__device__ __forceinline__ void l2l_box(const LevelView& v, double* __restrict__ child_yhat, double* __restrict__ ys,
+                                        int leaf, long b, Ready&& ready) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r = v.rank[b];
+  const int n = v.node_off[b + 1] - v.node_off[b];
+  const double* P = v.l2p + v.l2p_off[b];  // (row i, column c) at c*n + i
+  const double* yb = v.yhat + v.skel_off[b];
+  double* out = leaf ? ys + v.leaf_start[b] : child_yhat + v.node_off[b];
+  const int per = kDownWarps * ((n + 40 * kDownWarps - 1) / (40 * kDownWarps));  // panels
+  const int step = per > 0 ? ((n + per - 1) / per + 7) / 8 * 8 : 8;
+  if (warp == 0) prefetch_l2_region(P, P + (long)n * r, lane);
+  if (!ready()) return;
+  for (int i0 = warp * step; i0 < n; i0 += kDownWarps * step) {
+    const int nrow = min(step, n - i0);
+#define AFMM_L2L(NT)                                                                                  \
+  {                                                                                                   \
+    double y[NT], c[NT];                                                                              \
+    _Pragma("unroll") for (int k = 0; k < NT; ++k) /* (asked for beside the operator) */              \
+      c[k] = !leaf && lane < 8 && 8 * k + lane < nrow ? ld_src<kL2>(out + i0 + 8 * k + lane) : 0.0;   \
+    gemv_panel<NT, kL2>(P + i0, n, nrow, r, yb, y);                                                   \
+    _Pragma("unroll") for (int k = 0; k < NT; ++k)                                                    \
+      if (lane < 8 && 8 * k + lane < nrow) out[i0 + 8 * k + lane] = leaf ? y[k] : c[k] + y[k];        \
+  }
+    AFMM_TILES(nrow, AFMM_L2L)
+#undef AFMM_L2L
+  }
 }
 
 // M2L (src/AFMM2DTree.cpp:1156-1178) of one column from the stored blocks,
@@ -584,8 +713,9 @@ __device__ __forceinline__ void m2l_pair_panel(const LevelView& v, long first, i
 // (u - 2^31) is exact, and the block's power of two goes to the charge of a
 // column and to its sum (both exact).  At its start a warp asks for the first
 // `ahead` bytes of its columns in L2.
-template <bool Q32>
-__device__ __forceinline__ void m2l_pair_box(const LevelView& v, long b, uint32_t ahead, unsigned char* smem) {
+template <bool Q32, class Ready>
+__device__ __forceinline__ void m2l_pair_box(const LevelView& v, long b, uint32_t ahead, unsigned char* smem,
+                                             Ready&& ready) {
   __shared__ ForwardBox s_fb[kPairWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ForwardBox& fb = s_fb[warp];
@@ -602,6 +732,7 @@ __device__ __forceinline__ void m2l_pair_box(const LevelView& v, long b, uint32_
     const uintptr_t n = min((uintptr_t)ahead, ((uintptr_t)(w1 - w0) * r * E + 15) & ~(uintptr_t)15);
     if (w0 >= ca || w1 <= ca) prefetch_l2_bulk(a, (uint32_t)n);
   }
+  ready();  // (the charges' producers are done)
   const int nr = min(r, kPairRows);
   double* sqb = (double*)smem;        // the box's own charges
   double* yp = sqb + nr + warp * nr;  // the warp's sums of the box's rows
@@ -681,33 +812,6 @@ __device__ __forceinline__ void m2l_back_row(const LevelView& v, long row) {
 #pragma unroll
   for (int f = 0; f < kForwardSlots; ++f) s += t[f];
   v.yhat[row] = s;
-}
-
-// L2L (src/AFMM2DTree.cpp:1180-1197): t = (L2P_b yhat_b)[node row g] over the
-// column-major L2P, added to the child's incoming potential (node row g of
-// level j is skeleton row g of level j+1), or written as the leaf potential.
-template <bool kL2 = false>
-__device__ __forceinline__ void l2l_row(const LevelView& v, double* __restrict__ child_yhat, double* __restrict__ ys,
-                                        int leaf, long g) {
-  const int b = v.node_box[g];
-  const int r = v.rank[b];
-  const int n = v.node_off[b + 1] - v.node_off[b];
-  const int i = (int)(g - v.node_off[b]);
-  const double* P = v.l2p + v.l2p_off[b] + i;  // (i, c) at c*n + i
-  const double* yb = v.yhat + v.skel_off[b];
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-  int c = 0;
-#pragma unroll 4
-  for (; c + 3 < r; c += 4) {
-    a0 += P[(long)c * n] * ld_src<kL2>(yb + c);
-    a1 += P[(long)(c + 1) * n] * ld_src<kL2>(yb + c + 1);
-    a2 += P[(long)(c + 2) * n] * ld_src<kL2>(yb + c + 2);
-    a3 += P[(long)(c + 3) * n] * ld_src<kL2>(yb + c + 3);
-  }
-  for (; c < r; ++c) a0 += P[(long)c * n] * ld_src<kL2>(yb + c);
-  const double t = (a0 + a1) + (a2 + a3);
-  if (leaf) ys[v.leaf_start[b] + i] = t;
-  else child_yhat[g] += t;
 }
 
 // Source slots of leaf b's near field (neighbours 0..7, then the leaf itself),

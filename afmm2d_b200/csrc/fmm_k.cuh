@@ -53,6 +53,7 @@ struct P2p64Run {
     const int warps = near_warps(nv.nmax);
     const size_t smem = near_smem(nv.nmax, warps);
     allow_smem(k_p2p64<K>, smem);
+    same_carveout(k_p2p64<K>);
     k_p2p64<K><<<(int)(nv.run ? nv.nrun : nv.nleaf), 32 * warps, smem, s>>>(nv, kp, qs, warps);
     AFMM_LAUNCH_CHECK();
   }

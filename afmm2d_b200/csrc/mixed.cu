@@ -60,6 +60,7 @@ __global__ void k_anchor_leaf(long nleaf, const int32_t* __restrict__ start, con
 __global__ void k_gather_mixed(const double* __restrict__ q, const int64_t* __restrict__ perm, int N, double* qs,
                                float* qs32) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  dep_release();
   if (i >= N) return;
   double v = q[perm[i]];
   qs[i] = v;

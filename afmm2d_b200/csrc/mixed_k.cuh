@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(32 * kOtfWarps, 6) k_m2l_otf(LevelSet ls, Kern
   if (threadIdx.x < sizeof(ForwardBox) / 8) ((int64_t*)&fb)[threadIdx.x] = ((const int64_t*)(v.fwd + b))[threadIdx.x];
   __syncthreads();
   const int r = fb.r;
+  dep_release();
+  dep_wait();
   if (r == 0) return;
   const PairSegs sg{fb.row, fb.col, nullptr, kForwardSlots, fb.col[kForwardSlots]};
   for (int R0 = 0; R0 < r; R0 += kPairRows) {  // (one round unless the rank is beyond kPairRows)
@@ -55,8 +57,7 @@ struct M2lOtfRun {
     if (boxes == 0) return;
     const size_t smem = near_smem(std::min(rmax, kPairRows), kOtfWarps);
     allow_smem(k_m2l_otf<K>, smem);
-    k_m2l_otf<K><<<(int)boxes, 32 * kOtfWarps, smem, s>>>(ls, kp);
-    AFMM_LAUNCH_CHECK();
+    launch_dependent(k_m2l_otf<K>, boxes, 32 * kOtfWarps, smem, s, ls, kp);
   }
 };
 
@@ -155,6 +156,7 @@ struct P2p32Run {
     const int threads = (nv.nmax + 31) / 32 * 32;
     const size_t smem = (size_t)9 * nv.nmax * (sizeof(float2) + sizeof(float));
     allow_smem(k_p2p32<K>, smem);
+    same_carveout(k_p2p32<K>);
     k_p2p32<K><<<(int)nv.nleaf, threads, smem, s>>>(nv, kp, qs32, out);
     AFMM_LAUNCH_CHECK();
   }

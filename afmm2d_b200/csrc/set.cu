@@ -36,12 +36,12 @@ __global__ void k_set_scatter(SetDev d, SetSegs sg, double* __restrict__ y) {
 
 // ------------------------------------------------ persistent sweeps
 // The M2M of every level of every problem runs in one launch (the up-sweep),
-// and so does the L2L (the down-sweep).  Items are tiles of kSweepTile rows
-// of one depth, listed in dependency order (M2M: each problem's leaf level
-// first; L2L: level 2 first); a CTA takes the next item from a ticket counter,
-// waits until every row that the item reads has been published (per problem
-// and level counters), computes its rows with the FP64 path's row arithmetic
-// (same bits) and publishes them.  An item only waits for items earlier in
+// and so does the L2L (the down-sweep).  Items are boxes, listed by depth in
+// dependency order (M2M: each problem's leaf level first; L2L: level 2 first);
+// a CTA takes the next kSweepBoxes items from a ticket counter, waits until
+// the level that a box reads has been published (per problem and level
+// counters of boxes), computes it as the FP64 path does (same bits) and
+// publishes it.  An item only waits for items earlier in
 // the list, which CTAs already running hold, so the sweep cannot deadlock;
 // each wait is still bounded in time, and a wait that gives up sets
 // sync.err, makes every other wait give up and ends the launch early.
@@ -75,6 +75,16 @@ __device__ bool wait_published(const int* c, long need, int* err) {
   return false;
 }
 
+// Publishes the box that the CTA has just written.
+__device__ __forceinline__ void publish_box(int* done) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(done, 1);
+  }
+}
+
 // The next item of a sweep for the calling CTA (all threads), or -1.
 __device__ __forceinline__ int next_item(int* ticket, int nitems, int* s_item) {
   __syncthreads();  // every thread has read the previous item
@@ -84,65 +94,28 @@ __device__ __forceinline__ int next_item(int* ticket, int nitems, int* s_item) {
   return it < nitems ? it : -1;
 }
 
-// Publishes the tile [r0, r1) of depth table sg: rows per (problem, level).
-__device__ __forceinline__ void publish_rows(const SetSegs& sg, long r0, long r1, int s0, int s1, int* done) {
-  __threadfence();
-  __syncthreads();
-  for (int s = s0 + (int)threadIdx.x; s <= s1; s += blockDim.x) {
-    const long a = max(r0, sg.first[s]), b = min(r1, sg.first[s + 1]);
-    __threadfence();
-    atomicAdd(done + (long)sg.prob[s] * kMaxLevels + sg.level[s], (int)(b - a));
-  }
-}
-
-// Streams into L2 the interpolation blocks that the item's rows [r0, r1)
-// read -- the row-major copy for the M2M (skeleton rows), the column-major
-// L2P for the L2L (node rows): one contiguous region per problem and level
-// the item touches (a box's block follows its predecessor's).  Warp 0, before
-// the item waits for its inputs, so the fetch overlaps the wait.  Used by the
-// down-sweep (0.85 -> 0.67 ms on 256 problems of 2K-64K points); the
-// up-sweep's row-major reads are already contiguous per warp and measured
-// slower with it (0.41 -> 0.48 ms).
-__device__ __forceinline__ void prefetch_item_l2p(const SetDev& d, const SetSegs& sg, long r0, long r1, int s0,
-                                                  int s1, bool up, int lane) {
-  for (int s = s0; s <= s1; ++s) {
-    const LevelView& v = d.lv[(long)sg.prob[s] * kMaxLevels + sg.level[s]];
-    const long a = max(r0, sg.first[s]) - sg.first[s], e = min(r1, sg.first[s + 1]) - sg.first[s];
-    const int32_t* box = up ? v.skel_box : v.node_box;
-    const double* P = up ? v.l2p_rm : v.l2p;
-    prefetch_l2_region(P + v.l2p_off[box[a]], P + v.l2p_off[box[e - 1] + 1], lane);
-  }
-}
-
-// Up-sweep: M2M of every problem from its leaf level up to level 2 (skeleton
-// rows).  A non-leaf level reads the outgoing charges of the level below.
-__global__ void __launch_bounds__(kSweepTile) k_set_up(SetDev d, SweepPlan sw, SweepSync sy) {
+// Up-sweep: M2M of every problem from its leaf level up to level 2.  A
+// non-leaf level reads the outgoing charges of the level below.
+__global__ void __launch_bounds__(32 * kUpWarps, 20 / kUpWarps) k_set_up(SetDev d, SweepPlan sw, SweepSync sy) {
   __shared__ int s_item, s_ok;
   for (int it; (it = next_item(sy.ticket, sw.nitems, &s_item)) >= 0;) {
     const SetSegs sg = sw.segs[sw.item_depth[it]];
-    const long r0 = sw.item_row0[it], r1 = min(r0 + (long)kSweepTile, sg.total);
-    const int s0 = seg_of(sg, r0), s1 = seg_of(sg, r1 - 1);
-    if (threadIdx.x == 0) s_ok = 1;
-    __syncthreads();
-    for (int s = s0 + (int)threadIdx.x; s <= s1; s += blockDim.x) {
+    const long g0 = sw.item_first[it], g1 = min(g0 + (long)kSweepBoxes, sg.total);
+    int s = seg_of(sg, g0);
+    for (long g = g0; g < g1; ++g) {
+      while (g >= sg.first[s + 1]) ++s;
       const long pl = (long)sg.prob[s] * kMaxLevels + sg.level[s];
-      if (d.lv[pl].leaf_start == nullptr &&
-          !wait_published(sy.done_up + pl + 1, d.lv[pl + 1].nrows + sw.margin, sy.err))
-        s_ok = 0;
-    }
-    __threadfence();
-    __syncthreads();
-    if (!s_ok) return;  // the same in every thread of the CTA
-    const long g = r0 + threadIdx.x;
-    if (g < r1) {
-      const int s = seg_of(sg, g);
-      const int p = sg.prob[s], j = sg.level[s];
-      const LevelView& v = d.lv[(long)p * kMaxLevels + j];
+      const LevelView& v = d.lv[pl];
       const bool leaf = v.leaf_start != nullptr;
-      const double* src = leaf ? d.qs[p] : d.lv[(long)p * kMaxLevels + j + 1].qhat;
-      m2m_row<true>(v, src, leaf ? 1 : 0, g - sg.first[s]);
+      m2m_box<true>(v, leaf ? d.qs[sg.prob[s]] : d.lv[pl + 1].qhat, leaf ? 1 : 0, g - sg.first[s], [&] {
+        if (threadIdx.x == 0)
+          s_ok = leaf || wait_published(sy.done_up + pl + 1, d.lv[pl + 1].nbox + sw.margin, sy.err);
+        __syncthreads();
+        return s_ok != 0;
+      });
+      if (!s_ok) return;  // the same in every thread of the CTA
+      publish_box(sy.done_up + pl);
     }
-    publish_rows(sg, r0, r1, s0, s1, sy.done_up);
   }
 }
 
@@ -153,7 +126,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 6) k_set_m2l(SetDev d, SetSeg
   const long g = blockIdx.x;
   const int s = seg_of(sg, g);
   const LevelView v = d.lv[(long)sg.prob[s] * kMaxLevels + sg.level[s]];
-  m2l_pair_box<false>(v, g - sg.first[s], 12 * 1024, smem);
+  m2l_pair_box<false>(v, g - sg.first[s], 12 * 1024, smem, [] {});
 }
 
 __global__ void __launch_bounds__(256) k_set_m2l_back(SetDev d, SetSegs sg) {
@@ -163,36 +136,28 @@ __global__ void __launch_bounds__(256) k_set_m2l_back(SetDev d, SetSegs sg) {
   m2l_back_row(d.lv[(long)sg.prob[s] * kMaxLevels + sg.level[s]], g - sg.first[s]);
 }
 
-// Down-sweep: L2L of every problem from level 2 down to its leaf level (node
-// rows).  Level j > 2 reads incoming potentials that the L2L of level j - 1
-// adds into.
-__global__ void __launch_bounds__(kSweepTile) k_set_down(SetDev d, SweepPlan sw, SweepSync sy) {
+// Down-sweep: L2L of every problem from level 2 down to its leaf level.
+// Level j > 2 reads incoming potentials that the L2L of level j - 1 adds into.
+__global__ void __launch_bounds__(32 * kDownWarps, 28 / kDownWarps) k_set_down(SetDev d, SweepPlan sw, SweepSync sy) {
   __shared__ int s_item, s_ok;
   for (int it; (it = next_item(sy.ticket + 1, sw.nitems, &s_item)) >= 0;) {
     const SetSegs sg = sw.segs[sw.item_depth[it]];
-    const long r0 = sw.item_row0[it], r1 = min(r0 + (long)kSweepTile, sg.total);
-    const int s0 = seg_of(sg, r0), s1 = seg_of(sg, r1 - 1);
-    if (threadIdx.x == 0) s_ok = 1;
-    if (threadIdx.x < 32) prefetch_item_l2p(d, sg, r0, r1, s0, s1, false, threadIdx.x);
-    __syncthreads();
-    for (int s = s0 + (int)threadIdx.x; s <= s1; s += blockDim.x) {
+    const long g0 = sw.item_first[it], g1 = min(g0 + (long)kSweepBoxes, sg.total);
+    int s = seg_of(sg, g0);
+    for (long g = g0; g < g1; ++g) {
+      while (g >= sg.first[s + 1]) ++s;
       const long pl = (long)sg.prob[s] * kMaxLevels + sg.level[s];
-      if (sg.level[s] > 2 && !wait_published(sy.done_dn + pl - 1, d.lv[pl - 1].nnodes + sw.margin, sy.err))
-        s_ok = 0;
-    }
-    __threadfence();
-    __syncthreads();
-    if (!s_ok) return;  // the same in every thread of the CTA
-    const long g = r0 + threadIdx.x;
-    if (g < r1) {
-      const int s = seg_of(sg, g);
-      const int p = sg.prob[s], j = sg.level[s];
-      const LevelView& v = d.lv[(long)p * kMaxLevels + j];
+      const LevelView& v = d.lv[pl];
       const bool leaf = v.leaf_start != nullptr;
-      double* child = leaf ? nullptr : d.lv[(long)p * kMaxLevels + j + 1].yhat;
-      l2l_row<true>(v, child, d.ys[p], leaf ? 1 : 0, g - sg.first[s]);
+      l2l_box<true>(v, leaf ? nullptr : d.lv[pl + 1].yhat, d.ys[sg.prob[s]], leaf ? 1 : 0, g - sg.first[s], [&] {
+        if (threadIdx.x == 0)
+          s_ok = sg.level[s] == 2 || wait_published(sy.done_dn + pl - 1, d.lv[pl - 1].nbox + sw.margin, sy.err);
+        __syncthreads();
+        return s_ok != 0;
+      });
+      if (!s_ok) return;  // the same in every thread of the CTA
+      publish_box(sy.done_dn + pl);
     }
-    publish_rows(sg, r0, r1, s0, s1, sy.done_dn);
   }
 }
 
@@ -262,7 +227,7 @@ void record(SetPlan& sp, cudaStream_t s) {
   ++n;
   mark("m2m");
   if (sp.up.nitems > 0) {
-    k_set_up<<<sp.up.grid, kSweepTile, 0, s>>>(sp.dev, sp.up, sp.sync);
+    k_set_up<<<sp.up.grid, 32 * kUpWarps, 0, s>>>(sp.dev, sp.up, sp.sync);
     AFMM_LAUNCH_CHECK();
     ++n;
   }
@@ -276,7 +241,7 @@ void record(SetPlan& sp, cudaStream_t s) {
   }
   mark("l2l");
   if (sp.down.nitems > 0) {
-    k_set_down<<<sp.down.grid, kSweepTile, 0, s>>>(sp.dev, sp.down, sp.sync);
+    k_set_down<<<sp.down.grid, 32 * kDownWarps, 0, s>>>(sp.dev, sp.down, sp.sync);
     AFMM_LAUNCH_CHECK();
     ++n;
   }
@@ -328,13 +293,13 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
     sp.p2p_smem = std::max(sp.p2p_smem, near_smem(mp.near.nmax, warps[p]));
   }
   // M2M by depth below the leaf level; L2L by level from the top; each
-  // sweep's items are the depth tables' row tiles in that order
+  // sweep's items are the depth tables' boxes in that order, kSweepBoxes at a time
   sp.m2m.clear();
   sp.l2l.clear();
   std::vector<int32_t> up_d, dn_d;
   std::vector<int64_t> up_r, dn_r;
   auto tiles = [](long total, int depth, std::vector<int32_t>& dd, std::vector<int64_t>& rr) {
-    for (long r = 0; r < total; r += kSweepTile) {
+    for (long r = 0; r < total; r += kSweepBoxes) {
       dd.push_back(depth);
       rr.push_back(r);
     }
@@ -344,7 +309,7 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
     for (int p = 0; p < np; ++p) {
       const MatvecPlan& mp = *probs[p];
       const int j = mp.L - depth;
-      if (j >= 2) b.add(p, j, mp.lv[j].nrows);
+      if (j >= 2) b.add(p, j, mp.lv[j].nbox);
     }
     if (b.first.back() > 0) {
       tiles(b.first.back(), (int)sp.m2m.size(), up_d, up_r);
@@ -355,7 +320,7 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
     SegBuilder b;
     for (int p = 0; p < np; ++p) {
       const MatvecPlan& mp = *probs[p];
-      if (j <= mp.L) b.add(p, j, mp.lv[j].nnodes);
+      if (j <= mp.L) b.add(p, j, mp.lv[j].nbox);
     }
     if (b.first.back() > 0) {
       tiles(b.first.back(), (int)sp.l2l.size(), dn_d, dn_r);
@@ -365,16 +330,16 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
   int nsm = 0, dev = 0, per_sm_up = 0, per_sm_dn = 0;
   AFMM_CUDA(cudaGetDevice(&dev));
   AFMM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  AFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_up, k_set_up, kSweepTile, 0));
-  AFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_dn, k_set_down, kSweepTile, 0));
+  AFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_up, k_set_up, 32 * kUpWarps, 0));
+  AFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_dn, k_set_down, 32 * kDownWarps, 0));
   sp.up.segs = upload(sp.m2m, arena, s);
   sp.up.item_depth = upload(up_d, arena, s);
-  sp.up.item_row0 = upload(up_r, arena, s);
+  sp.up.item_first = upload(up_r, arena, s);
   sp.up.nitems = (int)up_d.size();
   sp.up.grid = (int)std::min<long>(sp.up.nitems, (long)std::max(per_sm_up, 1) * nsm);
   sp.down.segs = upload(sp.l2l, arena, s);
   sp.down.item_depth = upload(dn_d, arena, s);
-  sp.down.item_row0 = upload(dn_r, arena, s);
+  sp.down.item_first = upload(dn_r, arena, s);
   sp.down.nitems = (int)dn_d.size();
   sp.down.grid = (int)std::min<long>(sp.down.nitems, (long)std::max(per_sm_dn, 1) * nsm);
   const size_t ncnt = (size_t)np * kMaxLevels;

@@ -43,23 +43,23 @@ __device__ __forceinline__ int seg_of(const SetSegs& sg, long g) {
 }
 
 // A persistent sweep (every level of every problem in one launch): items are
-// tiles of kSweepTile rows of one depth's flat row space (segs[depth]), listed
-// in dependency order; CTAs take them in list order from a ticket counter.
-constexpr int kSweepTile = 128;
+// kSweepBoxes boxes of one depth's flat box space (segs[depth]), listed in
+// dependency order; CTAs take them in list order from a ticket counter.
+constexpr int kSweepBoxes = 1;
 struct SweepPlan {
   const SetSegs* segs = nullptr;    // per depth (device array)
   const int32_t* item_depth = nullptr;
-  const int64_t* item_row0 = nullptr;
+  const int64_t* item_first = nullptr;
   int nitems = 0;
   int grid = 0;                     // resident CTAs launched
-  int margin = 0;                   // added to every awaited row count (0; > 0 only to test the time limit)
+  int margin = 0;                   // added to every awaited box count (0; > 0 only to test the time limit)
 };
 
 // Counters of the persistent sweeps, zeroed at the start of every replay.
 struct SweepSync {
   int* ticket = nullptr;  // [2]: up-sweep, down-sweep
-  int* done_up = nullptr; // nprob x kMaxLevels: M2M rows published per (problem, level)
-  int* done_dn = nullptr; // nprob x kMaxLevels: L2L node rows published per (problem, level)
+  int* done_up = nullptr; // nprob x kMaxLevels: boxes whose M2M is published, per (problem, level)
+  int* done_dn = nullptr; // nprob x kMaxLevels: boxes whose L2L is published, per (problem, level)
   int* err = nullptr;     // [1]: a wait gave up (AFMM_TIMEOUT)
   size_t bytes = 0;       // size of the block starting at ticket
 };
