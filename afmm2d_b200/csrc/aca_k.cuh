@@ -146,6 +146,39 @@ __device__ inline ArgMax cluster_argmax(cg::cluster_group& cluster, ArgMax m, do
   return *s_out;
 }
 
+// Dot products in twice the working precision (Ogita, Rump and Oishi's Dot2,
+// SIAM J. Sci. Comput. 26(6), 2005): a += x y with the product's and the sum's
+// rounding errors collected in a.lo.  Ten operations a term where the
+// double-double addition takes twice as many; the error stays near 2^-100 of
+// the sum of |x y| for the lengths here, so the final rounding is the correctly
+// rounded dot product whatever the order of the terms.
+__device__ __forceinline__ void dot2_add(dd& a, double x, double y) {
+  const double p = __dmul_rn(x, y);
+  const dd s = dd_two_sum(a.hi, p);
+  a.hi = s.hi;
+  a.lo = __dadd_rn(a.lo, __dadd_rn(s.lo, __fma_rn(x, y, -p)));
+}
+
+__device__ __forceinline__ dd dd_shfl_xor(dd v, int m) {
+  return dd{__shfl_xor_sync(0xffffffffu, v.hi, m), __shfl_xor_sync(0xffffffffu, v.lo, m)};
+}
+
+// Sums of eight values over a warp: lane l ends with value (l >> 2) reversed in
+// its three bits, ((l >> 4) & 1) * 4 + ((l >> 3) & 1) * 2 + ((l >> 2) & 1).
+__device__ __forceinline__ dd warp_sum8(dd (&a)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 4, m = 16; h > 0; h >>= 1, m >>= 1)
+#pragma unroll
+    for (int t = 0; t < h; ++t) {
+      const bool up = lane & m;
+      const dd send = up ? a[t] : a[t + h], keep = up ? a[t + h] : a[t];
+      a[t] = dd_add(keep, dd_shfl_xor(send, m));
+    }
+  a[0] = dd_add(a[0], dd_shfl_xor(a[0], 2));
+  return dd_add(a[0], dd_shfl_xor(a[0], 1));
+}
+
 template <class K>
 __global__ void __launch_bounds__(ACA_T, 2) k_aca(AcaArgs A) {
   cg::cluster_group cluster = cg::this_cluster();
@@ -181,6 +214,7 @@ __global__ void __launch_bounds__(ACA_T, 2) k_aca(AcaArgs A) {
   __shared__ ArgMax s_red[ACA_WARPS];
   __shared__ ArgMax s_piv;
   __shared__ double s_colxy[2];
+  __shared__ dd s_dot[2][ACA_WARPS][8];
 
   const int vsp = A.rcap - A.vcap, usp = A.rcap - A.ucap;
   double* my_vspill = A.vspill + ((size_t)cid * C + crank) * (size_t)max(vsp, 0) * A.chunk;
@@ -279,40 +313,111 @@ __global__ void __launch_bounds__(ACA_T, 2) k_aca(AcaArgs A) {
         m = am_finish(block_argmax(m, s_red));
         ri = (m.i == NONE) ? 0 : m.i;  // src/ACA.cpp:84 (an empty set yields index 0)
         double normS = 0.0, prev = DBL_MAX;
-        // ---- main loop (src/ACA.cpp:86-130)
-        while (fabs(prev - normS) >= A.tol * prev && rank < mn) {
+        // ---- main loop (src/ACA.cpp:86-130), each step's stopping test taken
+        // after the next step's residual row: both read every V row, so one
+        // pass over V serves both.  Step k: residual of row ri against rows
+        // l < k of V, and (k > 1) the dot products V_l . V_{k-1}, l < k, of the
+        // step before; the norm update and the stopping test of that step; the
+        // pivot; V_k; U_k.
+        // (One pass over V a step, eight rows at a time with eight double-double
+        // sums in flight per thread, instead of one pass for the residual and one
+        // per dot product: 262,144 uniform points, log 39 -> 36 ms, 500,000
+        // mixture, 1/r 91 -> 76, 100,003 uniform, scaled 1/r 19 -> 11.5 ms for all
+        // levels; FP64 pipe 35% busy, the rest latency at 16 warps an SM.  Three
+        // CTAs an SM (80 registers) 67 ms; rows four at a time 40; the columns'
+        // residuals in registers 47 (its unrolled body misses the instruction
+        // cache).)
+        while (rank < mn) {
           const int k = rank;
+          const bool dots = k > 1;
+          if (!dots && !(fabs(prev - normS) >= A.tol * prev)) break;
           const double2 rr = rows_xy[ri];
           double* Vk = Vrow(k);
+          const double* Vp = Vrow(k - 1);
           for (int l = tid; l < k; l += ACA_T) uri[l] = Urow(l)[ri];
           __syncthreads();
-          // residual row over this CTA's columns
           ArgMax mm = am_empty();
-          for (int j = tid; j < nloc; j += ACA_T) {
-            double2 c = cols_xy[j];
-            double v = K::eval_exact(r2_exact(rr.x, rr.y, c.x, c.y), A.kp);
-            // the reference's order of subtractions; sixteen V loads issued ahead
-            int l = 0;
-            for (; l + 16 <= k; l += 16) {
-              double w[16];
-#pragma unroll
-              for (int t = 0; t < 16; ++t) w[t] = Vrow(l + t)[j];
-#pragma unroll
-              for (int t = 0; t < 16; ++t) v = __dsub_rn(v, __dmul_rn(uri[l + t], w[t]));
+          int buf = 0;
+          // the sums of rows l0 .. l0 + nl - 1 over the CTA's columns
+          auto finish_dots = [&](dd (&acc)[8], int l0, int nl) {
+            const dd s = warp_sum8(acc);
+            if ((lane & 3) == 0) s_dot[buf][warp][((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = s;
+            __syncthreads();
+            if (tid < nl) {
+              dd t = s_dot[buf][0][tid];
+              for (int w = 1; w < ACA_WARPS; ++w) t = dd_add(t, s_dot[buf][w][tid]);
+              vdot[l0 + tid] = t.hi;
+              vdlo[l0 + tid] = t.lo;
             }
-            for (; l + 4 <= k; l += 4) {
-              double w[4];
+            buf ^= 1;
+          };
+          // rows l0 .. l0 + nl - 1 at a time, all of them in shared memory or all
+          // in the spill slot; the running residual stays in row k's place
+          for (int l0 = 0, nl; l0 < k; l0 += nl) {
+            nl = min(min(8, k - l0), l0 < A.vcap ? A.vcap - l0 : 8);
+            const double* Vl = Vrow(l0);
+            dd acc[8];
+            double u[8], w[8];
 #pragma unroll
-              for (int t = 0; t < 4; ++t) w[t] = Vrow(l + t)[j];
-#pragma unroll
-              for (int t = 0; t < 4; ++t) v = __dsub_rn(v, __dmul_rn(uri[l + t], w[t]));
+            for (int t = 0; t < 8; ++t) {
+              acc[t] = dd{0.0, 0.0};
+              u[t] = t < nl ? uri[l0 + t] : 0.0;
+              w[t] = t < nl && tid < nloc ? Vl[(size_t)t * A.chunk + tid] : 0.0;
             }
-            for (; l < k; ++l) v = __dsub_rn(v, __dmul_rn(uri[l], Vrow(l)[j]));
-            Vk[j] = v;
-            if (col_ok[j]) am_add(mm, v, lo + j);
+            for (int j = tid; j < nloc; j += ACA_T) {
+              double v;
+              if (l0 == 0) {
+                const double2 c = cols_xy[j];
+                v = K::eval_exact(r2_exact(rr.x, rr.y, c.x, c.y), A.kp);
+              } else {
+                v = Vk[j];
+              }
+              const double vp = dots ? Vp[j] : 0.0;
+              double wn[8];  // the next column's entries, asked for ahead
+#pragma unroll
+              for (int t = 0; t < 8; ++t)
+                wn[t] = t < nl && j + ACA_T < nloc ? Vl[(size_t)t * A.chunk + j + ACA_T] : 0.0;
+              // the reference's order of subtractions
+#pragma unroll
+              for (int t = 0; t < 8; ++t) v = __dsub_rn(v, __dmul_rn(u[t], w[t]));
+              Vk[j] = v;
+              if (dots) {
+#pragma unroll
+                for (int t = 0; t < 8; ++t) dot2_add(acc[t], w[t], vp);
+              }
+              if (l0 + nl >= k && col_ok[j]) am_add(mm, v, lo + j);
+#pragma unroll
+              for (int t = 0; t < 8; ++t) w[t] = wn[t];
+            }
+            if (dots) finish_dots(acc, l0, nl);
           }
-          mm = block_argmax(mm, s_red);
+          mm = block_argmax(mm, s_red);  // (its barriers also publish vdot)
+          const size_t xo = (size_t)xpar * 2 * (A.rcap + 8);
+          if (dots)
+            for (int l = tid; l < k; l += ACA_T) {
+              xdot[xo + 2 * l] = vdot[l];
+              xdot[xo + 2 * l + 1] = vdlo[l];
+            }
           const ArgMax pv = cluster_argmax(cluster, mm, xarg + xpar * 8, &s_piv);
+          if (dots) {
+            for (int l = tid; l < k; l += ACA_T) {
+              dd s{0.0, 0.0};
+              for (int c = 0; c < C; ++c) {
+                const double* xc = xdot_of(c) + xo;
+                s = dd_add(s, dd{xc[2 * l], xc[2 * l + 1]});
+              }
+              vdot[l] = __dadd_rn(s.hi, s.lo);
+              vdlo[l] = __dmul_rn(2.0, fabs(__dmul_rn(udot[l], vdot[l])));
+            }
+            __syncthreads();
+            // norm update of step k - 1 (src/ACA.cpp:122-128), identical in every thread
+            if (k != 2) prev = normS;
+            const double t = sqrt(udot[k - 1]) * sqrt(vdot[k - 1]);
+            double ns = __dadd_rn(__dmul_rn(normS, normS), __dmul_rn(t, t));
+            for (int l = 0; l < k; ++l) ns = __dadd_rn(ns, vdlo[l]);
+            normS = sqrt(ns);
+            if (!(fabs(prev - normS) >= A.tol * prev)) break;
+          }
           xpar ^= 1;
           // Every CTA sees the same pv; an empty allowed set cannot occur
           // while rank < min(n1, n2), but stop rather than index out of range.
@@ -344,10 +449,13 @@ __global__ void __launch_bounds__(ACA_T, 2) k_aca(AcaArgs A) {
               A.rowpiv[(size_t)b * A.rcap + k] = ri;
               A.colpiv[(size_t)b * A.rcap + k] = pid;
             }
+            if (ownk == crank) col_ok[jok] = 0;
+            row_ok[ri] = 0;
           }
           __syncthreads();
           // residual column u (all rows, every CTA)
           double* Uk = Urow(k);
+          ArgMax mr = am_empty();
           for (int i = tid; i < n1; i += ACA_T) {
             double2 r = rows_xy[i];
             double u = K::eval_exact(r2_exact(r.x, r.y, s_colxy[0], s_colxy[1]), A.kp);
@@ -361,86 +469,31 @@ __global__ void __launch_bounds__(ACA_T, 2) k_aca(AcaArgs A) {
             }
             for (; l < k; ++l) u = __dsub_rn(u, __dmul_rn(vcol[l], Urow(l)[i]));
             Uk[i] = u;
+            if (row_ok[i]) am_add(mr, u, i);
           }
-          __syncthreads();
-          // Partial V_l . v over this CTA's columns and U_l . u (redundant in every
-          // CTA), accumulated in double-double: the cluster-wide sums are then
-          // rounded once, so they are the correctly rounded dot products
-          // whatever the summation order (the stopping test depends on them).
-          for (int l = warp; l <= k; l += ACA_WARPS) {
-            const double* Vl = Vrow(l);
-            dd sv{0.0, 0.0};
-            int j = lane;
-            for (; j + 480 < nloc; j += 512) {  // same order of additions, loads issued ahead
-              double a[16], c[16];
-#pragma unroll
-              for (int t = 0; t < 16; ++t) {
-                a[t] = Vl[j + 32 * t];
-                c[t] = Vk[j + 32 * t];
-              }
-#pragma unroll
-              for (int t = 0; t < 16; ++t) {
-                const double p = __dmul_rn(a[t], c[t]);
-                sv = dd_add(sv, dd{p, __fma_rn(a[t], c[t], -p)});
-              }
-            }
-            for (; j < nloc; j += 32) {
-              const double a = Vl[j], c = Vk[j];
-              const double p = __dmul_rn(a, c);
-              sv = dd_add(sv, dd{p, __fma_rn(a, c, -p)});
-            }
-            for (int o = 16; o > 0; o >>= 1)
-              sv = dd_add(sv, dd{__shfl_down_sync(0xffffffffu, sv.hi, o), __shfl_down_sync(0xffffffffu, sv.lo, o)});
-            if (lane == 0) {
-              vdot[l] = sv.hi;
-              vdlo[l] = sv.lo;
-            }
-            const double* Ul = Urow(l);
-            dd su{0.0, 0.0};
-            for (int i = lane; i < n1; i += 32) {
-              const double a = Ul[i], c = Uk[i];
-              const double p = __dmul_rn(a, c);
-              su = dd_add(su, dd{p, __fma_rn(a, c, -p)});
-            }
-            for (int o = 16; o > 0; o >>= 1)
-              su = dd_add(su, dd{__shfl_down_sync(0xffffffffu, su.hi, o), __shfl_down_sync(0xffffffffu, su.lo, o)});
-            if (lane == 0) udot[l] = __dadd_rn(su.hi, su.lo);
-          }
-          __syncthreads();
-          const size_t xo = (size_t)xpar * 2 * (A.rcap + 8);
-          for (int l = tid; l <= k; l += ACA_T) {
-            xdot[xo + 2 * l] = vdot[l];
-            xdot[xo + 2 * l + 1] = vdlo[l];
-          }
-          if (tid == 0) {
-            if (ownk == crank) col_ok[jok] = 0;
-            row_ok[ri] = 0;
-          }
-          cluster.sync();
-          for (int l = tid; l <= k; l += ACA_T) {
-            dd s{0.0, 0.0};
-            for (int c = 0; c < C; ++c) {
-              const double* xc = xdot_of(c) + xo;
-              s = dd_add(s, dd{xc[2 * l], xc[2 * l + 1]});
-            }
-            vdot[l] = __dadd_rn(s.hi, s.lo);
-          }
-          xpar ^= 1;
-          __syncthreads();
-          rank = k + 1;
-          // norm update (src/ACA.cpp:122-128), identical in every thread
-          if (rank != 2) prev = normS;
-          double un = sqrt(udot[k]), vn = sqrt(vdot[k]);
-          double t = un * vn;
-          double ns = __dadd_rn(__dmul_rn(normS, normS), __dmul_rn(t, t));
-          for (int l = 0; l <= k; ++l) ns = __dadd_rn(ns, __dmul_rn(2.0, fabs(__dmul_rn(udot[l], vdot[l]))));
-          normS = sqrt(ns);
           // next pivot row: largest |u| over remaining rows (src/ACA.cpp:129)
-          ArgMax mr = am_empty();
-          for (int i = tid; i < n1; i += ACA_T)
-            if (row_ok[i]) am_add(mr, Uk[i], i);
           mr = am_finish(block_argmax(mr, s_red));
           ri = (mr.i == NONE) ? 0 : mr.i;
+          rank = k + 1;
+          if (rank >= mn) break;  // (the loop ends whatever the norm is)
+          // U_l . u (redundant in every CTA), four lanes per l; the rows rotated
+          // by l, so that the lanes of a warp read different banks
+          const int n4 = (n1 + 3) & ~3;
+          for (int l0 = 0; l0 <= k; l0 += ACA_T / 4) {
+            const int l = l0 + (tid >> 2);
+            dd su{0.0, 0.0};
+            if (l <= k) {
+              const double* Ul = Urow(l);
+              int i = (tid & 3) + 4 * (l & 7);
+              for (int t = 0; t < n4; t += 4, i += 4) {
+                while (i >= n4) i -= n4;
+                if (i < n1) dot2_add(su, Ul[i], Uk[i]);
+              }
+            }
+            su = dd_add(su, dd_shfl_xor(su, 2));
+            su = dd_add(su, dd_shfl_xor(su, 1));
+            if (l <= k && (tid & 3) == 0) udot[l] = __dadd_rn(su.hi, su.lo);
+          }
         }
       }
     }
