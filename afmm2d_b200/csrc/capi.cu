@@ -504,7 +504,7 @@ void do_create(afmm_handle* h, const double* loc, int layout) {
   check_device();
   create_streams(h);
   cudaStream_t s = h->stream;
-  double* d_xy = h->arena.alloc<double>(2 * (size_t)N);
+  double* d_xy = h->arena.alloc_own<double>(2 * (size_t)N);
   AFMM_CUDA(cudaMemcpyAsync(d_xy, xy.data(), sizeof(double) * 2 * N, cudaMemcpyHostToDevice, s));
   h->d_perm = h->arena.alloc<int64_t>(N);
   h->d_pts = h->arena.alloc<double2>(N);
@@ -725,6 +725,7 @@ void finish_assemble(afmm_handle* h) {
   const double t_tab = now_s();
   int64_t m2l_total = 0, l2p_total = 0, rows_total = 0;
   std::vector<std::vector<int64_t>> back_off(L + 1);  // one-column M2L: sums of the forward columns
+  std::vector<std::vector<int32_t>> tables;           // chunk tables, kept until their copies are done
   for (int j = 2; j <= L; ++j) {
     LevelDev& v = h->lv[j];
     const std::vector<int32_t>& il = h->h_il[j];
@@ -786,7 +787,9 @@ void finish_assemble(afmm_handle* h) {
     for (int kind = 0; kind < 4; ++kind) {
       const int span = kind == 0 ? 8 : (kind == 3 ? 128 : kChunkRows);
       const bool nodes = kind == 2;
-      std::vector<int32_t> gb, gr;
+      tables.emplace_back();
+      tables.emplace_back();
+      std::vector<int32_t>&gb = tables[tables.size() - 2], &gr = tables.back();
       for (long b = 0; b < v.nbox; ++b) {
         const int rows = nodes ? v.h_node_off[b + 1] - v.h_node_off[b] : v.h_rank[b];
         const int first = nodes ? v.h_node_off[b] : v.h_skel_off[b];
@@ -803,7 +806,6 @@ void finish_assemble(afmm_handle* h) {
       if (!gb.empty()) {
         AFMM_CUDA(cudaMemcpyAsync(db, gb.data(), sizeof(int32_t) * gb.size(), cudaMemcpyHostToDevice, s));
         AFMM_CUDA(cudaMemcpyAsync(dr, gr.data(), sizeof(int32_t) * gr.size(), cudaMemcpyHostToDevice, s));
-        AFMM_CUDA(cudaStreamSynchronize(s));
       }
       if (kind == 0) {
         v.ngroups = (long)gb.size();

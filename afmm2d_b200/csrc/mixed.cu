@@ -106,8 +106,8 @@ void mixed_reserve(MixedState& ms, int N, int nrhs, DevArena& arena) {
 }
 
 void mixed_reserve_io(MixedState& ms, int N, int nrhs, DevArena& arena) {
-  ms.d_qin = arena.alloc<double>((size_t)N * nrhs);
-  ms.d_yout = arena.alloc<double>((size_t)N * nrhs);
+  ms.d_qin = arena.alloc_own<double>((size_t)N * nrhs);
+  ms.d_yout = arena.alloc_own<double>((size_t)N * nrhs);
   ms.host_cap = nrhs;
 }
 
