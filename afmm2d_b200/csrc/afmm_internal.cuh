@@ -81,8 +81,9 @@ struct KOneOverRScaled {
     return R2 == 0.0 ? 0.0 : rsqrt(R2) * w;
   }
   __device__ __forceinline__ static float eval32(float R2, float a, float) {
+    // a = 2^-L: R/a and a/R are exact scalings of R and of 1/R
     float R = sqrtf(R2);
-    return (R < a) ? __fdiv_rn(R, a) : __fdiv_rn(a, R);
+    return (R < a) ? R * __frcp_rn(a) : a * __frcp_rn(R);
   }
   __device__ __forceinline__ static float eval32_pos(float R2, float a, float p) { return eval32(R2, a, p); }
 };
@@ -112,8 +113,8 @@ struct KLog {
   __device__ __forceinline__ static float eval32(float R2, float a, float) {
     if (R2 < 1e-10f) return 0.0f;
     float l = logf(R2);
-    if (R2 < a * a) return __fdiv_rn(0.5f * R2 * l, a * a);
-    return 0.5f * l;
+    // a = 2^-L: the division by a * a is an exact scaling
+    return R2 < a * a ? (0.5f * R2 * l) * __frcp_rn(a * a) : 0.5f * l;
   }
   // ln(R2) = lg2(R2) ln 2; lg2.approx has absolute error ~2^-22.  a = 2^-L,
   // so 1/a^2 is an exact power of two (loop-invariant): the near branch

@@ -282,7 +282,7 @@ void sweep_m2m(const MatvecPlan& p, const double* qs, cudaStream_t s, int64_t* l
   for (int j = p.L; j >= 2; --j) {
     const LevelView& v = p.lv[j];
     if (v.nrows == 0) continue;
-    launch_dependent(k_m2m_box, v.nbox, 32 * kUpWarps, 0, s, v, j == p.L ? qs : p.lv[j + 1].qhat, j == p.L);
+    launch_dependent(p.small(), k_m2m_box, v.nbox, 32 * kUpWarps, 0, s, v, j == p.L ? qs : p.lv[j + 1].qhat, j == p.L);
     ++*launches;
   }
 }
@@ -291,14 +291,14 @@ void sweep_l2l(const MatvecPlan& p, double* ys, cudaStream_t s, int64_t* launche
   for (int j = 2; j <= p.L; ++j) {
     const LevelView& v = p.lv_down[j];  // a shard's subtrees at the sharded levels
     if (v.nnodes == 0) continue;
-    launch_dependent(k_l2l_box, v.nrun, 32 * kDownWarps, 0, s, v, j < p.L ? p.lv[j + 1].yhat : nullptr, ys, j == p.L);
+    launch_dependent(p.small(), k_l2l_box, v.nrun, 32 * kDownWarps, 0, s, v, j < p.L ? p.lv[j + 1].yhat : nullptr, ys, j == p.L);
     ++*launches;
   }
 }
 
-int m2l_back(const LevelSet& ls, cudaStream_t s) {
+int m2l_back(const LevelSet& ls, bool early, cudaStream_t s) {
   const long rows = ls.row0[ls.nlev];
-  launch_dependent(k_m2l_back, (rows + 255) / 256, 256, 0, s, ls);
+  launch_dependent(early, k_m2l_back, (rows + 255) / 256, 256, 0, s, ls);
   return 1;
 }
 
@@ -319,8 +319,8 @@ int m2l_apply_stored(const MatvecPlan& p, const LevelSet& levels, bool q32, cuda
   const size_t smem = m2l_pair_smem(*std::max_element(p.rmax, p.rmax + kMaxLevels));
   auto fn = q32 ? k_m2l_pair<true> : k_m2l_pair<false>;
   allow_smem(fn, smem);
-  launch_dependent(fn, boxes, 32 * kPairWarps, smem, s, ls);
-  return 1 + m2l_back(ls, s);
+  launch_dependent(p.small(), fn, boxes, 32 * kPairWarps, smem, s, ls);
+  return 1 + m2l_back(ls, p.small(), s);
 }
 
 void matvec_fp64(const MatvecPlan& p, const double* q, double* y, cudaStream_t s, StageTimer* tm, int64_t* launches) {
@@ -334,24 +334,20 @@ void matvec_fp64(const MatvecPlan& p, const double* q, double* y, cudaStream_t s
   k_gather<<<gb, 256, 0, s>>>(q, p.perm, N, p.qs);
   AFMM_LAUNCH_CHECK();
   ++*launches;
-  // the near field (FP64-bound) on its own lower-priority stream beside the
-  // far field (HBM- and latency-bound); 1,048,576 uniform points, log, TOL 10:
-  // 2.16 ms one after the other, 1.86 ms
-  const bool beside = !(tm && tm->serial);
-  auto near = [&](cudaStream_t st) {
-    kernel_table(p.kp.id).p2p64(p.near_own, p.kp, p.qs, st);
-    ++*launches;
-  };
-  if (beside) near_beside(p, s, tm, near);
-  if (tm) tm->mark(s, "m2m");
-  sweep_m2m(p, p.qs, s, launches);
-  if (tm) tm->mark(s, "m2l");
-  *launches += m2l_apply(p, s);
-  if (tm) tm->mark(s, "l2l");
-  sweep_l2l(p, p.ys, s, launches);
-  if (tm) tm->mark(s, "p2p");
-  if (beside) AFMM_CUDA(cudaStreamWaitEvent(s, p.ev_near, 0));  // (the "p2p" stage is this wait)
-  else near(s);
+  beside_near(
+      p, s, tm,
+      [&](cudaStream_t st) {
+        kernel_table(p.kp.id).p2p64(p.near_own, p.kp, p.qs, st);
+        ++*launches;
+      },
+      [&](cudaStream_t st) {
+        if (tm) tm->mark(st, "m2m");
+        sweep_m2m(p, p.qs, st, launches);
+        if (tm) tm->mark(st, "m2l");
+        *launches += m2l_apply(p, st);
+        if (tm) tm->mark(st, "l2l");
+        sweep_l2l(p, p.ys, st, launches);
+      });
   if (tm) tm->mark(s, "scatter");
   k_scatter<<<gb, 256, 0, s>>>(p.ys, p.near.part, p.perm, N, y);
   AFMM_LAUNCH_CHECK();

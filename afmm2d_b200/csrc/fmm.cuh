@@ -32,14 +32,15 @@ inline void same_carveout(F* fn) {
   AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, kCarveoutPercent));
 }
 
-// Launch on stream s as a programmatic dependent of the kernel before it: its
+// Launch on stream s, with `early` as a programmatic dependent of the kernel before it: its
 // CTAs may start (tables, operators into L2) as soon as all of that kernel's
 // have, and wait at dep_wait() for its end.  The product's chain of small
 // kernels (a level is a launch) then loses neither the launch gap nor the
 // latency of the tables: 4,096 points, one column, 57 -> 50 us; 100,003 points
 // 265 -> 225 us.
 template <class... P, class... A>
-inline void launch_dependent(void (*fn)(P...), long grid, int block, size_t smem, cudaStream_t s, A&&... args) {
+inline void launch_dependent(bool early, void (*fn)(P...), long grid, int block, size_t smem, cudaStream_t s,
+                             A&&... args) {
   same_carveout(fn);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -48,7 +49,7 @@ inline void launch_dependent(void (*fn)(P...), long grid, int block, size_t smem
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   AFMM_CUDA(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
@@ -338,6 +339,7 @@ struct StageTimer {
   }
 };
 
+constexpr int kSmallProduct = 1 << 19;  // points
 struct MatvecPlan {
   int N = 0, L = 0;
   KernelParams kp;
@@ -350,10 +352,12 @@ struct MatvecPlan {
   int n1max[kMaxLevels] = {0};  // largest node count per level
   LevelSet levels;       // levels 2..L for the M2L launch
   NearView near;
-  // the near field of a one-column product runs on this lower-priority stream
-  // beside the far field, into near.part; the scatter adds the two
-  cudaStream_t s_near = nullptr;
-  cudaEvent_t ev_q = nullptr, ev_near = nullptr;
+  // the near field of a one-column product runs beside the far field, into
+  // near.part, one of them on a stream of lower / higher priority than the
+  // product's own (beside_near); the scatter adds the two
+  cudaStream_t s_near = nullptr, s_far = nullptr;
+  cudaEvent_t ev_q = nullptr, ev_side = nullptr;
+  bool small() const { return N < kSmallProduct; }
   Tuning tune;
   // A shard of one problem (afmm_set_shard): the stored-block M2L and the
   // L2L of the levels at and below shard_level, and the near field, run only
@@ -367,16 +371,35 @@ struct MatvecPlan {
   NearView near_own;
 };
 
-// Runs near(stream) on the plan's near-field stream, after what is queued on s
-// so far; p.ev_near marks its end.
-template <class F>
-inline void near_beside(const MatvecPlan& p, cudaStream_t s, StageTimer* tm, F&& near) {
+// The near and the far field of a one-column product, after what is queued on s
+// so far and before what follows: near(stream), far(stream).  Below
+// kSmallProduct points the far field's chain of small kernels is the longer
+// path: it follows on s at once, as dependent launches, and the near field
+// goes to the side.  Above, the near field follows on s and fills the GPU
+// first, and the far field takes slots as the near field's CTAs leave them (its
+// stream has the higher priority): it so runs in the near field's tail too,
+// where large leaves leave most SMs idle.  (ms, first
+// / second way: 1,048,576 points, mixture, 1/r 1.31 / 1.16, uniform, log 1.58 / 1.53;
+// 500,000 0.565 / 0.573; 300,000 mixed 0.450 / 0.499; 4,096 0.052 / 0.064.)
+template <class Near, class Far>
+inline void beside_near(const MatvecPlan& p, cudaStream_t s, StageTimer* tm, Near&& near, Far&& far) {
+  if (tm && tm->serial) {
+    far(s);
+    if (tm) tm->mark(s, "p2p");
+    near(s);
+    return;
+  }
+  const cudaStream_t sn = p.small() ? p.s_near : s, sf = p.small() ? s : p.s_far;
   AFMM_CUDA(cudaEventRecord(p.ev_q, s));
-  AFMM_CUDA(cudaStreamWaitEvent(p.s_near, p.ev_q, 0));
-  const int sp = tm ? tm->span_begin(p.s_near, "p2p_kernel") : -1;  // the kernel's own duration
-  near(p.s_near);
-  if (tm) tm->span_end(p.s_near, sp);
-  AFMM_CUDA(cudaEventRecord(p.ev_near, p.s_near));
+  AFMM_CUDA(cudaStreamWaitEvent(p.small() ? sn : sf, p.ev_q, 0));
+  const int sp = tm ? tm->span_begin(sn, "p2p_kernel") : -1;  // the kernel's own duration
+  near(sn);
+  if (tm) tm->span_end(sn, sp);
+  if (p.small()) AFMM_CUDA(cudaEventRecord(p.ev_side, sn));
+  far(sf);
+  if (tm) tm->mark(sf, "p2p");  // (the "p2p" stage is the wait for the near field)
+  if (!p.small()) AFMM_CUDA(cudaEventRecord(p.ev_side, sf));
+  AFMM_CUDA(cudaStreamWaitEvent(s, p.ev_side, 0));
 }
 
 // Level and box range [k0, k1) of shard `index` of `count` on a tree of
@@ -1090,7 +1113,7 @@ int m2l_apply_stored(const MatvecPlan& p, const LevelSet& levels, bool q32, cuda
 // M2L of the given levels with the entries evaluated on the fly in FP64 (mixed.cu).
 int m2l_apply_otf(const MatvecPlan& p, const LevelSet& levels, cudaStream_t s);
 // Their second launch: the sums that other boxes worked out (m2l_back_row).
-int m2l_back(const LevelSet& ls, cudaStream_t s);
+int m2l_back(const LevelSet& ls, bool early, cudaStream_t s);
 // The FP64 sweeps shared by both precisions (leaf charges qs in FP64).
 void sweep_m2m(const MatvecPlan& p, const double* qs, cudaStream_t s, int64_t* launches);
 void sweep_l2l(const MatvecPlan& p, double* ys, cudaStream_t s, int64_t* launches);

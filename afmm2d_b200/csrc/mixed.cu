@@ -80,7 +80,7 @@ inline int nb(long n, int t) { return (int)((n + t - 1) / t); }
 int m2l_apply_otf(const MatvecPlan& p, const LevelSet& levels, cudaStream_t s) {
   if (levels.row0[levels.nlev] == 0) return 0;
   kernel_table(p.kp.id).m2l_otf(levels, *std::max_element(p.rmax, p.rmax + kMaxLevels), p.kp, s);
-  return 1 + m2l_back(levels, s);
+  return 1 + m2l_back(levels, p.small(), s);
 }
 
 
@@ -128,17 +128,6 @@ void matvec_mixed(const MatvecPlan& p, MixedState& ms, const double* q, int64_t 
     k_gather_mixed<<<nb(N, 256), 256, 0, s>>>(q + (long)c * ldq, p.perm, N, ms.qs, ms.qs32);
     AFMM_LAUNCH_CHECK();
     ++*launches;
-    // the near field beside the far field, as in the FP64 path (nv.part as its output: same single
-    // addition to the far field's potentials)
-    const bool beside = !(tm && tm->serial);
-    auto near = [&](cudaStream_t st) {
-      kernel_table(p.kp.id).p2p32(nv, p.kp, ms.qs32, nv.part, st);
-      ++*launches;
-    };
-    if (beside) near_beside(p, s, tm, near);
-    if (tm) tm->mark(s, "m2m");
-    sweep_m2m(p, ms.qs, s, launches);
-    if (tm) tm->mark(s, "m2l");
     // stored form: the 32-bit fixed-point blocks when kept, else the FP64
     // ones; the levels of the tuning mask (or all, without stored blocks)
     // evaluate the entries on the fly
@@ -147,13 +136,22 @@ void matvec_mixed(const MatvecPlan& p, MixedState& ms, const double* q, int64_t 
     const uint32_t otf = stored ? p.tune.otf_mixed : 0xffffffffu;
     // a shard's boxes at the sharded levels for the stored form; the on-the-fly levels whole
     const LevelSet st = level_subset(p.levels_m2l, otf, false), fly = level_subset(p.levels, otf, true);
-    if (st.nlev > 0) *launches += m2l_apply_stored(p, st, q32, s);
-    if (fly.nlev > 0) *launches += m2l_apply_otf(p, fly, s);
-    if (tm) tm->mark(s, "l2l");
-    sweep_l2l(p, ms.ys, s, launches);
-    if (tm) tm->mark(s, "p2p");
-    if (beside) AFMM_CUDA(cudaStreamWaitEvent(s, p.ev_near, 0));
-    else near(s);
+    // (nv.part as the near field's output: one addition to the far field's potentials)
+    beside_near(
+        p, s, tm,
+        [&](cudaStream_t sn) {
+          kernel_table(p.kp.id).p2p32(nv, p.kp, ms.qs32, nv.part, sn);
+          ++*launches;
+        },
+        [&](cudaStream_t sf) {
+          if (tm) tm->mark(sf, "m2m");
+          sweep_m2m(p, ms.qs, sf, launches);
+          if (tm) tm->mark(sf, "m2l");
+          if (st.nlev > 0) *launches += m2l_apply_stored(p, st, q32, sf);
+          if (fly.nlev > 0) *launches += m2l_apply_otf(p, fly, sf);
+          if (tm) tm->mark(sf, "l2l");
+          sweep_l2l(p, ms.ys, sf, launches);
+        });
     if (tm) tm->mark(s, "scatter");
     k_scatter64<<<nb(N, 256), 256, 0, s>>>(ms.ys, nv.part, p.perm, N, y + (long)c * ldy);
     AFMM_LAUNCH_CHECK();

@@ -36,8 +36,6 @@ __global__ void __launch_bounds__(32 * kOtfWarps, 6) k_m2l_otf(LevelSet ls, Kern
   if (threadIdx.x < sizeof(ForwardBox) / 8) ((int64_t*)&fb)[threadIdx.x] = ((const int64_t*)(v.fwd + b))[threadIdx.x];
   __syncthreads();
   const int r = fb.r;
-  dep_release();
-  dep_wait();
   if (r == 0) return;
   const PairSegs sg{fb.row, fb.col, nullptr, kForwardSlots, fb.col[kForwardSlots]};
   for (int R0 = 0; R0 < r; R0 += kPairRows) {  // (one round unless the rank is beyond kPairRows)
@@ -57,7 +55,9 @@ struct M2lOtfRun {
     if (boxes == 0) return;
     const size_t smem = near_smem(std::min(rmax, kPairRows), kOtfWarps);
     allow_smem(k_m2l_otf<K>, smem);
-    launch_dependent(k_m2l_otf<K>, boxes, 32 * kOtfWarps, smem, s, ls, kp);
+    same_carveout(k_m2l_otf<K>);
+    k_m2l_otf<K><<<(int)boxes, 32 * kOtfWarps, smem, s>>>(ls, kp);
+    AFMM_LAUNCH_CHECK();
   }
 };
 
@@ -65,7 +65,7 @@ struct M2lOtfRun {
 // with itself (the diagonal) takes the kernel's value at zero distance
 // without any FP64 work, so the self-interaction costs no divergent branch.
 template <class K>
-__device__ __forceinline__ float near_pair(const NearView& nv, const KernelParams& kp, int p, int q) {
+__device__ __noinline__ float near_pair(const NearView& nv, const KernelParams& kp, int p, int q) {
   if (p == q) return (float)K::at_zero(kp);
   const double2 a = nv.pts[p], c = nv.pts[q];
   return (float)K::eval_exact(r2_exact(a.x, a.y, c.x, c.y), kp);
@@ -77,7 +77,10 @@ __device__ __forceinline__ float near_pair(const NearView& nv, const KernelParam
 // owns one target and sums all of its source leaves (the FP32 entries are
 // cheap, so splitting the leaves over thread groups only adds imbalance and a
 // reduction: 1.12 vs 1.62 ms at 1M uniform points, log), FP32 partial sums
-// per source leaf added in FP64.  Writes the sums of leaf b's points to
+// per source leaf added in FP64.  Issue-bound: a source is one 16-byte load,
+// and the rare close pairs' FP64 form is a call (1M points: log 1.11 -> 0.95 ms,
+// Gaussian 0.93 -> 0.74; 100,003 scaled 1/r, M = 100, 0.75 -> 0.64, with its
+// divisions by powers of two as scalings).  Writes the sums of leaf b's points to
 // `out`; the scatter adds them to the far field's.
 template <class K>
 __global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ qs32, double* __restrict__ out) {
@@ -106,12 +109,11 @@ __global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ 
   }
   __syncthreads();
   const int ns = s_ns;
-  float2* sx = (float2*)smem;
-  float* sq = (float*)(sx + 9 * nv.nmax);
+  float4* sx = (float4*)smem;  // x, y, charge
   for (int m = 0; m < ns; ++m)
     for (int t = threadIdx.x; t < s_cnt[m]; t += blockDim.x) {
-      sx[s_off[m] + t] = nv.rel[s_src[m] + t];
-      sq[s_off[m] + t] = qs32[s_src[m] + t];
+      const float2 p = nv.rel[s_src[m] + t];
+      sx[s_off[m] + t] = make_float4(p.x, p.y, qs32[s_src[m] + t], 0.0f);
     }
   __syncthreads();
   const int i = threadIdx.x;
@@ -124,7 +126,7 @@ __global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ 
       float a0 = 0.0f, a1 = 0.0f;
       int t = 0;
       for (; t + 1 < nc; t += 2) {
-        const float2 p0 = sx[o + t], p1 = sx[o + t + 1];
+        const float4 p0 = sx[o + t], p1 = sx[o + t + 1];
         const float dx0 = ox - p0.x, dy0 = oy - p0.y, dx1 = ox - p1.x, dy1 = oy - p1.y;
         const float R0 = fmaf(dx0, dx0, dy0 * dy0), R1 = fmaf(dx1, dx1, dy1 * dy1);
         float k0, k1;
@@ -132,17 +134,17 @@ __global__ void k_p2p32(NearView nv, KernelParams kp, const float* __restrict__ 
         else k0 = K::eval32(R0, a32, p32);
         if (R1 < thr) k1 = near_pair<K>(nv, kp, s0 + i, s_src[m] + t + 1);
         else k1 = K::eval32(R1, a32, p32);
-        a0 = fmaf(k0, sq[o + t], a0);
-        a1 = fmaf(k1, sq[o + t + 1], a1);
+        a0 = fmaf(k0, p0.z, a0);
+        a1 = fmaf(k1, p1.z, a1);
       }
       if (t < nc) {
-        const float2 p0 = sx[o + t];
+        const float4 p0 = sx[o + t];
         const float dx0 = ox - p0.x, dy0 = oy - p0.y;
         const float R0 = fmaf(dx0, dx0, dy0 * dy0);
         float k0;
         if (R0 < thr) k0 = near_pair<K>(nv, kp, s0 + i, s_src[m] + t);
         else k0 = K::eval32(R0, a32, p32);
-        a0 = fmaf(k0, sq[o + t], a0);
+        a0 = fmaf(k0, p0.z, a0);
       }
       acc += (double)a0 + (double)a1;
     }
@@ -154,7 +156,7 @@ template <class K>
 struct P2p32Run {
   static void run(const NearView& nv, const KernelParams& kp, const float* qs32, double* out, cudaStream_t s) {
     const int threads = (nv.nmax + 31) / 32 * 32;
-    const size_t smem = (size_t)9 * nv.nmax * (sizeof(float2) + sizeof(float));
+    const size_t smem = (size_t)9 * nv.nmax * sizeof(float4);
     allow_smem(k_p2p32<K>, smem);
     same_carveout(k_p2p32<K>);
     k_p2p32<K><<<(int)nv.nleaf, threads, smem, s>>>(nv, kp, qs32, out);
