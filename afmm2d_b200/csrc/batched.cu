@@ -68,11 +68,12 @@ __global__ void __launch_bounds__(256) k_gather_b(const double* __restrict__ q, 
 // points, reads their sorted rows ys[iperm[j]][0:RC], and writes each column
 // of y as one contiguous run.
 // With ys_near, the near field's potentials are added to the far field's
-// (the one addition the near-field kernels would have made into ys).
+// (the one addition the near-field kernels would have made into ys), the sum
+// of `parts` arrays of N x RC when there are several.
 template <int RC>
 __global__ void __launch_bounds__(256) k_scatter_b(const double* __restrict__ ys, const double* __restrict__ ys_near,
-                                                   const int32_t* __restrict__ iperm, int N, int ncols, double* y,
-                                                   int64_t ldy) {
+                                                   int parts, const int32_t* __restrict__ iperm, int N, int ncols,
+                                                   double* y, int64_t ldy) {
   __shared__ double tile[RC][kTileJ + 1];
   const long j0 = (long)blockIdx.x * kTileJ;
   for (int idx = threadIdx.x; idx < (RC / 2) * kTileJ; idx += blockDim.x) {
@@ -82,7 +83,18 @@ __global__ void __launch_bounds__(256) k_scatter_b(const double* __restrict__ ys
     const long o = (long)iperm[j] * RC + 2 * cp;
     double2 v = *reinterpret_cast<const double2*>(ys + o);
     if (ys_near) {
-      const double2 w = *reinterpret_cast<const double2*>(ys_near + o);
+      double2 w = *reinterpret_cast<const double2*>(ys_near + o);
+      if (parts == kNearParts) {
+        double2 x[kNearParts - 1];
+#pragma unroll
+        for (int k = 1; k < kNearParts; ++k)
+          x[k - 1] = *reinterpret_cast<const double2*>(ys_near + (long)k * N * RC + o);
+#pragma unroll
+        for (int k = 1; k < kNearParts; ++k) {
+          w.x += x[k - 1].x;
+          w.y += x[k - 1].y;
+        }
+      }
       v.x += w.x;
       v.y += w.y;
     }
@@ -707,20 +719,28 @@ struct Pass {
     k_gather_b<RC><<<nbk(N, kTileJ), 256, 0, s>>>(q, ldq, ncols, p.iperm, N, bs.qs, bs.qhl, fp64);
     AFMM_LAUNCH_CHECK();
     ++*launches;
+    // FP64 throughout, small leaves: every pair of leaves once, into parts that the scatter adds
+    const bool pairs = fp64 && bs.near_parts != nullptr;
+    if (pairs && p.shard_count > 1)
+      AFMM_CUDA(cudaMemsetAsync(bs.near_parts, 0, sizeof(double) * kNearParts * (size_t)N * RC, s));
     // the near field does not depend on the far field: it runs on its own
     // lower-priority stream into ys_near, filling what the far-field
     // kernels leave of the GPU (after the far field when profiling serially)
     const bool overlap = bs.s_near != nullptr && !(tm && tm->serial);
-    if (overlap) {
-      AFMM_CUDA(cudaEventRecord(bs.ev_q, s));
+    if (overlap) AFMM_CUDA(cudaEventRecord(bs.ev_q, s));
+    auto near_beside = [&] {
       AFMM_CUDA(cudaStreamWaitEvent(bs.s_near, bs.ev_q, 0));
-      AFMM_CUDA(cudaMemsetAsync(bs.ys_near, 0, sizeof(double) * (size_t)N * RC, bs.s_near));
+      if (!pairs) AFMM_CUDA(cudaMemsetAsync(bs.ys_near, 0, sizeof(double) * (size_t)N * RC, bs.s_near));
       const int sp = tm ? tm->span_begin(bs.s_near, "p2p_kernel") : -1;  // the kernel's own duration
-      p2p(p, bs, nv, fp64, bs.s_near, bs.ys_near);
+      if (pairs) kernel_table(p.kp.id).near_dmma[RC == 16](nv, p.kp, bs.qs, bs.near_parts, true, bs.s_near);
+      else p2p(p, bs, nv, fp64, bs.s_near, bs.ys_near);
       if (tm) tm->span_end(bs.s_near, sp);
       AFMM_CUDA(cudaEventRecord(bs.ev_near, bs.s_near));
       ++*launches;
-    }
+    };
+    // (the pair form's CTAs are few and long: behind the sweep up, whose first
+    // kernel would wait for them; 16,384 points, 16 columns 119 -> 109 us)
+    if (overlap && !pairs) near_beside();
     if (tm) tm->mark(s, "m2m");
     for (int j = p.L; j >= 2; --j) {
       const LevelView& v = p.lv[j];
@@ -736,6 +756,7 @@ struct Pass {
       AFMM_LAUNCH_CHECK();
       ++*launches;
     }
+    if (overlap && pairs) near_beside();
     if (tm) tm->mark(s, "m2l");
     *launches += m2l(p, bs.d_qhat_lv, bs.d_yhat_lv, fp64, bs.err_dev, s);
     if (tm) tm->mark(s, "l2l");
@@ -757,11 +778,13 @@ struct Pass {
     if (overlap) {
       AFMM_CUDA(cudaStreamWaitEvent(s, bs.ev_near, 0));
     } else {
-      p2p(p, bs, nv, fp64, s);
+      if (pairs) kernel_table(p.kp.id).near_dmma[RC == 16](nv, p.kp, bs.qs, bs.near_parts, true, s);
+      else p2p(p, bs, nv, fp64, s);
       ++*launches;
     }
     if (tm) tm->mark(s, "scatter");
-    k_scatter_b<RC><<<nbk(N, kTileJ), 256, 0, s>>>(bs.ys, overlap ? bs.ys_near : nullptr, p.iperm, N, ncols, y, ldy);
+    k_scatter_b<RC><<<nbk(N, kTileJ), 256, 0, s>>>(bs.ys, pairs ? bs.near_parts : (overlap ? bs.ys_near : nullptr),
+                                                   pairs ? kNearParts : 1, p.iperm, N, ncols, y, ldy);
     AFMM_LAUNCH_CHECK();
     ++*launches;
   }
@@ -821,6 +844,20 @@ void batch_reserve(const MatvecPlan& p, BatchState& bs, DevArena& arena, cudaStr
   AFMM_CUDA(cudaMemcpyAsync((void*)bs.d_yhat_lv, hy.data(), sizeof(double*) * kMaxLevels, cudaMemcpyHostToDevice, s));
   AFMM_CUDA(cudaStreamSynchronize(s));
   bs.ready = true;
+}
+
+void batch_reserve_parts(const MatvecPlan& p, BatchState& bs, DevArena& arena) {
+  if (bs.parts_tried) return;
+  bs.parts_tried = true;
+  // (both pass widths: a call's remainder runs as an 8-column pass)
+  const KernelTable& kt = kernel_table(p.kp.id);
+  for (int w = 0; w < 2; ++w)
+    if (!kt.near_dmma[w](p.near, p.kp, nullptr, nullptr, false, nullptr)) return;
+  try {
+    bs.near_parts = arena.alloc<double>((size_t)kNearParts * p.N * kBatchMax);
+  } catch (const Error& e) {
+    if (e.status != AFMM_OOM) throw;  // no room: the near field works every pair out twice
+  }
 }
 
 void matvec_batched(const MatvecPlan& p, MixedState& ms, BatchState& bs, const double* q, int64_t ldq, double* y,

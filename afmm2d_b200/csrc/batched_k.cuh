@@ -364,6 +364,130 @@ __global__ void __launch_bounds__(128) k_p2p_dmma(NearView nv, KernelParams kp, 
   }
 }
 
+// The FP64 near field of a pass with every unordered pair of leaves worked out
+// once (the pairs of near_leaf, fmm.cuh; K(x, y) depends on |x - y| only): one
+// CTA per leaf, each warp blocks of 32 points of the leaf's five source leaves
+// against all targets, 8 x 8 entries at a time.  An entry is evaluated in the
+// lane that holds it in the A fragment of the targets' product (8 targets x 4
+// sources); two exchanges between lanes turn it into the A fragment of the sources'
+// product (8 sources x 4 targets).  The sources' sums stay in registers over
+// all targets, the targets' in a shared-memory row of the warp, added in warp
+// order at the end.  part: kNearParts x n x RC.  FP64 datapath: an entry costs
+// ~22 operations and RC / 2 in each product, so evaluating it once takes the
+// 9 (22 + RC / 2) of a point's row to 5 (22 + RC), at the same ~69% of that datapath
+// (1,048,576 points, 16 columns: log 1.84 -> 1.47 ms, Gaussian 1.60 -> 1.36).
+template <class K, int RC>
+__global__ void __launch_bounds__(256, 2) k_near_dmma(NearView nv, KernelParams kp, const double* __restrict__ qs,
+                                                      double* __restrict__ part, int warps) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ NearSources src;
+  const long b = nv.run ? (long)nv.run[blockIdx.x] : nv.leaf0 + blockIdx.x;
+  const int n = nv.leaf_cnt[b], n8 = (n + 7) & ~7;
+  const int s0 = nv.leaf_start[b];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) src.make(nv, b, lane);
+  double2* px = (double2*)smem;                       // targets
+  double2* sx = px + n8 + warp * 32;                  // the warp's sources
+  double* accs = (double*)(px + n8 + warps * 32);     // the warps' sums of the targets
+  double* acc = accs + (size_t)warp * n8 * RC;
+  for (int i = threadIdx.x; i < n8; i += blockDim.x)
+    px[i] = i < n ? nv.pts[s0 + i] : make_double2(kPadTgt64, kPadTgt64);
+  for (int i = threadIdx.x; i < warps * n8 * RC; i += blockDim.x) accs[i] = 0.0;
+  __syncthreads();
+  const int ns = src.ns, total = src.off[ns], nblk = (total + 31) >> 5;
+  const int trow = lane >> 2, tsrc = lane & 3;
+  const int from = 4 * (tsrc + (trow & 4)) + (trow & 3);
+  const int b1 = (warp + 1) * nblk / warps;
+  for (int blk = warp * nblk / warps; blk < b1; ++blk) {
+    const int f = 32 * blk + lane;
+    int m = 0;
+    while (m + 1 < ns && f >= src.off[m + 1]) ++m;
+    const bool ok = f < total;
+    const int idx = ok ? src.src[m] + (f - src.off[m]) : -1;  // the lane's source
+    const int dst = ok ? src.dst[m] : 0;
+    __syncwarp();
+    sx[lane] = ok ? nv.pts[idx] : make_double2(kPadSrc64, kPadSrc64);
+    __syncwarp();
+    const bool both = __any_sync(0xffffffffu, dst > 0);  // (a block of the leaf's own points: one product)
+    double qc[8][RC / 8], yc[4][RC / 8][2];
+#pragma unroll
+    for (int h = 0; h < 8; ++h) {
+      const int j = __shfl_sync(0xffffffffu, idx, 4 * h + tsrc);
+      load_b<RC>(qs + (long)max(j, 0) * RC, trow, j >= 0, qc[h]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int t = 0; t < RC / 8; ++t) yc[u][t][0] = yc[u][t][1] = 0.0;
+    for (int i0 = 0; i0 < n8; i0 += 8) {
+      const double2 xi = px[i0 + trow];
+      double qb[2][RC / 8], yb[RC / 8][2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = i0 + 4 * h + tsrc;
+        load_b<RC>(qs + (long)(s0 + min(i, n - 1)) * RC, trow, i < n, qb[h]);
+      }
+      double2* o = reinterpret_cast<double2*>(acc + (size_t)(i0 + trow) * RC + RC / 4 * tsrc);
+#pragma unroll
+      for (int h = 0; h < RC / 8; ++h) {  // (columns in load_b's order)
+        const double2 w = o[h];
+        if (RC == 16) {
+          yb[0][h] = w.x;
+          yb[RC / 8 - 1][h] = w.y;
+        } else {
+          yb[0][0] = w.x;
+          yb[0][1] = w.y;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        double e[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const double2 p = sx[8 * u + 4 * h + tsrc];
+          const double dx = xi.x - p.x, dy = xi.y - p.y;
+          e[h] = K::eval(dx * dx + dy * dy, kp);
+#pragma unroll
+          for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(yb[t][0], yb[t][1], e[h], qc[2 * u + h][t]);
+        }
+        if (both) {
+          // entry (i, j), in lane 4 i + (j & 3) and e[j / 4], to lane 4 j + (i & 3) and
+          // v[i / 4]: each lane sends and receives one entry twice
+          const double x = __shfl_sync(0xffffffffu, trow < 4 ? e[0] : e[1], from);
+          const double y = __shfl_sync(0xffffffffu, trow < 4 ? e[1] : e[0], from ^ 16);
+          const double v[2] = {trow < 4 ? x : y, trow < 4 ? y : x};
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(yc[u][t][0], yc[u][t][1], v[h], qb[h][t]);
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < RC / 8; ++h)
+        o[h] = RC == 16 ? make_double2(yb[0][h], yb[RC / 8 - 1][h]) : make_double2(yb[0][0], yb[0][1]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = __shfl_sync(0xffffffffu, idx, 8 * u + trow), d = __shfl_sync(0xffffffffu, dst, 8 * u + trow);
+      if (d > 0 && d != kNoPart) {
+        double2* o = reinterpret_cast<double2*>(part + ((size_t)(d - 1) * nv.n + j) * RC + RC / 4 * tsrc);
+#pragma unroll
+        for (int h = 0; h < RC / 8; ++h)
+          o[h] = RC == 16 ? make_double2(yc[u][0][h], yc[u][RC / 8 - 1][h]) : make_double2(yc[u][0][0], yc[u][0][1]);
+      }
+    }
+  }
+  __syncthreads();
+  if (b < nv.leaf0 || b >= nv.leaf0 + nv.nleaf) return;
+  for (int e = threadIdx.x; e < n * RC; e += blockDim.x) {
+    double v = accs[e];
+    for (int w = 1; w < warps; ++w) v += accs[(size_t)w * n8 * RC + e];
+    part[(size_t)s0 * RC + e] = v;
+    for (int s = 0; s < 4; ++s)
+      if (!src.back[s]) part[((size_t)(1 + s) * nv.n + s0) * RC + e] = 0.0;
+  }
+}
+
 inline int nbk(long n, int t) { return (int)((n + t - 1) / t); }
 
 // M2L with the entries evaluated on the fly, RC = 8 or 16 columns per pass,
@@ -386,6 +510,52 @@ void p2p_mma_batched(const NearView& nv, const KernelParams& kp, const uint2* qh
   allow_smem(k_p2p_mma<K, RC>, smem);
   k_p2p_mma<K, RC><<<(int)nv.nleaf, 32 * warps, smem, s>>>(nv, kp, qhl, ys);
   AFMM_LAUNCH_CHECK();
+}
+
+template <int RC>
+size_t near_dmma_smem(int nmax, int warps) {
+  const size_t n8 = (nmax + 7) & ~7;
+  return (n8 + 32 * warps) * sizeof(double2) + (size_t)warps * n8 * RC * sizeof(double);
+}
+
+// Its warps: four or five, whichever share the blocks more evenly (an SM holds
+// 16 of the kernel's warps: smaller CTAs leave less of it idle at the end of each);
+// near_warps's up to eight when the leaves are few.
+inline int near_dmma_warps(int nmax, bool few) {
+  if (few) return near_warps(nmax);
+  const int blocks = (5 * nmax + 31) / 32;
+  if (blocks <= 5) return std::max(blocks, 1);
+  return 5 * ((blocks + 4) / 5) <= 4 * ((blocks + 3) / 4) ? 5 : 4;
+}
+
+// k_near_dmma for all leaves of nv, when it is the better form (false: k_p2p_dmma).
+// The line, in FP64 operations per point at 16 columns: k_p2p_dmma works out
+// nine leaves of points in groups of 32 targets, k_near_dmma five in groups of
+// 8 and moves 1 KB of parts (~2,500 operations' time).  16 columns, k_p2p_dmma ->
+// k_near_dmma, near field and scatter, log / Gaussian / 1/r: 64-point leaves
+// (1,048,576) 1.90 -> 1.64 / 1.65 -> 1.53 / 1.31 -> 1.39 ms; 98 (400,000) 1.47 ->
+// 1.01 / 1.27 -> .95 / 1.02 -> .84; 49 (800,000) 1.54 -> 1.22 / 1.34 -> 1.16 / 1.07 ->
+// 1.07; whole calls with 32-point leaves (524,288) 1.11 -> 1.13 / .87 -> .93 / 1.12 ->
+// 1.21.  With too few leaves to fill the GPU what counts is that five to eight
+// warps share a leaf instead of one per 32 targets (4,096 points, 91 -> 41 us; a
+// call 105 -> 80).  Two CTAs must fit an SM with the warps' target rows: leaves
+// of up to 104 points.
+template <class K, int RC>
+bool near_dmma_batched(const NearView& nv, const KernelParams& kp, const double* qs, double* part, bool launch,
+                       cudaStream_t s) {
+  const bool few = nv.n <= 2L * 148 * nv.nmax;
+  const int warps = near_dmma_warps(nv.nmax, few);
+  if (near_dmma_smem<16>(nv.nmax, warps) > 110 * 1024) return false;
+  constexpr double entry = K::id == AFMM_KERNEL_LOG ? 22.0 : K::id == AFMM_KERNEL_GAUSSIAN ? 16.0 : 8.0;
+  const double twice = 9.0 * ((nv.nmax + 31) & ~31) * (entry + 8.0);
+  const double once = 5.0 * ((nv.nmax + 7) & ~7) * (entry + 16.0) + 2500.0;
+  if (!few && 1.05 * once > twice) return false;
+  if (!launch) return true;
+  const size_t smem = near_dmma_smem<RC>(nv.nmax, warps);
+  allow_smem(k_near_dmma<K, RC>, smem);
+  k_near_dmma<K, RC><<<(int)(nv.run ? nv.nrun : nv.nleaf), 32 * warps, smem, s>>>(nv, kp, qs, part, warps);
+  AFMM_LAUNCH_CHECK();
+  return true;
 }
 
 // FP64 near field of an FP64-batched pass (8 or 16 columns).

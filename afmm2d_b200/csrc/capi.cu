@@ -1679,6 +1679,7 @@ afmm_status afmm_matvec(afmm_handle* h, const double* q, double* y, int nrhs, in
     if (precision != AFMM_PREC_FP64) {
       mixed_reserve(h->mixed, h->N, 1, h->arena);
       if (nrhs > 1) batch_reserve(h->plan, h->batch, h->arena, s);
+      if (nrhs > 1 && precision == AFMM_PREC_FP64_BATCHED) batch_reserve_parts(h->plan, h->batch, h->arena);
     }
     // nc columns (leading dimensions ldq, ldy) on the handle's stream.  A
     // one-column call in FP64 batched mode is the plain FP64 apply, and in

@@ -1016,6 +1016,45 @@ __device__ __forceinline__ double pair_target_sum(const PairSmem& sm, int n, int
   return v;
 }
 
+// Source leaves of leaf b in the pairwise near fields: the leaf itself, then its
+// neighbours in slots 0..3.  Per segment the first point, the position in the
+// flat list, and what the sums go to (PairSegs); whether slots 4..7 exist.
+struct NearSources {
+  int src[5], off[6], dst[5], back[4], ns;
+  // By one warp.
+  __device__ __forceinline__ void make(const NearView& nv, long b, int lane) {
+    // lane 0: the leaf; lanes 1..4: neighbour slots 0..3; lanes 5..8: slots 4..7
+    long c = -1;
+    int cnt = 0, start = 0;
+    if (lane < 9) {
+      c = lane == 0 ? b : (long)nv.nbr[b * 8 + lane - 1];
+      if (c >= 0 && lane < 5) {
+        start = nv.leaf_start[c];
+        cnt = nv.leaf_cnt[c];
+      }
+    }
+    const unsigned valid = __ballot_sync(0xffffffffu, lane < 5 && c >= 0);
+    int pre = cnt;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, pre, o);
+      if (lane >= o) pre += t;
+    }
+    if (lane < 5 && c >= 0) {
+      const int m = __popc(valid & ((1u << lane) - 1u));
+      src[m] = start;
+      off[m] = pre - cnt;
+      // (a leaf outside the shard gets no sums; part 0 is the leaf's own)
+      dst[m] = lane == 0 ? 0 : (c >= nv.leaf0 && c < nv.leaf0 + nv.nleaf ? lane + 1 : kNoPart);
+    }
+    if (lane == 4) {
+      ns = __popc(valid);
+      off[__popc(valid)] = pre;
+    }
+    if (lane >= 5 && lane < 9) back[lane - 5] = c >= 0;
+  }
+};
+
 // Near field (src/AFMM2DTree.cpp:1199-1213) of leaf b, kernel evaluated on the
 // fly, every unordered pair of leaves once: K(x, y) depends on |x - y| only, so
 // the pairs of leaf b with the neighbours in slots 0..3 give both leaves' sums
@@ -1037,51 +1076,20 @@ __device__ __forceinline__ double pair_target_sum(const PairSmem& sm, int n, int
 template <class K>
 __device__ __forceinline__ void near_leaf(const NearView& nv, const KernelParams& kp, const double* __restrict__ qs,
                                           int warps, long b, unsigned char* smem) {
-  __shared__ int s_src[5], s_off[6], s_dst[5], s_back[4], s_ns;
+  __shared__ NearSources src;
   const int n = nv.leaf_cnt[b];
   const int s0 = nv.leaf_start[b];
   const bool own = b >= nv.leaf0 && b < nv.leaf0 + nv.nleaf;
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    // lane 0: the leaf; lanes 1..4: neighbour slots 0..3; lanes 5..8: slots 4..7
-    long c = -1;
-    int cnt = 0, start = 0;
-    if (lane < 9) {
-      c = lane == 0 ? b : (long)nv.nbr[b * 8 + lane - 1];
-      if (c >= 0 && lane < 5) {
-        start = nv.leaf_start[c];
-        cnt = nv.leaf_cnt[c];
-      }
-    }
-    const unsigned valid = __ballot_sync(0xffffffffu, lane < 5 && c >= 0);
-    int pre = cnt;
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, pre, o);
-      if (lane >= o) pre += t;
-    }
-    if (lane < 5 && c >= 0) {
-      const int m = __popc(valid & ((1u << lane) - 1u));
-      s_src[m] = start;
-      s_off[m] = pre - cnt;
-      // (a leaf outside the shard gets no sums; part 0 is the leaf's own)
-      s_dst[m] = lane == 0 ? 0 : (c >= nv.leaf0 && c < nv.leaf0 + nv.nleaf ? lane + 1 : kNoPart);
-    }
-    if (lane == 4) {
-      s_ns = __popc(valid);
-      s_off[__popc(valid)] = pre;
-    }
-    if (lane >= 5 && lane < 9) s_back[lane - 5] = c >= 0;
-  }
+  if (threadIdx.x < 32) src.make(nv, b, threadIdx.x);
   const PairSmem sm(smem, n);
   __syncthreads();
-  pair_targets<K>(PairPoints{nv.pts, qs, nv.part, nv.n}, kp, PairSegs{s_src, s_off, s_dst, s_ns, s_off[s_ns]}, s0, n, n,
-                  warps, sm);
+  pair_targets<K>(PairPoints{nv.pts, qs, nv.part, nv.n}, kp,
+                  PairSegs{src.src, src.off, src.dst, src.ns, src.off[src.ns]}, s0, n, n, warps, sm);
   if (!own) return;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     nv.part[s0 + i] = pair_target_sum(sm, n, warps, i, sm.self[i]);
     for (int s = 0; s < 4; ++s)
-      if (!s_back[s]) nv.part[(size_t)(1 + s) * nv.n + s0 + i] = 0.0;
+      if (!src.back[s]) nv.part[(size_t)(1 + s) * nv.n + s0 + i] = 0.0;
   }
 }
 

@@ -18,7 +18,7 @@ namespace afmm {
 
 // Bumped whenever KernelTable or an argument type of its launchers changes:
 // a table compiled against other headers is refused at registration.
-constexpr int kKernelTableAbi = 5;
+constexpr int kKernelTableAbi = 6;
 
 // Fingerprint of the layouts of the launchers' argument types (sizes and a
 // few field offsets), recorded in every table where it is compiled: a table
@@ -48,6 +48,10 @@ struct KernelTable {
                          cudaStream_t) = {nullptr, nullptr};
   void (*p2p_mma[2])(const NearView&, const KernelParams&, const uint2*, double*, cudaStream_t) = {nullptr, nullptr};
   void (*p2p_dmma[2])(const NearView&, const KernelParams&, const double*, double*, cudaStream_t) = {nullptr, nullptr};
+  // FP64 near field with every pair of leaves once, into kNearParts parts;
+  // false: leaves too large for it (nothing is launched without `launch`)
+  bool (*near_dmma[2])(const NearView&, const KernelParams&, const double*, double*, bool launch,
+                       cudaStream_t) = {nullptr, nullptr};
   // mixed near field of 16-column passes on tcgen05 tiles (p2p_tc_k.cuh);
   // leaves of at most 64 points; sets *err on a bounded-wait timeout
   void (*p2p_tc16)(const NearView&, const KernelParams&, const uint2*, double*, int L, int* err,

@@ -39,6 +39,10 @@ struct BatchState {
   // The near field runs on its own lower-priority stream beside the far
   // field, into ys_near (zeroed per pass); the scatter adds it to ys.
   double* ys_near = nullptr;
+  // FP64-batched passes with every pair of leaves worked out once: kNearParts x
+  // N x kBatchMax sums (null when they did not fit: the near field into ys_near)
+  double* near_parts = nullptr;
+  bool parts_tried = false;
   cudaStream_t s_near = nullptr;
   cudaEvent_t ev_q = nullptr, ev_near = nullptr;
   ~BatchState() {
@@ -49,6 +53,8 @@ struct BatchState {
   }
 };
 void batch_reserve(const MatvecPlan& p, BatchState& bs, DevArena& arena, cudaStream_t s);
+// The parts of FP64-batched near fields, when the leaves are small enough and the memory is there.
+void batch_reserve_parts(const MatvecPlan& p, BatchState& bs, DevArena& arena);
 // The M2L stage alone of a batched pass of rc columns (on the batch buffers'
 // current outgoing charges); returns the launches made.
 int m2l_batched(const MatvecPlan& p, BatchState& bs, int rc, int fp64, cudaStream_t s);

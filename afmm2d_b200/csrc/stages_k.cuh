@@ -28,6 +28,8 @@ KernelTable make_kernel_table(const char* name) {
   t.p2p_mma[1] = &batched_detail::p2p_mma_batched<K, 16>;
   t.p2p_dmma[0] = &batched_detail::p2p_dmma_batched<K, 8>;
   t.p2p_dmma[1] = &batched_detail::p2p_dmma_batched<K, 16>;
+  t.near_dmma[0] = &batched_detail::near_dmma_batched<K, 8>;
+  t.near_dmma[1] = &batched_detail::near_dmma_batched<K, 16>;
   t.p2p_tc16 = &p2p_tc_detail::p2p_tc_batched16<K>;
   t.aca_occupancy = &aca_detail::AcaLaunch<K>::occupancy;
   t.aca_run = &aca_detail::AcaLaunch<K>::run;

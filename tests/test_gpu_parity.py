@@ -403,6 +403,28 @@ def test_pairwise_near_field_leaf_sizes(kernel, N, M):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kernel,N,M", [("log", 16, 1), ("gaussian", 112, 7), ("one_over_r", 130, 8), ("log", 500, 31),
+                                        ("one_over_r_scaled", 531, 33), ("gaussian", 1661, 103), ("log", 1680, 105),
+                                        ("log", 41984, 41), ("one_over_r", 100352, 98)])
+def test_pairwise_batched_near_field_leaf_sizes(kernel, N, M):
+    """FP64 batched near field with every pair of leaves once (8- and 16-column passes, one after the other in a
+    call of 19), at leaves of 1 to 104 points around its tiles of 8 and blocks of 32 and on both sides of its
+    largest leaf, few leaves and many, against the one-column products.  Only the summation order differs."""
+    rng = np.random.default_rng(N)
+    a = A.AFMM(N, M, 6, rng.uniform(0, 1, (N, 2)), kernel=kernel, kparam=0.01 if kernel == "gaussian" else None)
+    a.assemble()
+    Q = rng.standard_normal((N, 19))
+    y = [a.computeMatVecProduct(np.ascontiguousarray(Q[:, c])) for c in (0, 4, 18)]
+    for cols in (5, 19):
+        Yb = a.computeMatVecProduct(np.asfortranarray(Q[:, :cols]), precision="fp64_batched")
+        np.testing.assert_array_equal(
+            a.computeMatVecProduct(np.asfortranarray(Q[:, :cols]), precision="fp64_batched"), Yb)
+        for c, yc in zip((0, 4, 18), y):
+            if c < cols:
+                assert np.linalg.norm(yc - Yb[:, c]) <= FP64_BATCHED_TOL * np.linalg.norm(yc)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kernel,N,M,tol,least", [("gaussian", 700, 40, 2, 1), ("log", 5000, 64, 4, 8),
                                                   ("log", 16384, 256, 12, 41), ("one_over_r", 16000, 400, 12, 60)])
 def test_pairwise_m2l_ranks(kernel, N, M, tol, least):
