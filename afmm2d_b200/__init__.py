@@ -395,7 +395,7 @@ class AFMM:
         _check(lib().afmm_set_tuning(self._h, _ptr(v), len(v)), self._h)
 
     def set_profiling(self, on=True):
-        """True / 1: per-stage CUDA events; 2: the same with the batched near
+        """True / 1: per-stage CUDA events; 2: the same with the near
         field run after the far field (each stage its kernels' own time)."""
         _check(lib().afmm_set_profiling(self._h, int(on)), self._h)
 

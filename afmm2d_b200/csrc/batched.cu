@@ -1,12 +1,11 @@
-// Batched mixed-precision matvec: RC right-hand sides per pass (RC = 4, 8 or
-// 16), each operator entry read or evaluated once and applied to all of them.
+// Batched matvec, mixed or FP64: RC right-hand sides per pass (RC = 8 or 16),
+// each operator entry read or evaluated once and applied to all of them.
 //
 // Layout: point-major blocks, value (i, c) at i*RC + c, for the sorted charges
 // and potentials and for the outgoing / incoming vectors of every level, so a
 // warp's lanes (consecutive rows of one box) read the same RC-vector of a
 // source with one broadcast load.
-//  * M2M / L2L: FP64 L2P (row-major / column-major), one thread per output
-//    row with RC FP64 accumulators.
+//  * M2M / L2L: FP64 L2P (row-major / column-major) on the FP64 tensor cores.
 //  * M2L: the stored blocks (one HBM read for all RC columns; the 32-bit
 //    fixed-point copy in mixed precision, the FP64 blocks otherwise), or
 //    entries evaluated on the fly in FP64 from the skeleton coordinates when
@@ -15,8 +14,8 @@
 //  * Near field: entries in FP32 from leaf-relative coordinates with the FP64
 //    fallback for close pairs (as in the single-RHS mixed path), multiplied
 //    on the TF32 tensor cores in a three-term high/low split (16 targets x 8
-//    sources tiles), tile sums per source leaf accumulated in FP64.
-// With RC = 4 the same products run on the FMA pipes.
+//    sources tiles), tile sums per source leaf accumulated in FP64.  FP64
+//    passes: FP64 entries on the FP64 tensor cores.
 #include <algorithm>
 #include <type_traits>
 

@@ -374,8 +374,9 @@ __global__ void __launch_bounds__(128) k_p2p_dmma(NearView nv, KernelParams kp, 
 // all targets, the targets' in a shared-memory row of the warp, added in warp
 // order at the end.  part: kNearParts x n x RC.  FP64 datapath: an entry costs
 // ~22 operations and RC / 2 in each product, so evaluating it once takes the
-// 9 (22 + RC / 2) of a point's row to 5 (22 + RC), at the same ~69% of that datapath
-// (1,048,576 points, 16 columns: log 1.84 -> 1.47 ms, Gaussian 1.60 -> 1.36).
+// 9 (22 + RC / 2) of a point's row to 5 (22 + RC); it keeps that datapath 59% busy
+// (k_p2p_dmma ~69%), with fixed-latency stalls at 15 warps an SM (1,048,576
+// points, 16 columns: log 1.84 -> 1.47 ms, Gaussian 1.60 -> 1.36).
 template <class K, int RC>
 __global__ void __launch_bounds__(256, 2) k_near_dmma(NearView nv, KernelParams kp, const double* __restrict__ qs,
                                                       double* __restrict__ part, int warps) {

@@ -187,10 +187,9 @@ afmm_status afmm_get_l2p(afmm_handle* h, int level, int k, int32_t* rows, int32_
 
 /* Per-stage device times (ms) of the last matvec and setup, when profiling is
  * on.  names/values arrays of capacity `cap`; *n receives the count.  Stages
- * on the handle's stream are the intervals between consecutive marks; in a
- * batched pass the near field runs on a second stream beside the far field,
- * so its span is the separate "p2p_kernel" entry and "p2p" is the far
- * field's wait for it.  afmm_set_profiling(h, 2) profiles with the near
+ * on the handle's stream are the intervals between consecutive marks; the near
+ * field runs on a second stream beside the far field, so its span is the
+ * separate "p2p_kernel" entry and "p2p" is the wait for it.  afmm_set_profiling(h, 2) profiles with the near
  * field run after the far field on the handle's stream (same results), so
  * that "p2p" is the near-field kernel's own duration. */
 afmm_status afmm_set_profiling(afmm_handle* h, int on);
@@ -335,8 +334,8 @@ afmm_status afmm_destroy(afmm_handle* h);
  * by the caller and must outlive the set) and records, once, a CUDA graph in
  * which every stage of the FP64 matvec is one fused launch over all problems
  * (gather; the M2M of every level as one persistent up-sweep; M2L of all
- * levels; the L2L of every level as one persistent down-sweep; near field;
- * scatter).  In a sweep, work items wait on the device, each for at most
+ * levels and the sum of its two halves; the L2L of every level as one persistent
+ * down-sweep; the near field as a branch beside these; scatter).  In a sweep, work items wait on the device, each for at most
  * two seconds, until the level they read is complete; a wait that gives up
  * makes afmm_set_matvec return AFMM_TIMEOUT (the output is then incomplete;
  * the set stays usable).  afmm_set_matvec replays it: q and y hold the
