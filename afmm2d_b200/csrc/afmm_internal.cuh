@@ -187,22 +187,32 @@ std::atomic<int64_t>& device_alloc_counter();
 
 // Device allocations owned by a handle; freed together.  Pieces of up to
 // kPiece bytes are carved from slabs (256-byte aligned), each as large as all
-// slabs before it together, from 1 to 64 MiB: a handle has some 30 arrays per
-// level, and a cudaMalloc / cudaFree pair costs the setup ~0.15 ms whatever its
-// size (262,144 points: create + close 29 -> 20 ms, row tables 5.4 -> 3.0).
+// slabs before it together, from 0.5 to 64 MiB (or the piece alone when there is
+// no room for that): a handle has some 30 arrays per level, and a cudaMalloc /
+// cudaFree pair costs the setup ~0.15 ms (262,144 points: create + close 29 -> 20
+// ms, row tables 5.4 -> 3.0).  Above ~1 MiB the driver maps memory for each
+// one: first slabs of 1 MiB cost 1,306 points 0.6 ms in the setup and 0.4 in the
+// first batched product.
 struct DevArena {
-  static constexpr size_t kPiece = 16u << 20, kSlabMin = 1u << 20, kSlabMax = 64u << 20;
+  static constexpr size_t kPiece = 16u << 20, kSlabMin = 512u << 10, kSlabMax = 64u << 20;
   std::vector<void*> ptrs;
   size_t bytes = 0;
   unsigned char* slab = nullptr;
   size_t slab_size = 0, slab_used = 0, slabs = 0;
-  void* raw(size_t n) {
+  // Of n bytes, or of *least when there is no room for n (*least: what there was).
+  void* raw(size_t n, size_t* least = nullptr) {
     void* p = nullptr;
     cudaError_t e = cudaMalloc(&p, n);
+    if (e != cudaSuccess && least && *least < n) {
+      cudaGetLastError();
+      n = *least;
+      e = cudaMalloc(&p, n);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       throw Error{AFMM_OOM, "cudaMalloc of " + std::to_string(n) + " bytes failed"};
     }
+    if (least) *least = n;
     device_alloc_counter().fetch_add(1, std::memory_order_relaxed);
     ptrs.push_back(p);
     bytes += n;
@@ -219,8 +229,8 @@ struct DevArena {
     const size_t need = (n * sizeof(T) + 255) & ~(size_t)255;
     if (need > kPiece) return (T*)raw(n * sizeof(T));
     if (slab_used + need > slab_size) {
-      const size_t size = std::max(need, std::min(kSlabMax, std::max(kSlabMin, slabs)));
-      slab = (unsigned char*)raw(size);
+      size_t size = need;
+      slab = (unsigned char*)raw(std::max(need, std::min(kSlabMax, std::max(kSlabMin, slabs))), &size);
       slab_size = size;
       slab_used = 0;
       slabs += size;
