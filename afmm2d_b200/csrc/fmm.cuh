@@ -653,7 +653,10 @@ inline size_t m2l_pair_smem(int rmax) {
 
 // One group of (up to) 32 columns of m2l_pair_panel: P is the entry of the
 // lane's first row in its first column.  Only the last tile can hold rows past
-// the panel's end, and only a tail group columns past the warp's.
+// the panel's end, and only a tail group (not FULL) columns past the panel's:
+// what stands at sq past those is another panel's charge, or no charge at all
+// (past the staged columns come the sums that other lanes are writing), and a
+// zero entry does not cancel it when it is not finite, so it is not read.
 template <bool Q32, int NT, bool FULL>
 __device__ __forceinline__ double m2l_pair_group(const void* __restrict__ P, long r, int left, const double* sq,
                                                  bool last, const double (&qb)[NT], double (&y)[NT]) {
@@ -662,7 +665,7 @@ __device__ __forceinline__ double m2l_pair_group(const void* __restrict__ P, lon
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const bool vc = FULL || 4 * j + csub < left;
-    const double qc = sq[4 * j];  // (zero past the warp's columns)
+    const double qc = vc ? sq[4 * j] : 0.0;
     double m[NT];
 #pragma unroll
     for (int k = 0; k < NT; ++k) {
