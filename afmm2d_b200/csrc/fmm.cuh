@@ -925,6 +925,8 @@ __device__ __forceinline__ void pair_block(const PairPoints& P, const KernelPara
     x[u] = P.xy[idx[u]];
     w[u] = P.q[idx[u]];
     sum[u] = 0.0;
+    // (a lane without a part in the targets' sums adds 0 * 0 there: its charge may be infinite)
+    if (KIND == 2 && dst[u] <= 0) w[u] = 0.0;
   }
 #pragma unroll 4
   for (int t = 0; t < n; ++t) {

@@ -37,3 +37,19 @@ def test_infinite_charge_in_the_far_field_tables(precision):
             st = A.AFMMSet([a])
             assert np.all(st.matvec([q])[0][others] == -np.inf), leaf
             st.close()
+
+
+@pytest.mark.parametrize("N,M", [(7168, 7), (41984, 41), (8320, 130)])
+def test_infinite_charge_in_ragged_leaves(N, M):
+    """Leaves that do not fill the near field's blocks of 32 sources: a block then holds sources of the leaf
+    itself beside others, and unused lanes.  The Gaussian is positive, at distance zero too, so one infinite
+    charge makes its leaf's potentials +inf, and no far field of the leaf holds it."""
+    rng = np.random.default_rng(N)
+    a = A.AFMM(N, M, 6, rng.uniform(0, 1, (N, 2)), kernel="gaussian", kparam=0.1)
+    a.assemble()
+    members = leaf_members(a)
+    q0 = rng.standard_normal(N)
+    for leaf in range(0, len(members), max(1, len(members) // 11)):
+        q = q0.copy()
+        q[members[leaf][leaf % len(members[leaf])]] = np.inf
+        assert np.all(a.computeMatVecProduct(q)[members[leaf]] == np.inf), leaf
