@@ -81,4 +81,8 @@ __device__ __forceinline__ double exp_t32(double x) {
   return x < -708.0 ? 0.0 : y;
 }
 
+// The names under which user kernels were first offered these functions.
+__device__ __forceinline__ double log_tang(double x) { return log_t32(x); }
+__device__ __forceinline__ double exp_tang(double x) { return exp_t32(x); }
+
 }  // namespace afmm
