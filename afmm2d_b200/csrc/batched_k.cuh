@@ -391,8 +391,9 @@ __global__ void __launch_bounds__(256, 2) k_near_dmma(NearView nv, KernelParams 
   double2* sx = px + n8 + warp * 32;                  // the warp's sources
   double* accs = (double*)(px + n8 + warps * 32);     // the warps' sums of the targets
   double* acc = accs + (size_t)warp * n8 * RC;
-  for (int i = threadIdx.x; i < n8; i += blockDim.x)
-    px[i] = i < n ? nv.pts[s0 + i] : make_double2(kPadTgt64, kPadTgt64);
+  // (targets and sources past the last are the last one again, with no charge: a
+  // far-off place would make a growing user kernel's entries overflow, and 0 * inf is not 0)
+  for (int i = threadIdx.x; i < n8; i += blockDim.x) px[i] = nv.pts[s0 + min(i, n - 1)];
   for (int i = threadIdx.x; i < warps * n8 * RC; i += blockDim.x) accs[i] = 0.0;
   __syncthreads();
   const int ns = src.ns, total = src.off[ns], nblk = (total + 31) >> 5;
@@ -400,14 +401,15 @@ __global__ void __launch_bounds__(256, 2) k_near_dmma(NearView nv, KernelParams 
   const int from = 4 * (tsrc + (trow & 4)) + (trow & 3);
   const int b1 = (warp + 1) * nblk / warps;
   for (int blk = warp * nblk / warps; blk < b1; ++blk) {
-    const int f = 32 * blk + lane;
+    const int f = min(32 * blk + lane, total - 1);
     int m = 0;
     while (m + 1 < ns && f >= src.off[m + 1]) ++m;
-    const bool ok = f < total;
-    const int idx = ok ? src.src[m] + (f - src.off[m]) : -1;  // the lane's source
+    const bool ok = 32 * blk + lane < total;
+    const int place = src.src[m] + (f - src.off[m]);
+    const int idx = ok ? place : -1;  // the lane's source
     const int dst = ok ? src.dst[m] : 0;
     __syncwarp();
-    sx[lane] = ok ? nv.pts[idx] : make_double2(kPadSrc64, kPadSrc64);
+    sx[lane] = nv.pts[place];
     __syncwarp();
     const bool both = __any_sync(0xffffffffu, dst > 0);  // (a block of the leaf's own points: one product)
     double qc[8][RC / 8], yc[4][RC / 8][2];

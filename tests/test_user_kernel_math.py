@@ -34,3 +34,19 @@ def test_entries(plugin):
         f = A.kernel_eval(kernel, 2.0 ** -7, xy1, xy2, mode="fp64", param=param)
         g = A.kernel_eval(kernel, 2.0 ** -7, xy1, xy2, mode="exact", param=param)
         assert np.all(np.abs(f - g) <= ulps * 2.0 ** -52 * np.abs(g))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,M", [(4352, 68), (4160, 65)])
+def test_growing_kernel_in_batched_passes(plugin, N, M):
+    """r^4 log r overflows at the far-off places that a tile may be padded with: the FP64 batched near field, at
+    leaves that do and do not fill a tile of four or eight, gives the one-column product's potentials."""
+    rng = np.random.default_rng(N)
+    a = A.AFMM(N, M, 6, rng.uniform(0, 1, (N, 2)), kernel=SPLINE)
+    a.assemble()
+    Q = rng.standard_normal((N, 19))
+    for cols in (5, 19):
+        Y = a.computeMatVecProduct(np.asfortranarray(Q[:, :cols]), precision="fp64_batched")
+        for c in (0, cols - 1):
+            y = a.computeMatVecProduct(np.ascontiguousarray(Q[:, c]))
+            assert np.linalg.norm(Y[:, c] - y) <= 1e-12 * np.linalg.norm(y)
