@@ -199,19 +199,31 @@ struct DevArena {
   size_t bytes = 0;
   unsigned char* slab = nullptr;
   size_t slab_size = 0, slab_used = 0, slabs = 0;
+  // What only makes calls faster (an alloc_own piece; *spare is where its user
+  // looks for it) is given back when an allocation of this arena, or of one
+  // that has it as its lender, finds no room without.
+  double** spare = nullptr;
+  DevArena* lender = nullptr;
+  bool give_back() {
+    if (!spare || !*spare) return lender && lender->give_back();
+    release(*spare);
+    *spare = nullptr;
+    return true;
+  }
   // Of n bytes, or of *least when there is no room for n (*least: what there was).
   void* raw(size_t n, size_t* least = nullptr) {
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, n);
-    if (e != cudaSuccess && least && *least < n) {
+    auto fits = [&](size_t k) {
+      if (cudaMalloc(&p, k) == cudaSuccess) {
+        n = k;
+        return true;
+      }
       cudaGetLastError();
-      n = *least;
-      e = cudaMalloc(&p, n);
-    }
-    if (e != cudaSuccess) {
-      cudaGetLastError();
+      return false;
+    };
+    auto some = [&] { return fits(n) || (least && *least < n && fits(*least)); };
+    if (!some() && !(give_back() && some()))
       throw Error{AFMM_OOM, "cudaMalloc of " + std::to_string(n) + " bytes failed"};
-    }
     if (least) *least = n;
     device_alloc_counter().fetch_add(1, std::memory_order_relaxed);
     ptrs.push_back(p);
@@ -242,7 +254,7 @@ struct DevArena {
   void release(void* p) {
     for (auto& q : ptrs)
       if (q == p) {
-        cudaFree(q);
+        cudaFree(q);  // (waits for the device)
         q = nullptr;
       }
   }

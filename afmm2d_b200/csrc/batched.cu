@@ -852,10 +852,18 @@ void batch_reserve_parts(const MatvecPlan& p, BatchState& bs, DevArena& arena) {
   const KernelTable& kt = kernel_table(p.kp.id);
   for (int w = 0; w < 2; ++w)
     if (!kt.near_dmma[w](p.near, p.kp, nullptr, nullptr, false, nullptr)) return;
+  // Without them the near field works every pair out twice, so they leave at
+  // least as much memory free as they take (host calls' staging, autotuning and
+  // sets need less), and go first when that is used up as well.
+  const size_t n = (size_t)kNearParts * p.N * kBatchMax;
+  size_t free_b = 0, total_b = 0;
+  AFMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  if (free_b / 2 < n * sizeof(double)) return;
   try {
-    bs.near_parts = arena.alloc<double>((size_t)kNearParts * p.N * kBatchMax);
+    bs.near_parts = arena.alloc_own<double>(n);
+    arena.spare = &bs.near_parts;
   } catch (const Error& e) {
-    if (e.status != AFMM_OOM) throw;  // no room: the near field works every pair out twice
+    if (e.status != AFMM_OOM) throw;
   }
 }
 

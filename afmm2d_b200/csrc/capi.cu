@@ -1400,6 +1400,7 @@ void do_autotune(afmm_handle* h, int what) {
   // outgoing charges of every level for the M2L timings: one FP64 matvec and
   // one 16-column mixed pass of seeded random charges
   DevArena tmp;
+  tmp.lender = &h->arena;
   const int R = kBatchMax;
   double* dq = tmp.alloc<double>((size_t)N * R);
   double* dy = tmp.alloc<double>((size_t)N * R);
@@ -1739,6 +1740,7 @@ afmm_status afmm_eval_error(afmm_handle* h, int nsample, uint64_t seed, double* 
     for (long k : leaves)
       for (int i = 0; i < h->h_leaf_cnt[k]; ++i) rows.push_back(h->h_leaf_start[k] + i);
     DevArena tmp;
+    tmp.lender = &h->arena;
     int32_t* d_rows = tmp.alloc<int32_t>(rows.size());
     double* d_out = tmp.alloc<double>(rows.size());
     cudaStream_t s = h->stream;

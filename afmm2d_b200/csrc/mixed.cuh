@@ -53,7 +53,8 @@ struct BatchState {
   }
 };
 void batch_reserve(const MatvecPlan& p, BatchState& bs, DevArena& arena, cudaStream_t s);
-// The parts of FP64-batched near fields, when the leaves are small enough and the memory is there.
+// The parts of FP64-batched near fields, when the leaves are small enough and there is memory to spare (the
+// arena's spare piece).
 void batch_reserve_parts(const MatvecPlan& p, BatchState& bs, DevArena& arena);
 // The M2L stage alone of a batched pass of rc columns (on the batch buffers'
 // current outgoing charges); returns the launches made.

@@ -1,0 +1,35 @@
+"""Calls on a device with little memory left: what only makes calls faster gives way to what they need."""
+import numpy as np
+import pytest
+
+import afmm2d_b200 as A
+from test_gpu_parity import FP64_BATCHED_TOL
+
+pytestmark = pytest.mark.gpu
+
+
+def test_host_staging_takes_the_place_of_the_near_field_parts():
+    """A device call of 16 columns takes the batched near field's parts (168 MB); then 40 MB are left, and a host
+    call of 16 columns needs 67 for its staging."""
+    torch = pytest.importorskip("torch")
+    N = 262144
+    rng = np.random.default_rng(2)
+    a = A.AFMM(N, 64, 6, rng.uniform(0, 1, (N, 2)), kernel="log")
+    a.assemble()
+    Q = np.asfortranarray(rng.standard_normal((N, 16)))
+    y0 = a.computeMatVecProduct(Q[:, 3])
+    qd = torch.from_numpy(np.ascontiguousarray(Q.T)).cuda()
+    yd = torch.empty_like(qd)
+    free0 = torch.cuda.mem_get_info()[0]
+    a.matvec_device(qd.data_ptr(), yd.data_ptr(), 16, N, "fp64_batched")
+    assert free0 - torch.cuda.mem_get_info()[0] >= 5 * 16 * 8 * N  # the parts among what it took
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        Y = a.computeMatVecProduct(Q, precision="fp64_batched")
+        Y2 = a.computeMatVecProduct(Q, precision="fp64_batched")
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert np.linalg.norm(Y[:, 3] - y0) <= FP64_BATCHED_TOL * np.linalg.norm(y0)
+    np.testing.assert_array_equal(Y, Y2)
+    assert np.linalg.norm(yd[3].cpu().numpy() - y0) <= FP64_BATCHED_TOL * np.linalg.norm(y0)
