@@ -743,6 +743,11 @@ void finish_assemble(afmm_handle* h) {
       v.h_m2l_off[b + 1] = v.h_m2l_off[b] + e * v.h_rank[b];
       back_off[j][b + 1] = back_off[j][b] + f;
     }
+    v.fwd = h->arena.alloc<ForwardBox>(v.nbox);
+    v.back = h->arena.alloc<double>(back_off[j][v.nbox]);
+    v.back_off = h->arena.alloc<int64_t>(v.nbox + 1);
+    v.back_src = h->arena.alloc<int64_t>((size_t)v.nbox * kForwardSlots);
+    AFMM_CUDA(cudaMemcpyAsync(v.back_off, back_off[j].data(), sizeof(int64_t) * (v.nbox + 1), cudaMemcpyHostToDevice, s));
     m2l_total += v.h_m2l_off[v.nbox];
     l2p_total += v.h_l2p_off[v.nbox];
     rows_total += v.total_rank;
@@ -750,7 +755,8 @@ void finish_assemble(afmm_handle* h) {
   {
     // AUTO stores the blocks when they fit beside what the matvecs still
     // allocate (the row-major L2P copy, the mixed and 16-column batched
-    // buffers) with 2 GB to spare
+    // buffers) with 2 GB to spare; the one-column M2L's sums, which every
+    // storage needs, are allocated above and so counted
     size_t free_b = 0, total_b = 0;
     AFMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const double need = 8.0 * (double)m2l_total;
@@ -769,11 +775,6 @@ void finish_assemble(afmm_handle* h) {
     h->setup_phase[5].second += now_s() - t_al;
     v.qhat = h->arena.alloc<double>(v.total_rank + 2);  // + 16 B: whole-piece L2 prefetches
     v.yhat = h->arena.alloc<double>(v.total_rank);
-    v.fwd = h->arena.alloc<ForwardBox>(v.nbox);
-    v.back = h->arena.alloc<double>(back_off[j][v.nbox]);
-    v.back_off = h->arena.alloc<int64_t>(v.nbox + 1);
-    v.back_src = h->arena.alloc<int64_t>((size_t)v.nbox * kForwardSlots);
-    AFMM_CUDA(cudaMemcpyAsync(v.back_off, back_off[j].data(), sizeof(int64_t) * (v.nbox + 1), cudaMemcpyHostToDevice, s));
     // row -> box maps for the thread-per-row sweeps
     v.skel_box = h->arena.alloc<int32_t>(v.total_rank);
     v.node_box = h->arena.alloc<int32_t>(v.h_node_off[v.nbox]);
