@@ -1222,8 +1222,11 @@ void host_pipeline(afmm_handle* h, const double* q, double* y, int nrhs, int64_t
   const int N = h->N;
   const size_t need = 2 * (size_t)W;
   if (h->mixed.host_cap < need) {
-    if (h->mixed.d_qin) h->arena.release(h->mixed.d_qin);
-    if (h->mixed.d_yout) h->arena.release(h->mixed.d_yout);
+    h->mixed.host_cap = 0;  // (nothing is left of the old ones should the new ones not fit)
+    for (double** p : {&h->mixed.d_qin, &h->mixed.d_yout}) {
+      if (*p) h->arena.release(*p);
+      *p = nullptr;
+    }
     mixed_reserve_io(h->mixed, N, (int)need, h->arena);
   }
   cudaStream_t s = h->stream, si = h->s_h2d, so = h->s_d2h;

@@ -33,3 +33,27 @@ def test_host_staging_takes_the_place_of_the_near_field_parts():
     assert np.linalg.norm(Y[:, 3] - y0) <= FP64_BATCHED_TOL * np.linalg.norm(y0)
     np.testing.assert_array_equal(Y, Y2)
     assert np.linalg.norm(yd[3].cpu().numpy() - y0) <= FP64_BATCHED_TOL * np.linalg.norm(y0)
+
+
+def test_host_call_after_one_whose_staging_did_not_fit():
+    """Growing the staging gives the smaller one up first: when the larger does not fit, the call is refused and
+    the next one-column call allocates its own again."""
+    torch = pytest.importorskip("torch")
+    N = 262144
+    rng = np.random.default_rng(3)
+    a = A.AFMM(N, 64, 6, rng.uniform(0, 1, (N, 2)), kernel="one_over_r")
+    a.assemble()
+    q = rng.standard_normal((N, 16))
+    qd = torch.from_numpy(np.ascontiguousarray(q.T)).cuda()
+    a.matvec_device(qd.data_ptr(), torch.empty_like(qd).data_ptr(), 16, N, "mixed")  # its other buffers exist
+    y = a.computeMatVecProduct(q[:, 0])
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (32 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(A.AFMMError):
+            a.computeMatVecProduct(np.asfortranarray(q), precision="mixed")
+        again = a.computeMatVecProduct(q[:, 0])
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    np.testing.assert_array_equal(again, y)
+    assert a.computeMatVecProduct(np.asfortranarray(q), precision="mixed").shape == (N, 16)
