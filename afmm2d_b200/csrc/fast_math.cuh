@@ -10,47 +10,51 @@
 // (129 entries of 8 and 16 bytes, 24 lines) took ~24 L1 cycles per 32 entries
 // where the ~25 FP64 operations of an entry take 13 (64 lanes per SM and
 // cycle), so the FP64 near field of the log kernel was bound by its table.  A
-// word line is one L1 cycle: four of them here, at the price of two more
-// polynomial steps.  FP64 near field at 1,048,576 uniform points, log: 1.48 ->
-// 1.34 ms; on-the-fly M2L of 262,144 spiral points, log: 0.87 -> 0.80 ms.
+// word line is one L1 cycle: four of them here, at the price of three more
+// polynomial steps (when the tables were changed, every pair then evaluated
+// twice: FP64 near field at 1,048,576 uniform points, log, 1.48 -> 1.34 ms).
 #pragma once
 
 #include "math_tables.cuh"
 
 namespace afmm {
 
-// ln x for positive normal x.  x = 2^k m with m in [1 - 2^-6, 2 - 2^-6);
-// F = 1 + j/32 is the breakpoint nearest m, c = 1/F to 21 bits, u = m c - 1
-// (one rounding, below 2^-59; exact for j = 0, where c = 1), |u| <= 2^-6:
+// ln x for positive normal x.  x = 2^k m with m in [1 - 2^-6, 2 - 2^-6), j/32
+// nearest m - 1, c near 1/m of six or seven bits, so that u = m c - 1 is exact
+// (make_math_tables.py: log_centre), |u| < 0.0198, c = 1 for j = 0:
 //   ln x = (k ln2_hi + L_hi) + (u + (k ln2_lo + L_lo + u^2 q(u))),  L = -ln c.
 // ln2_hi and L_hi are multiples of 2^-42, so the first bracket is exact for
 // every exponent, and it is zero around x = 1 (j = 0, k = 0, on both sides),
-// where small results keep full relative accuracy.  q is the truncated
-// Chebyshev expansion of (ln(1+u) - u)/u^2 (error below 2^-57 of u).  14 FP64
-// operations.  Within one ulp (tests compare it with the correctly rounded
-// log); zero, subnormal and non-finite inputs give an unspecified value
-// without a trap, which the kernel functors select away.
+// where small results keep full relative accuracy; elsewhere it is larger than
+// u, and their sum's rounding error joins the small terms.  q is the truncated
+// Chebyshev expansion of (ln(1+u) - u)/u^2.  17 FP64 operations.  Error below
+// 0.53 ulp (tests); with c of 21 bits, a rounded u, one term less in q and u
+// added to the small terms (14 operations) it was 1.2 ulp, in the form with the
+// 129-entry table 0.76.  What the accuracy costs: near field at 1,048,576 points
+// 0.79 -> 0.83 ms, on-the-fly M2L of 131,072 0.22 -> 0.23.  Zero, subnormal and non-finite inputs give an
+// unspecified value without a trap, which the kernel functors select away.
 __device__ __forceinline__ double log_t32(double x) {
   const int hx = __double2hiint(x);
   const int t = hx + 0x4000;  // rounds the fraction to 5 bits, carrying into the exponent
   const int j = (t >> 15) & 31;
   const double m = __hiloint2double(hx - ((t & 0xfff00000) - 0x3ff00000), __double2loint(x));
-  // k = biased exponent - 1023, as a double without an integer conversion
-  const double kd = __hiloint2double(0x43300000, (t >> 20) & 0x7ff) - 4503599627371519.0;  // - (2^52 + 1023)
+  const double kd = (double)((t >> 20) - 1023);  // (a conversion: it does not take the FP64 pipe's time)
   const unsigned int* T = &kLogT32[0][j];
   const double c = __hiloint2double((int)__ldg(T), 0);
   const double Lh = __hiloint2double((int)__ldg(T + 32), (int)__ldg(T + 64));
   const double Ll = __hiloint2double((int)__ldg(T + 96), 0);
-  const double u = fma(m, c, -1.0);
+  const double u = fma(m, c, -1.0);  // exact
   const double hi = fma(kd, kLn2Hi, Lh);  // exact
   const double lo = fma(kd, kLn2Lo, Ll);
-  double q = fma(kLogQ6, u, kLogQ5);
+  double q = fma(kLogQ7, u, kLogQ6);
+  q = fma(q, u, kLogQ5);
   q = fma(q, u, kLogQ4);
   q = fma(q, u, kLogQ3);
   q = fma(q, u, kLogQ2);
   q = fma(q, u, kLogQ1);
   q = fma(q, u, kLogQ0);
-  return hi + (u + fma(q, u * u, lo));
+  const double s = hi + u;
+  return s + ((u - (s - hi)) + fma(q, u * u, lo));
 }
 
 // exp x.  x = (32 m + j) ln2/32 + r with N = 32 m + j the integer nearest

@@ -8,10 +8,11 @@ every double exponent k) and lo = ln F - hi rounded to double; ln 2 = entry
 128.
 exp: 2^(j/32) for j = 0..31 as hi + lo (hi the correctly rounded double), and
 ln2/32 as L1 + L2 with L1 a multiple of 2^-42 (N * L1 exact for |N| < 2^16).
-log_t32: for j = 0..31 and F = 1 + j/32: c = 1/F rounded to 21 significant bits
-(a double whose low word is zero), and -ln c as hi (a multiple of 2^-42) + lo
-(21 significant bits); the coefficients of q(u), |u| <= 2^-6, the truncated
-Chebyshev expansion of (ln(1+u) - u)/u^2.
+log_t32: for j = 0..31 and m in the interval of width 1/32 around 1 + j/32: c near
+its inverse, a multiple of 1/64 or of 1/128, so that u = m c - 1 is a double for
+every double m (log_centre), and -ln c as hi (a multiple of 2^-42) + lo (21
+significant bits); the coefficients of q(u), |u| <= 0.0198 (the largest), the
+truncated Chebyshev expansion of (ln(1+u) - u)/u^2.
 exp_t32: 2^(j/32) as above, lo to 21 significant bits.
 Both as arrays of 32 words, one 128-byte line each: a warp's lookup of one
 word touches one line whatever the lanes' indexes are.
@@ -54,10 +55,27 @@ def round21(x):
     return v
 
 
-def log_poly(degree):
-    """Truncated Chebyshev expansion of g(u) = (ln(1+u) - u)/u^2 on
-    [-2^-6, 2^-6], as monomial coefficients of u rounded to double."""
-    n, h = 40, Decimal(2) ** -6
+def log_centre(j):
+    """(c, largest |m c - 1|) for the doubles m in [1 + (j - 1/2)/32, 1 + (j + 1/2)/32).  m is a multiple of
+    2^-52 (2^-53 below 1, where c = 1), so m c - 1 is one of 2^-58 for c a multiple of 1/64, exact up to 2^-5,
+    and of 2^-59 for a multiple of 1/128, exact up to 2^-6."""
+    lo, hi = Fraction(2 * (32 + j) - 1, 64), Fraction(2 * (32 + j) + 1, 64)
+    if j == 0:
+        return Fraction(1), Fraction(1, 64)
+    best = None
+    for den, limit in ((64, Fraction(1, 32)), (128, Fraction(1, 64))):
+        for a in range(den // 2, den + 1):
+            c = Fraction(a, den)
+            u = max(abs(lo * c - 1), abs(hi * c - 1))
+            if u <= limit and (best is None or u < best[1]):
+                best = c, u
+    return best
+
+
+def log_poly(degree, h):
+    """Truncated Chebyshev expansion of g(u) = (ln(1+u) - u)/u^2 on [-h, h],
+    as monomial coefficients of u rounded to double."""
+    n, h = 40, Decimal(h.numerator) / Decimal(h.denominator)
 
     def g(u):  # its Taylor series: -1/2 + u/3 - u^2/4 + ...
         return sum(Decimal((-1) ** (k + 1)) * u ** k / (k + 2) for k in range(40))
@@ -136,8 +154,9 @@ def main():
               f"constexpr double k32OverLn2 = {inv.hex()};"]
     # log_t32 and exp_t32
     lw, ew = [[], [], [], []], [[], [], []]
+    centres = [log_centre(j) for j in range(32)]
     for j in range(32):
-        c = round21(Fraction(32, 32 + j))
+        c = float(centres[j][0])
         L = -Decimal(c).ln()  # (0 for j = 0)
         hi = Fraction(round(Fraction(L) * 2 ** 42), 2 ** 42)
         assert Fraction(float(hi)) == hi
@@ -151,7 +170,7 @@ def main():
     lines += word_array("kLogT32", lw)
     lines += ["", "// high, low word of the high part of 2^(j/32); high word of its low part"]
     lines += word_array("kExpT32", ew)
-    lines += [""] + [f"constexpr double kLogQ{i} = {c.hex()};" for i, c in enumerate(log_poly(6))]
+    lines += [""] + [f"constexpr double kLogQ{i} = {c.hex()};" for i, c in enumerate(log_poly(7, max(u for _, u in centres)))]
     lines += ["", "}  // namespace afmm", ""]
     with open(os.path.join(HERE, "math_tables.cuh"), "w") as f:
         f.write("\n".join(lines))
