@@ -73,12 +73,20 @@ struct KOneOverRScaled {
     double R = __dsqrt_rn(R2);
     return (R < p.a) ? __ddiv_rn(R, p.a) : __ddiv_rn(p.a, R);
   }
-  // with y = 1/R and R = R2 y, both branches are y times a factor (a = 2^-L,
-  // so R/a is an exact scaling of R): no square root and no division, within
-  // two ulp.  FP64 near field at 100,003 uniform points (M = 100): 1.17 -> 0.63 ms
+  // With y = 1/R both branches are a value times a power of two (a = 2^-L): R
+  // and y.  R = R2 y with P. Markstein's correction by the residual R2 - R^2 (IBM
+  // J. Res. Dev. 34(1), 1990), the square root's rounding in all but extremely rare
+  // cases, so the near branch is off by 0.5 ulp and the far one by rsqrt's
+  // 0.51 (0.5 and 0.99 with a square root and a division; 1.28 in the near branch
+  // without the correction).  R2 is compared by its bits, off the FP64 pipe
+  // (a2 is a power of two).  FP64 near field at 100,003 uniform points
+  // (M = 100), every pair evaluated twice: 1.17 ms with square root and division, 0.63 here.
   __device__ __forceinline__ static double eval(double R2, const KernelParams& p) {
-    const double w = R2 < p.a2 ? R2 * (p.a * p.inv_a2) : p.a;
-    return R2 == 0.0 ? 0.0 : rsqrt(R2) * w;
+    const double y = rsqrt(R2), R0 = R2 * y;
+    const double R = fma(fma(-R0, R0, R2), 0.5 * y, R0);
+    const bool near = __double2hiint(R2) < __double2hiint(p.a2);
+    const double v = (near ? R : y) * (near ? p.a * p.inv_a2 : p.a);
+    return __double_as_longlong(R2) == 0 ? 0.0 : v;
   }
   __device__ __forceinline__ static float eval32(float R2, float a, float) {
     // a = 2^-L: R/a and a/R are exact scalings of R and of 1/R

@@ -177,3 +177,33 @@ def test_device_log_error(lo, hi):
     ok = (x >= 1e-10) & (x != 1.0)
     err = np.abs(v.astype(np.longdouble) - ref)[ok] / np.spacing(np.abs(ref[ok].astype(np.float64)))
     assert ok.sum() > 0.99 * len(d) and err.max() <= LOG_ULPS + 0.002
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lo,hi,ulps", [(1e-6, 1.0 - 1e-9, 0.502), (1.0, 300.0, 0.992)])
+def test_device_scaled_entries(lo, hi, ulps):
+    """FP64 entries of the scaled 1/r on either side of R = a, of exact squared distances, against 80-bit
+    arithmetic: no further off than the square root (R/a) and the square root and division (a/R) that they
+    stand for, 0.5 ulp and 0.991."""
+    import afmm2d_b200 as A
+    rng = np.random.default_rng(9)
+    a = 2.0 ** -5
+    d = a * np.exp(rng.uniform(np.log(lo), np.log(hi), 400000))
+    x = d * d
+    p = np.stack([d, np.zeros_like(d)], axis=1)
+    v = A.kernel_eval("one_over_r_scaled", a, p, np.zeros_like(p), mode="fp64")
+    R = np.sqrt(x.astype(np.longdouble))
+    ref = np.where(x < a * a, R / a, a / R)
+    err = np.abs(v.astype(np.longdouble) - ref) / np.spacing(ref.astype(np.float64))
+    assert err.max() <= ulps
+
+
+@pytest.mark.gpu
+def test_device_scaled_entries_at_the_ends():
+    import afmm2d_b200 as A
+    a = 2.0 ** -5
+    d = np.array([0.0, 1e-100, 1e-30, np.nextafter(a, 0), a, np.nextafter(a, 1), 1e30, 1e150, 1e200])
+    p = np.stack([d, np.zeros_like(d)], axis=1)
+    got = A.kernel_eval("one_over_r_scaled", a, p, np.zeros_like(p), mode="fp64")
+    exact = A.kernel_eval("one_over_r_scaled", a, p, np.zeros_like(p), mode="exact")
+    assert np.all(np.abs(got - exact) <= np.spacing(exact)) and got[0] == 0.0 and got[-1] == 0.0
