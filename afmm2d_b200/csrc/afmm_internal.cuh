@@ -111,7 +111,7 @@ struct KLog {
   // branches are l times a factor (the same bits as 0.5*R2*l/a/a and 0.5*l),
   // selected without divergence.  R2 is not negative, so it is compared by
   // its bits: integer compares, off the FP64 pipe that bounds the callers
-  // (a2 is a power of two: its low word is zero).  l is within one ulp.
+  // (a2 is a power of two: its low word is zero).  l is within 0.53 ulp.
   __device__ __forceinline__ static double eval(double R2, const KernelParams& p) {
     const double near = R2 * (0.5 * p.inv_a2);
     const double w = __double2hiint(R2) < __double2hiint(p.a2) ? near : 0.5;

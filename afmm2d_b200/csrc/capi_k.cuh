@@ -57,7 +57,13 @@ __global__ void k_kernel_pairs(const double2* __restrict__ a, const double2* __r
     out[t] = K::eval_exact(r2_exact(p.x, p.y, q.x, q.y), kp);
   } else if (mode == 1) {
     double dx = p.x - q.x, dy = p.y - q.y;
-    out[t] = K::eval(dx * dx + dy * dy, kp);
+    const double R2 = dx * dx + dy * dy;
+    // The built-in kernels with a branch at R = a compare R2 with a2 by its high
+    // word, the whole of it in a tree (a = 2^-L); here a may be any number, so the
+    // branch is decided first.
+    if constexpr (K::id == AFMM_KERNEL_LOG || K::id == AFMM_KERNEL_ONE_OVER_R_SCALED)
+      kp.a2 = R2 < kp.a2 ? __longlong_as_double(0x7ff0000000000000LL) : 0.0;
+    out[t] = K::eval(R2, kp);
   } else {
     float dx = (float)(p.x - q.x), dy = (float)(p.y - q.y);
     out[t] = (double)K::eval32(fmaf(dx, dx, dy * dy), (float)kp.a, (float)kp.param);

@@ -207,3 +207,18 @@ def test_device_scaled_entries_at_the_ends():
     got = A.kernel_eval("one_over_r_scaled", a, p, np.zeros_like(p), mode="fp64")
     exact = A.kernel_eval("one_over_r_scaled", a, p, np.zeros_like(p), mode="exact")
     assert np.all(np.abs(got - exact) <= np.spacing(exact)) and got[0] == 0.0 and got[-1] == 0.0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", ["log", "one_over_r_scaled"])
+def test_device_entries_of_any_box_size(kernel):
+    """kernel_eval takes any box size a: the branch of a separation just below and just above one that is not a
+    power of two is the kernel's, at separations that differ from it in their last digits only.  A few ulps:
+    a * (1 / a^2) for 1 / a, and the two functions' own."""
+    import afmm2d_b200 as A
+    for a in (0.3, 0.0123, 0.7 * 2.0 ** -9):
+        d = a * (1.0 + np.concatenate([-np.logspace(-15, -4, 60), [0.0], np.logspace(-15, -4, 60)]))
+        p = np.stack([d, np.zeros_like(d)], axis=1)
+        got = A.kernel_eval(kernel, a, p, np.zeros_like(p), mode="fp64")
+        exact = A.kernel_eval(kernel, a, p, np.zeros_like(p), mode="exact")
+        assert np.all(np.abs(got - exact) <= 4 * np.spacing(np.abs(exact))), a
