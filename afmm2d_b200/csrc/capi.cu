@@ -1315,6 +1315,12 @@ float time_ms(cudaStream_t s, int reps, F&& f) {
   return t[t.size() / 2];
 }
 
+// Counted up whenever a tuned kernel or the meaning of a tuned value changes:
+// entries of other kernels in a cache file are not taken.  (1, not written: before
+// the one-column M2L worked pairs of boxes out once and pf_fp64 became the
+// bytes asked for at a warp's start.)
+constexpr int kTuningKernels = 2;
+
 std::string tuning_key(afmm_handle* h) {
   cudaDeviceProp pr;
   AFMM_CUDA(cudaGetDeviceProperties(&pr, h->device));
@@ -1324,7 +1330,8 @@ std::string tuning_key(afmm_handle* h) {
   return "dev=" + name + "|N=" + std::to_string(h->N) + "|M=" + std::to_string(h->M) + "|L=" + std::to_string(h->L) +
          "|kernel=" + std::to_string(h->kernel_id) + "|tol=" + std::to_string(h->tol_pow) +
          "|stored=" + std::to_string((h->m2l_stored ? 1 : 0) + (h->m2l_q_stored ? 2 : 0)) +
-         "|ranks=" + std::to_string(h->counts[2]) + "|entries=" + std::to_string(h->counts[4]);
+         "|ranks=" + std::to_string(h->counts[2]) + "|entries=" + std::to_string(h->counts[4]) +
+         "|kernels=" + std::to_string(kTuningKernels);
 }
 
 constexpr int kTuningValues = 8;
