@@ -1234,12 +1234,15 @@ void host_pipeline(afmm_handle* h, const double* q, double* y, int nrhs, int64_t
   if (nrhs <= W) {  // one pass: nothing to overlap, so everything on the handle's stream
     for (int c = 0; c < nrhs; ++c)
       AFMM_CUDA(cudaMemcpyAsync(h->mixed.d_qin + (size_t)c * N, q + (size_t)c * ld, bytes, cudaMemcpyHostToDevice, s));
-    // With large leaves the kernels are queued once the charges are there:
-    // queued behind the copy they all start together, and the far field's small
-    // kernels then come before the near field instead of into its tail (100,003
-    // points, M = 100, pinned: 0.64 against 0.48 ms).  With leaves of up to 64
-    // points the order matters little and the wait costs 10 us.
-    if (h->plan.near.nmax > 64) AFMM_CUDA(cudaStreamSynchronize(s));
+    // A one-column product of few, large leaves is queued once its charges are
+    // there: queued behind the copy its kernels all start together, and the far
+    // field's small ones then come before the near field instead of into its tail.
+    // Without / with the wait, pinned, us: 100,003 points, leaves of 391, FP64 707 /
+    // 516, mixed 775 / 721; 200,003, 196, 551 / 532 and 956 / 857; 131,072, 128, 447 / 457
+    // and 516 / 488.  With leaves of up to 64 points the wait only costs (131,072, 32,
+    // 316 / 338), and beside batched passes and products that start with the
+    // near field it makes no difference (within 1%).
+    if (nrhs == 1 && h->plan.small() && h->plan.near.nmax > 64) AFMM_CUDA(cudaStreamSynchronize(s));
     compute(h->mixed.d_qin, h->mixed.d_yout, nrhs);
     for (int c = 0; c < nrhs; ++c)
       AFMM_CUDA(cudaMemcpyAsync(y + (size_t)c * ld, h->mixed.d_yout + (size_t)c * N, bytes, cudaMemcpyDeviceToHost, s));
