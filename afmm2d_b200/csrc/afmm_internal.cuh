@@ -326,7 +326,6 @@ struct LevelDev {
   int32_t* node_ids = nullptr;  // node lists (sorted-point ids)
   int32_t* rank = nullptr;      // nbox
   int32_t* skel_box = nullptr;  // skeleton row -> box
-  int32_t* node_box = nullptr;  // node row -> box
   int32_t* grp_box = nullptr;   // row group (<= 8 rows of one box) -> box
   int32_t* grp_row = nullptr;   // row group -> first skeleton row
   long ngroups = 0;

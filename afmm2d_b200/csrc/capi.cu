@@ -399,7 +399,6 @@ void build_plan(afmm_handle* h) {
     v.back_off = d.back_off;
     v.back_src = d.back_src;
     v.skel_box = d.skel_box;
-    v.node_box = d.node_box;
     v.grp_box = d.grp_box;
     v.grp_row = d.grp_row;
     v.ngroups = d.ngroups;
@@ -775,12 +774,10 @@ void finish_assemble(afmm_handle* h) {
     h->setup_phase[5].second += now_s() - t_al;
     v.qhat = h->arena.alloc<double>(v.total_rank + 2);  // + 16 B: whole-piece L2 prefetches
     v.yhat = h->arena.alloc<double>(v.total_rank);
-    // row -> box maps for the thread-per-row sweeps
+    // skeleton row -> box, for the sums that other boxes worked out (m2l_back_row)
     v.skel_box = h->arena.alloc<int32_t>(v.total_rank);
-    v.node_box = h->arena.alloc<int32_t>(v.h_node_off[v.nbox]);
     fill_box_map(v.skel_off, v.nbox, v.skel_box, s);
-    fill_box_map(v.node_off, v.nbox, v.node_box, s);
-    h->launches += 2;
+    ++h->launches;
     // row groups of at most 8 skeleton rows of one box (on-the-fly M2L
     // tiles), balanced chunks of at most kChunkRows skeleton rows (M2L / M2M
     // tiles) or node rows (L2L tiles): a box of n rows is cut into

@@ -78,7 +78,6 @@ struct LevelView {
   double* qhat = nullptr;
   double* yhat = nullptr;
   const int32_t* skel_box = nullptr;  // skeleton row -> box
-  const int32_t* node_box = nullptr;  // node row -> box
   const int32_t* grp_box = nullptr;   // row group (<= 8 rows of one box) -> box
   const int32_t* grp_row = nullptr;   // row group -> first skeleton row
   long ngroups = 0;

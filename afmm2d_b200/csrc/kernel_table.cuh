@@ -18,7 +18,7 @@ namespace afmm {
 
 // Bumped whenever KernelTable or an argument type of its launchers changes:
 // a table compiled against other headers is refused at registration.
-constexpr int kKernelTableAbi = 6;
+constexpr int kKernelTableAbi = 7;
 
 // Fingerprint of the layouts of the launchers' argument types (sizes and a
 // few field offsets), recorded in every table where it is compiled: a table
