@@ -46,9 +46,7 @@ void aca_level(const AcaLevelIn& in, AcaLevelOut& out, DevArena& arena, AcaScrat
   // coordinates, flags, per-rank vectors, V-dot exchange) while they fit in a
   // quarter of the budget; whatever does not fit lives in a per-CTA slot of
   // global memory.  U then takes up to a quarter and V the rest.
-  int dev = 0, nsm = 148;
-  AFMM_CUDA(cudaGetDevice(&dev));
-  AFMM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int nsm = sm_count();
   long want_ctas = 2L * nsm;
   size_t budget = in.nbox >= want_ctas ? 100 * 1024 : 200 * 1024;
   if (in.ctas_per_sm == 1 || in.ctas_per_sm == 2) {  // set-up tuning overrides
@@ -230,7 +228,7 @@ void aca_level(const AcaLevelIn& in, AcaLevelOut& out, DevArena& arena, AcaScrat
     p.gscratch = nullptr;
     p.gx = nullptr;
     if (global_factor) {
-      grid = (int)std::min<long>(in.nbox, 148 * 8);
+      grid = (int)std::min<long>(in.nbox, 8L * nsm);
       const size_t n_fac = (size_t)grid * rmax * rmax;
       const size_t n_x = (size_t)grid * rmax * p.xs;
       scratch.factors.reserve(DevScratch::need({sizeof(double) * n_fac, sizeof(double) * n_x}));

@@ -193,6 +193,14 @@ struct KGaussian {
 // counts it here (read by afmm_get_device_alloc_count).
 std::atomic<int64_t>& device_alloc_counter();
 
+// Multiprocessors of the current device.
+inline int sm_count() {
+  int dev = 0, n = 0;
+  AFMM_CUDA(cudaGetDevice(&dev));
+  AFMM_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+  return n;
+}
+
 // Device allocations owned by a handle; freed together.  Pieces of up to
 // kPiece bytes are carved from slabs (256-byte aligned), each as large as all
 // slabs before it together, from 0.5 to 64 MiB (or the piece alone when there is

@@ -541,12 +541,12 @@ inline int near_dmma_warps(int nmax, bool few) {
 // 1.07; whole calls with 32-point leaves (524,288) 1.11 -> 1.13 / .87 -> .93 / 1.12 ->
 // 1.21.  With too few leaves to fill the GPU what counts is that five to eight
 // warps share a leaf instead of one per 32 targets (4,096 points, 91 -> 41 us; a
-// call 105 -> 80).  Two CTAs must fit an SM with the warps' target rows: leaves
-// of up to 104 points.
+// call 105 -> 80): `few`, up to two leaves an SM.  Two CTAs must fit an SM with
+// the warps' target rows: leaves of up to 104 points.
 template <class K, int RC>
 bool near_dmma_batched(const NearView& nv, const KernelParams& kp, const double* qs, double* part, bool launch,
                        cudaStream_t s) {
-  const bool few = nv.n <= 2L * 148 * nv.nmax;
+  const bool few = nv.n <= 2L * sm_count() * nv.nmax;
   const int warps = near_dmma_warps(nv.nmax, few);
   if (near_dmma_smem<16>(nv.nmax, warps) > 110 * 1024) return false;
   constexpr double entry = K::id == AFMM_KERNEL_LOG ? 22.0 : K::id == AFMM_KERNEL_GAUSSIAN ? 16.0 : 8.0;

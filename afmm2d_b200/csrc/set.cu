@@ -327,9 +327,8 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
       sp.l2l.push_back(b.upload(arena, s));
     }
   }
-  int nsm = 0, dev = 0, per_sm_up = 0, per_sm_dn = 0;
-  AFMM_CUDA(cudaGetDevice(&dev));
-  AFMM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int nsm = sm_count();
+  int per_sm_up = 0, per_sm_dn = 0;
   AFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_up, k_set_up, 32 * kUpWarps, 0));
   AFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_dn, k_set_down, 32 * kDownWarps, 0));
   sp.up.segs = upload(sp.m2m, arena, s);
