@@ -38,8 +38,8 @@ __global__ void k_set_scatter(SetDev d, SetSegs sg, double* __restrict__ y) {
 // The M2M of every level of every problem runs in one launch (the up-sweep),
 // and so does the L2L (the down-sweep).  Items are boxes, listed by depth in
 // dependency order (M2M: each problem's leaf level first; L2L: level 2 first);
-// a CTA takes the next kSweepBoxes items from a ticket counter, waits until
-// the level that a box reads has been published (per problem and level
+// a CTA takes the next box from a ticket counter, waits until the level that it
+// reads has been published (per problem and level
 // counters of boxes), computes it as the FP64 path does (same bits) and
 // publishes it.  An item only waits for items earlier in
 // the list, which CTAs already running hold, so the sweep cannot deadlock;
@@ -100,22 +100,19 @@ __global__ void __launch_bounds__(32 * kUpWarps, 20 / kUpWarps) k_set_up(SetDev 
   __shared__ int s_item, s_ok;
   for (int it; (it = next_item(sy.ticket, sw.nitems, &s_item)) >= 0;) {
     const SetSegs sg = sw.segs[sw.item_depth[it]];
-    const long g0 = sw.item_first[it], g1 = min(g0 + (long)kSweepBoxes, sg.total);
-    int s = seg_of(sg, g0);
-    for (long g = g0; g < g1; ++g) {
-      while (g >= sg.first[s + 1]) ++s;
-      const long pl = (long)sg.prob[s] * kMaxLevels + sg.level[s];
-      const LevelView& v = d.lv[pl];
-      const bool leaf = v.leaf_start != nullptr;
-      m2m_box<true>(v, leaf ? d.qs[sg.prob[s]] : d.lv[pl + 1].qhat, leaf ? 1 : 0, g - sg.first[s], [&] {
-        if (threadIdx.x == 0)
-          s_ok = leaf || wait_published(sy.done_up + pl + 1, d.lv[pl + 1].nbox + sw.margin, sy.err);
-        __syncthreads();
-        return s_ok != 0;
-      });
-      if (!s_ok) return;  // the same in every thread of the CTA
-      publish_box(sy.done_up + pl);
-    }
+    const long g = sw.item_first[it];
+    const int s = seg_of(sg, g);
+    const long pl = (long)sg.prob[s] * kMaxLevels + sg.level[s];
+    const LevelView& v = d.lv[pl];
+    const bool leaf = v.leaf_start != nullptr;
+    m2m_box<true>(v, leaf ? d.qs[sg.prob[s]] : d.lv[pl + 1].qhat, leaf ? 1 : 0, g - sg.first[s], [&] {
+      if (threadIdx.x == 0)
+        s_ok = leaf || wait_published(sy.done_up + pl + 1, d.lv[pl + 1].nbox + sw.margin, sy.err);
+      __syncthreads();
+      return s_ok != 0;
+    });
+    if (!s_ok) return;  // the same in every thread of the CTA
+    publish_box(sy.done_up + pl);
   }
 }
 
@@ -142,22 +139,19 @@ __global__ void __launch_bounds__(32 * kDownWarps, 28 / kDownWarps) k_set_down(S
   __shared__ int s_item, s_ok;
   for (int it; (it = next_item(sy.ticket + 1, sw.nitems, &s_item)) >= 0;) {
     const SetSegs sg = sw.segs[sw.item_depth[it]];
-    const long g0 = sw.item_first[it], g1 = min(g0 + (long)kSweepBoxes, sg.total);
-    int s = seg_of(sg, g0);
-    for (long g = g0; g < g1; ++g) {
-      while (g >= sg.first[s + 1]) ++s;
-      const long pl = (long)sg.prob[s] * kMaxLevels + sg.level[s];
-      const LevelView& v = d.lv[pl];
-      const bool leaf = v.leaf_start != nullptr;
-      l2l_box<true>(v, leaf ? nullptr : d.lv[pl + 1].yhat, d.ys[sg.prob[s]], leaf ? 1 : 0, g - sg.first[s], [&] {
-        if (threadIdx.x == 0)
-          s_ok = sg.level[s] == 2 || wait_published(sy.done_dn + pl - 1, d.lv[pl - 1].nbox + sw.margin, sy.err);
-        __syncthreads();
-        return s_ok != 0;
-      });
-      if (!s_ok) return;  // the same in every thread of the CTA
-      publish_box(sy.done_dn + pl);
-    }
+    const long g = sw.item_first[it];
+    const int s = seg_of(sg, g);
+    const long pl = (long)sg.prob[s] * kMaxLevels + sg.level[s];
+    const LevelView& v = d.lv[pl];
+    const bool leaf = v.leaf_start != nullptr;
+    l2l_box<true>(v, leaf ? nullptr : d.lv[pl + 1].yhat, d.ys[sg.prob[s]], leaf ? 1 : 0, g - sg.first[s], [&] {
+      if (threadIdx.x == 0)
+        s_ok = sg.level[s] == 2 || wait_published(sy.done_dn + pl - 1, d.lv[pl - 1].nbox + sw.margin, sy.err);
+      __syncthreads();
+      return s_ok != 0;
+    });
+    if (!s_ok) return;  // the same in every thread of the CTA
+    publish_box(sy.done_dn + pl);
   }
 }
 
@@ -293,13 +287,13 @@ void set_build(SetPlan& sp, const std::vector<const MatvecPlan*>& probs, DevAren
     sp.p2p_smem = std::max(sp.p2p_smem, near_smem(mp.near.nmax, warps[p]));
   }
   // M2M by depth below the leaf level; L2L by level from the top; each
-  // sweep's items are the depth tables' boxes in that order, kSweepBoxes at a time
+  // sweep's items are the depth tables' boxes in that order
   sp.m2m.clear();
   sp.l2l.clear();
   std::vector<int32_t> up_d, dn_d;
   std::vector<int64_t> up_r, dn_r;
   auto tiles = [](long total, int depth, std::vector<int32_t>& dd, std::vector<int64_t>& rr) {
-    for (long r = 0; r < total; r += kSweepBoxes) {
+    for (long r = 0; r < total; ++r) {
       dd.push_back(depth);
       rr.push_back(r);
     }

@@ -43,9 +43,8 @@ __device__ __forceinline__ int seg_of(const SetSegs& sg, long g) {
 }
 
 // A persistent sweep (every level of every problem in one launch): items are
-// kSweepBoxes boxes of one depth's flat box space (segs[depth]), listed in
-// dependency order; CTAs take them in list order from a ticket counter.
-constexpr int kSweepBoxes = 1;
+// the boxes of the depths' flat box spaces (segs[depth]), listed in dependency
+// order; CTAs take them in list order from a ticket counter.
 struct SweepPlan {
   const SetSegs* segs = nullptr;    // per depth (device array)
   const int32_t* item_depth = nullptr;
