@@ -854,11 +854,14 @@ void batch_reserve_parts(const MatvecPlan& p, BatchState& bs, DevArena& arena) {
     if (!kt.near_dmma[w](p.near, p.kp, nullptr, nullptr, false, nullptr)) return;
   // Without them the near field works every pair out twice, so they leave at
   // least as much memory free as they take (host calls' staging, autotuning and
-  // sets need less), and go first when that is used up as well.
+  // sets need less), and go first when that is used up as well.  (Small ones
+  // are not worth the ~0.1 ms that the question takes.)
   const size_t n = (size_t)kNearParts * p.N * kBatchMax;
-  size_t free_b = 0, total_b = 0;
-  AFMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if (free_b / 2 < n * sizeof(double)) return;
+  if (n * sizeof(double) > DevArena::kPiece) {
+    size_t free_b = 0, total_b = 0;
+    AFMM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (free_b / 2 < n * sizeof(double)) return;
+  }
   try {
     bs.near_parts = arena.alloc_own<double>(n);
     arena.spare = &bs.near_parts;
