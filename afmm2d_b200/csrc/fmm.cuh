@@ -377,9 +377,13 @@ struct MatvecPlan {
 // goes to the side.  Above, the near field follows on s and fills the GPU
 // first, and the far field takes slots as the near field's CTAs leave them (its
 // stream has the higher priority): it so runs in the near field's tail too,
-// where large leaves leave most SMs idle.  (ms, first
-// / second way: 1,048,576 points, mixture, 1/r 1.31 / 1.16, uniform, log 1.58 / 1.53;
-// 500,000 0.565 / 0.573; 300,000 mixed 0.450 / 0.499; 4,096 0.052 / 0.064.)
+// where large leaves leave most SMs idle.  Time of the second way over the first,
+// FP64 / mixed, over leaves of 32 to 391 points and four kernels: 0.89-1.13 /
+// 0.96-1.18 up to 131,072 points (above 1 with leaves of 32 to 64: there the chain is
+// the longer path, and two streams' launches cost 10 us), 0.96-1.05 / 0.94-1.13 at
+// 262,144, 0.85-1.02 / 0.93-1.01 at 400,000, 0.86-1.02 / 0.90-1.02 at 600,000 and more
+// (1,048,576 points, mixture, 1/r 1.29 -> 1.12 ms; uniform, log, leaves of 256 3.41 ->
+// 3.48).  The line is where nothing loses more than 2% any longer.
 template <class Near, class Far>
 inline void beside_near(const MatvecPlan& p, cudaStream_t s, StageTimer* tm, Near&& near, Far&& far) {
   if (tm && tm->serial) {
