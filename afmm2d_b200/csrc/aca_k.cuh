@@ -507,7 +507,7 @@ template <class K>
 struct AcaLaunch {
   static void run(const AcaArgs& a, int C, int ncl, size_t smem, cudaStream_t s) {
     auto fn = k_aca<K>;
-    AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(fn, smem);
     if (C > 8) AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ncl * C);
@@ -525,7 +525,7 @@ struct AcaLaunch {
   }
   static void occupancy(int C, size_t smem, int* ncl) {
     auto fn = k_aca<K>;
-    AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(fn, smem);
     if (C > 8) AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
@@ -660,10 +660,10 @@ template <class K>
 struct L2pRun {
   static void run(const L2pArgs& a, size_t smem, bool global_factor, int grid, cudaStream_t s) {
     if (global_factor) {
-      AFMM_CUDA(cudaFuncSetAttribute(k_l2p<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(k_l2p<K, true>, smem);
       k_l2p<K, true><<<grid, L2P_T, smem, s>>>(a);
     } else {
-      AFMM_CUDA(cudaFuncSetAttribute(k_l2p<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(k_l2p<K, false>, smem);
       k_l2p<K, false><<<grid, L2P_T, smem, s>>>(a);
     }
     AFMM_LAUNCH_CHECK();

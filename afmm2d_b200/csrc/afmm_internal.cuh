@@ -193,6 +193,22 @@ struct KGaussian {
 // counts it here (read by afmm_get_device_alloc_count).
 std::atomic<int64_t>& device_alloc_counter();
 
+// Allows `bytes` of dynamic shared memory for kernel `fn` (needed above 48 KB
+// with the kernel's static shared memory, a few KB at most).  The limit is the
+// function's, for every handle, set and thread: it goes to the most that the
+// function can have, once, so that nobody finds it lowered to another's bytes
+// between here and the launch.
+template <class F>
+inline void allow_smem(F* fn, size_t bytes) {
+  if (bytes <= 40 * 1024) return;
+  cudaFuncAttributes a;
+  AFMM_CUDA(cudaFuncGetAttributes(&a, fn));
+  const size_t most = 227 * 1024 - a.sharedSizeBytes;
+  if (bytes > most) throw Error{AFMM_BAD_ARG, "per-box rank too large for the sweep kernels"};
+  if ((size_t)a.maxDynamicSharedSizeBytes < most)
+    AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 // Multiprocessors of the current device.
 inline int sm_count() {
   int dev = 0, n = 0;

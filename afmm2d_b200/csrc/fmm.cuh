@@ -12,16 +12,6 @@ namespace afmm {
 
 constexpr int kMaxLevels = 16;
 
-// Allows `bytes` of dynamic shared memory for kernel `fn` (needed above 48 KB
-// with the kernel's static shared memory, a few KB at most).
-template <class F>
-inline void allow_smem(F* fn, size_t bytes) {
-  if (bytes > 40 * 1024) {
-    if (bytes > 227 * 1024) throw Error{AFMM_BAD_ARG, "per-box rank too large for the sweep kernels"};
-    AFMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  }
-}
-
 // The split of the SM's memory between shared memory and L1 that the kernels of
 // one product ask for (about 100 KB shared): an SM changes it only when it is
 // empty, so kernels that differ in it do not run side by side on one SM.

@@ -496,7 +496,7 @@ void kd_sort_run(const KdScratch& sc, const double* d_xy, int N, int L, int64_t*
   AFMM_CUDA(cudaMemcpyAsync(sc.starts, h_starts.data(), sizeof(int64_t) * (nseg + 1), cudaMemcpyHostToDevice, s));
   size_t smem = (size_t)kSmallSeg * 8 + (size_t)kSmallSeg * 4 * 3 + (size_t)(kSmallSeg + 1) * 4 +
                 (size_t)(2 * kSmallSeg + 1) * 4;
-  AFMM_CUDA(cudaFuncSetAttribute(k_kd_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(k_kd_bottom, smem);
   int32_t* out32 = (seq == sc.perm32) ? sc.perm_y : sc.perm32;  // perm_y is no longer needed
   k_kd_bottom<<<(int)nseg, BT_THREADS, smem, s>>>(seq, sc.starts, lb, L, sc.rank_x0, sc.rank_x, sc.rank_y, out32);
   k_finish_perm<<<gb, T, 0, s>>>(out32, d_xy, N, d_perm, d_xy_sorted);
