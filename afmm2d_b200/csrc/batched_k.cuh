@@ -373,10 +373,10 @@ __global__ void __launch_bounds__(128) k_p2p_dmma(NearView nv, KernelParams kp, 
 // product (8 sources x 4 targets).  The sources' sums stay in registers over
 // all targets, the targets' in a shared-memory row of the warp, added in warp
 // order at the end.  part: kNearParts x n x RC.  FP64 datapath: an entry costs
-// ~22 operations and RC / 2 in each product, so evaluating it once takes the
-// 9 (22 + RC / 2) of a point's row to 5 (22 + RC); it keeps that datapath 59% busy
+// ~25 operations (log) and RC / 2 in each product, so evaluating it once takes the
+// 9 (25 + RC / 2) of a point's row to 5 (25 + RC); it keeps that datapath 61% busy
 // (k_p2p_dmma ~69%), with fixed-latency stalls at 15 warps an SM (1,048,576
-// points, 16 columns: log 1.84 -> 1.47 ms, Gaussian 1.60 -> 1.36).
+// points, 16 columns: log 1.94 -> 1.50 ms, Gaussian 1.60 -> 1.37).
 template <class K, int RC>
 __global__ void __launch_bounds__(256, 2) k_near_dmma(NearView nv, KernelParams kp, const double* __restrict__ qs,
                                                       double* __restrict__ part, int warps) {
@@ -535,11 +535,11 @@ inline int near_dmma_warps(int nmax, bool few) {
 // The line, in FP64 operations per point at 16 columns: k_p2p_dmma works out
 // nine leaves of points in groups of 32 targets, k_near_dmma five in groups of
 // 8 and moves 1 KB of parts (~2,500 operations' time).  16 columns, k_p2p_dmma ->
-// k_near_dmma, near field and scatter, log / Gaussian / 1/r: 64-point leaves
-// (1,048,576) 1.90 -> 1.64 / 1.65 -> 1.53 / 1.31 -> 1.39 ms; 98 (400,000) 1.47 ->
-// 1.01 / 1.27 -> .95 / 1.02 -> .84; 49 (800,000) 1.54 -> 1.22 / 1.34 -> 1.16 / 1.07 ->
-// 1.07; whole calls with 32-point leaves (524,288) 1.11 -> 1.13 / .87 -> .93 / 1.12 ->
-// 1.21.  With too few leaves to fill the GPU what counts is that five to eight
+// k_near_dmma, near field and scatter, log / Gaussian / scaled 1/r / 1/r: 64-point
+// leaves (1,048,576) 2.01 -> 1.68 / 1.67 -> 1.55 / 1.48 -> 1.43 / 1.31 -> 1.39 ms; 98
+// (400,000) 1.55 -> 1.12 / 1.28 -> 1.05 / 1.15 -> .94 / 1.02 -> .93; 49 (800,000) 1.63 ->
+// 1.16 / 1.35 -> 1.09 / 1.20 -> 1.01 / 1.07 -> .98; whole calls with 32-point leaves
+// (524,288) 1.16 -> 1.14 / .88 -> .94 / 1.21 -> 1.28 / 1.13 -> 1.22.  With too few leaves to fill the GPU what counts is that five to eight
 // warps share a leaf instead of one per 32 targets (4,096 points, 91 -> 41 us; a
 // call 105 -> 80): `few`, up to two leaves an SM.  Two CTAs must fit an SM with
 // the warps' target rows: leaves of up to 104 points.
@@ -549,7 +549,10 @@ bool near_dmma_batched(const NearView& nv, const KernelParams& kp, const double*
   const bool few = nv.n <= 2L * sm_count() * nv.nmax;
   const int warps = near_dmma_warps(nv.nmax, few);
   if (near_dmma_smem<16>(nv.nmax, warps) > 110 * 1024) return false;
-  constexpr double entry = K::id == AFMM_KERNEL_LOG ? 22.0 : K::id == AFMM_KERNEL_GAUSSIAN ? 16.0 : 8.0;
+  constexpr double entry = K::id == AFMM_KERNEL_LOG                ? 25.0
+                           : K::id == AFMM_KERNEL_GAUSSIAN         ? 16.0
+                           : K::id == AFMM_KERNEL_ONE_OVER_R_SCALED ? 13.0
+                                                                    : 8.0;
   const double twice = 9.0 * ((nv.nmax + 31) & ~31) * (entry + 8.0);
   const double once = 5.0 * ((nv.nmax + 7) & ~7) * (entry + 16.0) + 2500.0;
   if (!few && 1.05 * once > twice) return false;
