@@ -31,8 +31,8 @@ namespace afmm {
 // 0.53 ulp (tests); with c of 21 bits, a rounded u, one term less in q and u
 // added to the small terms (14 operations) it was 1.2 ulp, in the form with the
 // 129-entry table 0.76.  What the accuracy costs: near field at 1,048,576 points
-// 0.79 -> 0.83 ms, on-the-fly M2L of 131,072 0.22 -> 0.23.  Zero, subnormal and non-finite inputs give an
-// unspecified value without a trap, which the kernel functors select away.
+// 0.79 -> 0.83 ms.  Zero, subnormal and non-finite inputs give an unspecified
+// value without a trap, which the kernel functors select away.
 __device__ __forceinline__ double log_t32(double x) {
   const int hx = __double2hiint(x);
   const int t = hx + 0x4000;  // rounds the fraction to 5 bits, carrying into the exponent
@@ -61,10 +61,9 @@ __device__ __forceinline__ double log_t32(double x) {
 // x 32/ln2, j = N mod 32, |r| <= ln2/64 (r = x - N L1 - N L2, N L1 exact);
 //   exp(x) = 2^m (S_hi + (S_lo + S p(r))),  S = 2^(j/32) = S_hi + S_lo,
 // p(r) = exp(r) - 1 by its Taylor polynomial to r^6 (truncation below
-// 2^-58); 2^m is added to the exponent bits.  13 FP64 operations.  Error
-// within about one ulp for x in [-708, 709.7] (tests compare it with the
-// correctly rounded exp); below -708 it returns 0 (the true value is under
-// 2^-1021).
+// 2^-58); 2^m is added to the exponent bits.  13 FP64 operations.  Error at
+// most 0.55 ulp for x in [-708, 709.7] (tests over that range); below -708 it
+// returns 0 (the true value is under 2^-1021).
 __device__ __forceinline__ double exp_t32(double x) {
   const double shifter = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
   const double t = fma(x, k32OverLn2, shifter);

@@ -1060,15 +1060,15 @@ struct NearSources {
 // with itself the leaf's own.  Per point nv.part[0] takes the leaf's own
 // work and part[1 + s] what its neighbour in slot 4 + s worked out for it
 // (zero without one); the scatter adds the five in that order.  An entry costs
-// 15 to 22 FP64 operations and about as many integer ones, its use two, so
+// 12 to 25 FP64 operations and about as many integer ones, its use two, so
 // working it out once for both leaves (5/9 of the entries) pays for the target
 // sums that go from lane to lane through shared memory (four cycles of 18 an
-// entry pair takes there).  What bounds it now is issue (63% of the slots,
-// FP64 pipe 49% busy) and the polynomials' dependent steps: 80 registers (24
+// entry pair takes there).  What bounds it now is issue (62% of the slots,
+// FP64 pipe 53% busy) and the polynomials' dependent steps: 80 registers (24
 // warps an SM) measured faster than 102 or 64.  Near field at 1,048,576 uniform
 // points, one CTA per leaf, all nine source leaves before -> now: log 1.34 ->
-// 0.79 ms, Gaussian 1.03 -> 0.66, 1/r (mixture) 0.64 -> 0.42; 100,003 points of
-// scaled 1/r (M = 100) 0.63 -> 0.42.  Run by one CTA of near_warps(nmax) warps
+// 0.83 ms, Gaussian 1.03 -> 0.67, 1/r (mixture) 0.64 -> 0.42; 100,003 points of
+// scaled 1/r (M = 100) 0.63 -> 0.40.  Run by one CTA of near_warps(nmax) warps
 // that share the blocks of 32 source points evenly (more may be present); the
 // sums of the warps are added in warp order.
 template <class K>

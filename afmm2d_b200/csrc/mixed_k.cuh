@@ -21,7 +21,7 @@ __device__ __forceinline__ float fallback_r2(float span_b, float span_c) {
 // first): the box's skeleton points against those of its forward
 // interaction-list boxes, every entry worked out once for both (pair_targets,
 // as the FP64 near field; the sums as in m2l_pair_box).  Issue-bound like it:
-// 262,144 spiral points, log, TOL 12: 0.80 -> 0.34 ms (one thread per skeleton
+// 262,144 spiral points, log, TOL 12: 0.80 -> 0.35 ms (one thread per skeleton
 // row, every entry worked out for both sides).
 constexpr int kOtfWarps = 4;
 template <class K>
