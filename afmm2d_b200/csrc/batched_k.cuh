@@ -108,10 +108,15 @@ constexpr float kPadSrc = 1.0e15f, kPadTgt = -1.0e15f;
 // warp vote sends the rare close pairs to the FP64 fallback.  The high*high
 // products and the two correction products accumulate in separate FP32 tiles
 // (independent MMA chains), which are added per source leaf into FP64 sums
-// kept in shared memory.
+// kept in shared memory.  Issue-bound; how the compiler orders the loads of a
+// step among its entries depends on the registers it is told to keep to: 16
+// columns for five CTAs an SM (1,048,576 points, log / Gaussian / 1/r 1.21 / 0.69 /
+// 0.65 ms; four 1.31 / .75 / .73, six 1.59 / .85 / .70, left to it 1.32 / .77 / .73), 8
+// columns left to it (.99 / .53 / .44; five .99 / .53 / .50).
 template <class K, int RC>
-__global__ void __launch_bounds__(128, 5) k_p2p_mma(NearView nv, KernelParams kp, const uint2* __restrict__ qhl,
-                                                 double* __restrict__ ys) {
+__global__ void __launch_bounds__(128, RC == 16 ? 5 : 0) k_p2p_mma(NearView nv, KernelParams kp,
+                                                                      const uint2* __restrict__ qhl,
+                                                                      double* __restrict__ ys) {
   constexpr int NE = 2 * (RC / 8) * 4;  // FP64 sums per lane
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_src[9], s_cnt[9], s_coff[10], s_ns;
