@@ -289,9 +289,23 @@ constexpr double kPadSrc64 = 1.0e100, kPadTgt64 = -1.0e100;
 // far stand-ins; each lane evaluates one FP64 entry per tile and 4-source step
 // with the FP64 matvec form K::eval (the diagonal included, as in the FP64
 // path), and the 8 x 4 entry tiles multiply the 4 x RC FP64 charge blocks
-// (mma.sync m8n8k4, FP64 accumulation).
+// (mma.sync m8n8k4, FP64 accumulation).  Of a step's four tiles kAhead have
+// their entries before their products, and kCtas (0: the compiler's choice) CTAs
+// an SM bound the registers: short formulas gain from four at once (1/r, 8
+// columns, 12,000 points in 64 leaves 0.38 -> 0.29 ms, 800,000 in 4,096 2.52 -> 2.42; 16
+// columns .41 -> .35, 3.44 -> 3.50), the long table-driven functions from enough
+// registers to run into each other by themselves (log, 8 columns, kCtas 0 -> 4: .45 ->
+// .36, 4.48 -> 4.46; Gaussian .35 -> .27, 3.56 -> 3.43; Gaussian, 16 columns, 819,200
+// points 4.46 -> 4.33; log, 16 columns, worse: 5.27 -> 5.63 at 800,000).
 template <class K, int RC>
-__global__ void __launch_bounds__(128) k_p2p_dmma(NearView nv, KernelParams kp, const double* __restrict__ qs,
+struct DmmaOrder {
+  static constexpr bool kGauss = K::id == AFMM_KERNEL_GAUSSIAN, kTable = kGauss || K::id == AFMM_KERNEL_LOG;
+  static constexpr int kAhead = !kTable ? 4 : (kGauss && RC == 16 ? 2 : 1);
+  static constexpr int kCtas = kTable && (kGauss || RC == 8) ? 4 : 0;
+};
+
+template <class K, int RC>
+__global__ void __launch_bounds__(128, DmmaOrder<K, RC>::kCtas) k_p2p_dmma(NearView nv, KernelParams kp, const double* __restrict__ qs,
                                                   double* __restrict__ ys) {
   constexpr int NTT = 4;  // 8-row target tiles per warp
   extern __shared__ __align__(16) unsigned char smem[];
@@ -342,12 +356,19 @@ __global__ void __launch_bounds__(128) k_p2p_dmma(NearView nv, KernelParams kp, 
         const bool vj = j < nc;
         double bq[RC / 8];
         load_b<RC>(qs + (long)(src + j) * RC, trow, vj, bq);
+        constexpr int A = DmmaOrder<K, RC>::kAhead;
 #pragma unroll
-        for (int u = 0; u < NTT; ++u) {
-          const double dx = x[u].x - p.x, dy = x[u].y - p.y;
-          const double a = K::eval(dx * dx + dy * dy, kp);
+        for (int u0 = 0; u0 < NTT; u0 += A) {
+          double a[A];
 #pragma unroll
-          for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(c[u][t][0], c[u][t][1], a, bq[t]);
+          for (int u = 0; u < A; ++u) {
+            const double dx = x[u0 + u].x - p.x, dy = x[u0 + u].y - p.y;
+            a[u] = K::eval(dx * dx + dy * dy, kp);
+          }
+#pragma unroll
+          for (int u = 0; u < A; ++u)
+#pragma unroll
+            for (int t = 0; t < RC / 8; ++t) mma_f64_8x8x4(c[u0 + u][t][0], c[u0 + u][t][1], a[u], bq[t]);
         }
       }
     }
@@ -538,28 +559,39 @@ inline int near_dmma_warps(int nmax, bool few) {
 
 // k_near_dmma for all leaves of nv, when it is the better form (false: k_p2p_dmma).
 // The line, in FP64 operations per point at 16 columns: k_p2p_dmma works out
-// nine leaves of points in groups of 32 targets, k_near_dmma five in groups of
-// 8 and moves 1 KB of parts (~2,500 operations' time).  16 columns, k_p2p_dmma ->
-// k_near_dmma, near field and scatter, log / Gaussian / scaled 1/r / 1/r: 64-point
-// leaves (1,048,576) 2.01 -> 1.68 / 1.67 -> 1.55 / 1.48 -> 1.43 / 1.31 -> 1.39 ms; 98
-// (400,000) 1.55 -> 1.12 / 1.28 -> 1.05 / 1.15 -> .94 / 1.02 -> .93; 49 (800,000) 1.63 ->
-// 1.16 / 1.35 -> 1.09 / 1.20 -> 1.01 / 1.07 -> .98; whole calls with 32-point leaves
-// (524,288) 1.16 -> 1.14 / .88 -> .94 / 1.21 -> 1.28 / 1.13 -> 1.22.  With too few leaves to fill the GPU what counts is that five to eight
-// warps share a leaf instead of one per 32 targets (4,096 points, 91 -> 41 us; a
-// call 105 -> 80): `few`, up to two leaves an SM.  Two CTAs must fit an SM with
-// the warps' target rows: leaves of up to 104 points.
+// nine leaves of points in groups of 32 targets, a warp each, up to four warps a
+// CTA, so that with five or six groups warps wait in the second round (`idle`);
+// k_near_dmma works out five in groups of 8 and moves 1 KB of parts (~2,500
+// operations' time), and with fewer than three CTAs an SM its latencies show.
+// Whole calls, 16 columns, k_p2p_dmma / k_near_dmma, log, Gaussian, scaled 1/r, 1/r
+// (ms; 4,096 leaves, above 16,384):
+//   leaves of 48 points  2.19 / 1.70  1.72 / 1.43  2.03 / 1.81  1.83 / 1.70
+//             56         2.47 / 2.13  1.94 / 1.81  2.26 / 2.20  2.03 / 2.06
+//             88         1.39 / 1.10  1.17 / 1.01  1.15 / 1.06  1.04 / 0.99
+//             112        2.00 / 1.85  1.64 / 1.66  1.63 / 1.66  1.47 / 1.62
+//             136        3.23 / 2.34  2.63 / 2.12  2.58 / 2.00  2.47 / 1.93
+//             152        3.63 / 3.09  2.97 / 2.83  2.93 / 2.68  2.84 / 2.62
+//             200        5.83 / 5.24  4.81 / 4.79  4.51 / 4.33  3.97 / 4.26
+// and with 32-point leaves (524,288 points) 1.16 / 1.14, .88 / .94, 1.21 / 1.28,
+// 1.13 / 1.22.  With too few leaves to fill the GPU (`few`: up to two an SM) what
+// counts is that five to eight warps share a leaf instead of one per 32 targets
+// (4,096 points, 91 -> 41 us; 12,000 points in 64 leaves .44 -> .17 ms), whatever shared
+// memory their target rows take.
 template <class K, int RC>
 bool near_dmma_batched(const NearView& nv, const KernelParams& kp, const double* qs, double* part, bool launch,
                        cudaStream_t s) {
   const bool few = nv.n <= 2L * sm_count() * nv.nmax;
   const int warps = near_dmma_warps(nv.nmax, few);
-  if (near_dmma_smem<16>(nv.nmax, warps) > 110 * 1024) return false;
+  const size_t smem16 = near_dmma_smem<16>(nv.nmax, warps);
+  if (smem16 > (few ? 220 : 110) * 1024) return false;
   constexpr double entry = K::id == AFMM_KERNEL_LOG                ? 25.0
                            : K::id == AFMM_KERNEL_GAUSSIAN         ? 16.0
                            : K::id == AFMM_KERNEL_ONE_OVER_R_SCALED ? 13.0
                                                                     : 8.0;
-  const double twice = 9.0 * ((nv.nmax + 31) & ~31) * (entry + 8.0);
-  const double once = 5.0 * ((nv.nmax + 7) & ~7) * (entry + 16.0) + 2500.0;
+  const int groups = (nv.nmax + 31) / 32;
+  const double idle = groups > 4 ? 1.0 - groups / (4.0 * ((groups + 3) / 4)) : 0.0;
+  const double twice = 9.0 * (32 * groups) * (entry + 8.0) * (1.0 + 1.8 * idle * idle);
+  const double once = (5.0 * ((nv.nmax + 7) & ~7) * (entry + 16.0) + 2500.0) * (smem16 > 74 * 1024 ? 1.29 : 1.0);
   if (!few && 1.05 * once > twice) return false;
   if (!launch) return true;
   const size_t smem = near_dmma_smem<RC>(nv.nmax, warps);
