@@ -57,3 +57,27 @@ def test_host_call_after_one_whose_staging_did_not_fit():
         torch.cuda.empty_cache()
     np.testing.assert_array_equal(again, y)
     assert a.computeMatVecProduct(np.asfortranarray(q), precision="mixed").shape == (N, 16)
+
+
+def test_batched_near_field_without_room_for_its_parts():
+    """With less than twice the parts' bytes free they are not taken, and the call works every pair out twice."""
+    torch = pytest.importorskip("torch")
+    N = 262144
+    parts = 5 * 16 * 8 * N
+    rng = np.random.default_rng(4)
+    a = A.AFMM(N, 64, 6, rng.uniform(0, 1, (N, 2)), kernel="log")
+    a.assemble()
+    q = rng.standard_normal((N, 16))
+    qd = torch.from_numpy(np.ascontiguousarray(q.T)).cuda()
+    yd = torch.empty_like(qd)
+    a.matvec_device(qd.data_ptr(), yd.data_ptr(), 16, N, "mixed")  # its other buffers exist
+    y = a.computeMatVecProduct(q[:, 5])
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - 3 * parts // 2, dtype=torch.uint8, device="cuda")
+    try:
+        free = torch.cuda.mem_get_info()[0]
+        a.matvec_device(qd.data_ptr(), yd.data_ptr(), 16, N, "fp64_batched")
+        assert free - torch.cuda.mem_get_info()[0] < parts // 2
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert np.linalg.norm(yd[5].cpu().numpy() - y) <= FP64_BATCHED_TOL * np.linalg.norm(y)
